@@ -107,97 +107,6 @@ __host__ __device__ constexpr InteriorChunk<LT> interior_chunk() {
     return k;
 }
 
-template <int LT, int NV, typename CT, int W = 32>
-__device__ __forceinline__ void warp_solve_interior(const DevTables<CT> &T, CT (&d)[NV][LT], int lane);
-
-// Solve NV right-hand sides held as d[v][t] by the lanes of one warp; the
-// solution overwrites d.  All 32 lanes must call it (warp shuffles).  W < 32:
-// every W lanes solve a line of their own (lines with p <= W chunks and at
-// most log2(W) + 1 PCR steps), `lane` is the lane within its W-lane segment.
-template <int LT, int NV, typename CT, int W = 32>
-__device__ __forceinline__ void warp_solve(const DevTables<CT> &T, CT (&d)[NV][LT], int lane) {
-    if (LT >= 2 && T.interior) {
-        warp_solve_interior<LT, NV, CT, W>(T, d, lane);
-        return;
-    }
-    const int len = lane_len(lane, LT, T.p, T.last_len);
-#pragma unroll
-    for (int t = 0; t < LT; ++t) {
-        const CT f1 = T.fwd1[t * 32 + lane];
-        if (t == 0) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) d[v][0] = f1 * d[v][0];
-        } else {
-            const CT f2 = T.fwd2[t * 32 + lane];
-#pragma unroll
-            for (int v = 0; v < NV; ++v) d[v][t] = f1 * d[v][t] + f2 * d[v][t - 1];
-        }
-    }
-#pragma unroll
-    for (int t = LT - 2; t >= 0; --t) {
-        const CT b1 = T.bwd1[t * 32 + lane], b2 = T.bwd2[t * 32 + lane];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) d[v][t] = b1 * d[v][t] + b2 * d[v][t + 1];
-    }
-    CT y0[NV], y1[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        y0[v] = d[v][0];
-        y1[v] = CT(0);
-#pragma unroll
-        for (int t = 1; t < LT; ++t)
-            if (t == len - 1) y1[v] = d[v][t];
-    }
-    {
-        const CT ka = T.k1[lane], kb = T.k2[lane], kc = T.k1[32 + lane], kd = T.k2[32 + lane];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const CT up1 = __shfl_up_sync(0xffffffffu, y1[v], 1, W);
-            const CT dn0 = __shfl_down_sync(0xffffffffu, y0[v], 1, W);
-            const CT n0 = y0[v] - ka * up1 - kb * y1[v];
-            const CT n1 = y1[v] - kc * y0[v] - kd * dn0;
-            y0[v] = n0;
-            y1[v] = n1;
-        }
-    }
-#pragma unroll
-    for (int s = 1; s < kPcrSteps; ++s) {
-        if (s >= T.pcr) break;
-        const int dl = 1 << (s - 1);
-        const CT ka = T.k1[s * 64 + lane], kb = T.k2[s * 64 + lane];
-        const CT kc = T.k1[s * 64 + 32 + lane], kd = T.k2[s * 64 + 32 + lane];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const CT u0 = __shfl_up_sync(0xffffffffu, y0[v], dl, W);
-            const CT d0 = __shfl_down_sync(0xffffffffu, y0[v], dl, W);
-            const CT u1 = __shfl_up_sync(0xffffffffu, y1[v], dl, W);
-            const CT d1 = __shfl_down_sync(0xffffffffu, y1[v], dl, W);
-            y0[v] = y0[v] - ka * u0 - kb * d0;
-            y1[v] = y1[v] - kc * u1 - kd * d1;
-        }
-    }
-    const CT ib0 = T.invb[lane], ib1 = T.invb[32 + lane];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const CT X0 = y0[v] * ib0, X1 = y1[v] * ib1;
-#pragma unroll
-        for (int t = 0; t < LT; ++t) {
-            CT x = d[v][t] - T.rca[t * 32 + lane] * X0 - T.rcc[t * 32 + lane] * X1;
-            if (t == 0) x = X0;
-            if (t != 0 && t == len - 1) x = X1;
-            d[v][t] = x;
-        }
-        if (T.cyclic) {
-            const CT last = len >= 2 ? X1 : X0;
-            const CT ya = __shfl_sync(0xffffffffu, X0, 0, W);
-            const CT yb = __shfl_sync(0xffffffffu, last, T.p - 1, W);
-            const CT beta = (ya + T.cyc_s2 * yb) * T.cyc_s1;
-#pragma unroll
-            for (int t = 0; t < LT; ++t) d[v][t] -= beta * T.cycz[t * 32 + lane];
-        }
-    }
-}
-
 // Per-row factors of a line whose lanes all share them: every chunk is full
 // (n a multiple of LT) and the matrix rows that shape a chunk's elimination
 // are the constant interior rows, as for the compact derivative with the
@@ -214,15 +123,35 @@ struct ChunkFactors {
 __device__ __forceinline__ float cf_fma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double cf_fma(double a, double b, double c) { return fma(a, b, c); }
 
-// warp_solve for lines with ChunkFactors (all chunks full, no cyclic
-// correction): NV right-hand sides held as d[v][t], FP32 or FP64.  The
-// structure of the tables fixes fwd2 = 0 for rows 0 and 1 of a chunk, bwd1 = 1
-// and bwd2 = 0 for row LT - 2, and bwd1 = 1 for rows 1 .. LT - 3; those
-// products are left out.  All 32 lanes must call it.
-template <int LT, int NV, typename CT, int W = 32>
-__device__ __forceinline__ void warp_solve_cf(const ChunkFactors<LT, CT> &U, const DevTables<CT> &T,
-                                              CT (&d)[NV][LT], int lane) {
-    static_assert(LT >= 2, "chunk");
+// The interior_chunk<LT> values as factors the compiler folds to immediates.
+template <int LT, typename CT>
+__device__ __forceinline__ ChunkFactors<LT, CT> interior_factors() {
+    constexpr InteriorChunk<LT> K = interior_chunk<LT>();
+    ChunkFactors<LT, CT> U{};
+#pragma unroll
+    for (int t = 0; t < LT; ++t) {
+        U.f1[t] = (CT)K.fwd1[t];
+        U.f2[t] = (CT)K.fwd2[t];
+        U.b1[t] = (CT)K.bwd1[t];
+        U.b2[t] = (CT)K.bwd2[t];
+        U.nra[t] = (CT)(-K.rca[t]);
+        U.nrc[t] = (CT)(-K.rcc[t]);
+    }
+    return U;
+}
+
+// ----------------------------------------------------------------------------
+// The three parts of the partitioned solve.  A chunk's rows may sit in a lane
+// of the warp that solves the line (warp_solve) or in a thread of a column
+// tile (column.cuh); the reduced system is always solved by one warp per line.
+// ----------------------------------------------------------------------------
+
+// 1. local elimination of chunk c's rows d[v][0 .. LT-1] (forward, then
+// backward sweep).  The structure of the tables fixes fwd2 = 0 for rows 0 and
+// 1 of a chunk, bwd1 = 1 and bwd2 = 0 for row LT - 2, and bwd1 = 1 for rows
+// 1 .. LT - 3; the form with shared factors leaves those products out.
+template <int LT, int NV, typename CT>
+__device__ __forceinline__ void chunk_eliminate_cf(const ChunkFactors<LT, CT> &U, CT (&d)[NV][LT]) {
 #pragma unroll
     for (int t = 0; t < LT; ++t)
 #pragma unroll
@@ -233,12 +162,40 @@ __device__ __forceinline__ void warp_solve_cf(const ChunkFactors<LT, CT> &U, con
 #pragma unroll
         for (int v = 0; v < NV; ++v)
             d[v][t] = t == 0 ? cf_fma(U.b2[0], d[v][1], U.b1[0] * d[v][0]) : cf_fma(U.b2[t], d[v][t + 1], d[v][t]);
-    CT y0[NV], y1[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        y0[v] = d[v][0];
-        y1[v] = d[v][LT - 1];
+}
+template <int LT, int NV, typename CT>
+__device__ __forceinline__ void chunk_eliminate(const DevTables<CT> &T, CT (&d)[NV][LT], int c) {
+    if (T.interior) {
+        chunk_eliminate_cf<LT, NV, CT>(interior_factors<LT, CT>(), d);
+        return;
     }
+#pragma unroll
+    for (int t = 0; t < LT; ++t) {
+        const CT f1 = T.fwd1[t * 32 + c];
+        if (t == 0) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) d[v][0] = f1 * d[v][0];
+        } else {
+            const CT f2 = T.fwd2[t * 32 + c];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) d[v][t] = f1 * d[v][t] + f2 * d[v][t - 1];
+        }
+    }
+#pragma unroll
+    for (int t = LT - 2; t >= 0; --t) {
+        const CT b1 = T.bwd1[t * 32 + c], b2 = T.bwd2[t * 32 + c];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) d[v][t] = b1 * d[v][t] + b2 * d[v][t + 1];
+    }
+}
+
+// 2. the reduced system: lane c holds the first and last eliminated rows
+// y0[v], y1[v] of chunk c and gets the solution there in their place.  All 32
+// lanes must call it (warp shuffles).  W < 32: every W lanes solve a line of
+// their own (lines with p <= W chunks and at most log2(W) + 1 PCR steps),
+// `lane` is the lane within its W-lane segment.
+template <int NV, typename CT, int W = 32>
+__device__ __forceinline__ void reduced_solve(const DevTables<CT> &T, CT (&y0)[NV], CT (&y1)[NV], int lane) {
     {
         const CT ka = T.k1[lane], kb = T.k2[lane], kc = T.k1[32 + lane], kd = T.k2[32 + lane];
 #pragma unroll
@@ -270,31 +227,84 @@ __device__ __forceinline__ void warp_solve_cf(const ChunkFactors<LT, CT> &U, con
     const CT ib0 = T.invb[lane], ib1 = T.invb[32 + lane];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        const CT X0 = y0[v] * ib0, X1 = y1[v] * ib1;
-        d[v][0] = X0;
-#pragma unroll
-        for (int t = 1; t + 1 < LT; ++t) d[v][t] = cf_fma(U.nrc[t], X1, cf_fma(U.nra[t], X0, d[v][t]));
-        d[v][LT - 1] = X1;
+        y0[v] = y0[v] * ib0;
+        y1[v] = y1[v] * ib1;
     }
 }
 
-// warp_solve for tables flagged `interior`: the per-row factors are the
-// compile-time interior_chunk<LT> values.
-template <int LT, int NV, typename CT, int W>
-__device__ __forceinline__ void warp_solve_interior(const DevTables<CT> &T, CT (&d)[NV][LT], int lane) {
-    if constexpr (LT >= 2) {
-        constexpr InteriorChunk<LT> K = interior_chunk<LT>();
-        ChunkFactors<LT, CT> U{};
+// 3. back-substitution of chunk c (len rows) from its end values X0, X1.
+template <int LT, typename CT>
+__device__ __forceinline__ void chunk_substitute_cf(const ChunkFactors<LT, CT> &U, CT (&d)[LT], CT X0, CT X1) {
+    d[0] = X0;
 #pragma unroll
-        for (int t = 0; t < LT; ++t) {
-            U.f1[t] = (CT)K.fwd1[t];
-            U.f2[t] = (CT)K.fwd2[t];
-            U.b1[t] = (CT)K.bwd1[t];
-            U.b2[t] = (CT)K.bwd2[t];
-            U.nra[t] = (CT)(-K.rca[t]);
-            U.nrc[t] = (CT)(-K.rcc[t]);
+    for (int t = 1; t + 1 < LT; ++t) d[t] = cf_fma(U.nrc[t], X1, cf_fma(U.nra[t], X0, d[t]));
+    d[LT - 1] = X1;
+}
+template <int LT, typename CT>
+__device__ __forceinline__ void chunk_substitute(const DevTables<CT> &T, CT (&d)[LT], CT X0, CT X1, int c, int len) {
+    if (T.interior) {
+        chunk_substitute_cf<LT, CT>(interior_factors<LT, CT>(), d, X0, X1);
+        return;
+    }
+#pragma unroll
+    for (int t = 0; t < LT; ++t) {
+        CT x = d[t] - T.rca[t * 32 + c] * X0 - T.rcc[t * 32 + c] * X1;
+        if (t == 0) x = X0;
+        if (t != 0 && t == len - 1) x = X1;
+        d[t] = x;
+    }
+}
+
+// warp_solve for lines with ChunkFactors (all chunks full, no cyclic
+// correction): NV right-hand sides held as d[v][t], FP32 or FP64.  All 32
+// lanes must call it.
+template <int LT, int NV, typename CT, int W = 32>
+__device__ __forceinline__ void warp_solve_cf(const ChunkFactors<LT, CT> &U, const DevTables<CT> &T,
+                                              CT (&d)[NV][LT], int lane) {
+    static_assert(LT >= 2, "chunk");
+    chunk_eliminate_cf<LT, NV, CT>(U, d);
+    CT y0[NV], y1[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        y0[v] = d[v][0];
+        y1[v] = d[v][LT - 1];
+    }
+    reduced_solve<NV, CT, W>(T, y0, y1, lane);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) chunk_substitute_cf<LT, CT>(U, d[v], y0[v], y1[v]);
+}
+
+// Solve NV right-hand sides held as d[v][t] by the lanes of one warp; the
+// solution overwrites d.  All 32 lanes must call it; W as reduced_solve.
+template <int LT, int NV, typename CT, int W = 32>
+__device__ __forceinline__ void warp_solve(const DevTables<CT> &T, CT (&d)[NV][LT], int lane) {
+    if (T.interior) {
+        warp_solve_cf<LT, NV, CT, W>(interior_factors<LT, CT>(), T, d, lane);
+        return;
+    }
+    const int len = lane_len(lane, LT, T.p, T.last_len);
+    chunk_eliminate<LT, NV, CT>(T, d, lane);
+    CT y0[NV], y1[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        y0[v] = d[v][0];
+        y1[v] = CT(0);
+#pragma unroll
+        for (int t = 1; t < LT; ++t)
+            if (t == len - 1) y1[v] = d[v][t];
+    }
+    reduced_solve<NV, CT, W>(T, y0, y1, lane);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        chunk_substitute<LT, CT>(T, d[v], y0[v], y1[v], lane, len);
+        if (T.cyclic) {
+            const CT last = len >= 2 ? y1[v] : y0[v];
+            const CT ya = __shfl_sync(0xffffffffu, y0[v], 0, W);
+            const CT yb = __shfl_sync(0xffffffffu, last, T.p - 1, W);
+            const CT beta = (ya + T.cyc_s2 * yb) * T.cyc_s1;
+#pragma unroll
+            for (int t = 0; t < LT; ++t) d[v][t] -= beta * T.cycz[t * 32 + lane];
         }
-        warp_solve_cf<LT, NV, CT, W>(U, T, d, lane);
     }
 }
 
@@ -497,6 +507,31 @@ __device__ __forceinline__ void deriv_rhs(const FT *f, int n, int lane, int nsta
             }
             if (lane == own_hi1) set_at<LT, CT>(d, (n - 1) - lane * LT, e1);
             if (lane == own_hi2) set_at<LT, CT>(d, (n - 2) - lane * LT, e2);
+        }
+    }
+}
+
+// Right-hand side of the compact derivative for chunk c from its window
+// w = f[c LT - 2 .. c LT + LT + 1]: interior rows, and the rows of the physical
+// closure where a face has it.  Window entries outside the line only reach
+// rows that are replaced (here, or by the caller for interface faces); rows
+// past the line's end are zero.
+template <int LT, typename CT>
+__device__ __forceinline__ void chunk_rhs(const CT (&w)[LT + 4], int c, int n, int nstart, int nend, CT (&d)[LT]) {
+    const int j0 = c * LT;
+#pragma unroll
+    for (int t = 0; t < LT; ++t)
+        d[t] = j0 + t < n ? xmul(CT(kAa), w[t + 3] - w[t + 1]) + xmul(CT(kBb), w[t + 4] - w[t]) : CT(0);
+    if (nstart == 0 && c == 0) {
+        d[0] = xmul(CT(kAb00), w[2]) + xmul(CT(kAb01), w[3]) + xmul(CT(kAb02), w[4]);
+        d[1] = xmul(CT(kAb10), w[4] - w[2]);
+    }
+    if (nend == 0 && j0 + LT >= n - 1) {
+#pragma unroll
+        for (int t = 0; t < LT; ++t) {
+            if (j0 + t == n - 1)
+                d[t] = -(xmul(CT(kAb00), w[t + 2]) + xmul(CT(kAb01), w[t + 1]) + xmul(CT(kAb02), w[t]));
+            if (j0 + t == n - 2) d[t] = xmul(-CT(kAb10), w[t + 1] - w[t + 3]);
         }
     }
 }

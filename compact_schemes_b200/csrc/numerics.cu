@@ -12,8 +12,8 @@
 #include <cstdio>
 #include <cstring>
 
+#include "column.cuh"
 #include "context.h"
-#include "tile.cuh"
 
 namespace csb {
 
@@ -238,134 +238,240 @@ __device__ __forceinline__ void store_line_regs(T *line, const T (&d)[LT], int l
         if (lane * LT + t < n) line[L::pos_ct(lane, t)] = d[t];
 }
 
-// Compact first derivative of one field along AXIS (deriv_kernel_1d/2d,
-// src/cuda/kernels/numerics_pc.hpp:124-249).
-template <int LT, int AXIS, typename T>
-__global__ void __launch_bounds__(kThreads)
-k_deriv(const T *__restrict__ in, T *__restrict__ out, DevTables<T> tab, int lxi, int let,
-        int nstart, int nend, const T *__restrict__ recv, T *__restrict__ drva, int64_t F, Coeffs cf) {
-    using L = LineLayout<LT>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sm = reinterpret_cast<T *>(smem_raw);
-    const int n = tab.n;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t line0 = (int64_t)blockIdx.x * kTileLines;
-    load_tile<LT, AXIS>(in, sm, line0, F, n, lxi, let);
-    if (AXIS == 0) __syncwarp();
-    else __syncthreads();
-    const int64_t fidx = line0 + w;
-    if (fidx < F) {
-        T d[1][LT];
-        T r4[4];
-        const T *rp = nullptr;
-        if (recv && (nstart || nend)) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) r4[k] = recv[k * F + fidx];
-            rp = r4;
-        }
-        T *line = sm + w * L::kSlot;
-        deriv_rhs<LT, T, T>(line, n, lane, nstart, nend, rp, cf, d[0]);
-        warp_solve<LT, 1, T>(tab, d, lane);
-        if (drva) {
-            if (lane == 0) drva[fidx] = d[0][0];
-            if (lane == (n - 1) / LT) drva[5 * F + fidx] = get_at<LT, T>(d[0], (n - 1) - lane * LT);
-        }
-        __syncwarp();
-        store_line_regs<LT, T>(line, d[0], lane, n);
-    }
-    if (AXIS == 0) __syncwarp();
-    else __syncthreads();
-    store_tile<LT, AXIS>(out, sm, line0, F, n, lxi, let);
-}
-
-// Same derivative with two lines per warp: a CTA of kThreads threads holds
-// kPairLines lines, warp w solves lines 2w and 2w+1 in one warp_solve (their
-// table loads and shuffle latencies are shared), and the y/z tiles cover 16
-// consecutive x positions (128-byte rows).  Used for chunks of up to 8 rows.
-constexpr int kPairLines = 16;
-#ifndef CSB_PAIR_MINB
-#define CSB_PAIR_MINB 3
-#endif
-
-template <int LT, int AXIS, typename T, bool STORE>
-__device__ __forceinline__ void pair_tile_io(const T *__restrict__ in, T *__restrict__ out, T *sm, int64_t line0,
-                                             int64_t F, int n, int lxi, int let) {
-    using L = LineLayout<LT>;
-    const int tid = threadIdx.x;
-    if (AXIS == 0) {
-        const int w = tid >> 5, lane = tid & 31;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int l = 2 * w + h;
-            const int64_t fidx = line0 + l;
-            if (fidx >= F) continue;
-            for (int j = lane; j < n; j += 32) {
-                if (STORE) out[fidx * n + j] = sm[l * L::kSlot + L::pos(j)];
-                else sm[l * L::kSlot + L::pos(j)] = in[fidx * n + j];
-            }
-        }
+// Vector access of VB bytes (16 or 32) to a lane's own chunk.
+template <int VB, typename T>
+__device__ __forceinline__ void load_vec(const T *p, T *v) {
+    if constexpr (VB == 32 && sizeof(T) == 8) {
+        asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p) : "memory");
+    } else if constexpr (VB == 32) {
+        asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+            : "l"(p) : "memory");
+    } else if constexpr (sizeof(T) == 8) {
+        const double2 x = *reinterpret_cast<const double2 *>(p);
+        v[0] = x.x; v[1] = x.y;
     } else {
-        const int l = tid % kPairLines;
-        const int64_t fidx = line0 + l;
-        if (fidx < F) {
-            const int64_t base = line_base<AXIS>(fidx, lxi, let), s = line_stride<AXIS>(lxi, let);
-            for (int j = tid / kPairLines; j < n; j += kThreads / kPairLines) {
-                if (STORE) out[base + j * s] = sm[l * L::kSlot + L::pos(j)];
-                else sm[l * L::kSlot + L::pos(j)] = in[base + j * s];
-            }
-        }
+        const float4 x = *reinterpret_cast<const float4 *>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    }
+}
+template <int VB, typename T>
+__device__ __forceinline__ void store_vec(T *p, const T *v) {
+    if constexpr (VB == 32 && sizeof(T) == 8) {
+        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                     : "memory");
+    } else if constexpr (VB == 32) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
+                     "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+    } else if constexpr (sizeof(T) == 8) {
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    } else {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
     }
 }
 
-template <int LT, int AXIS, typename T>
-__global__ void __launch_bounds__(kThreads, CSB_PAIR_MINB)
-k_deriv_pair(const T *__restrict__ in, T *__restrict__ out, DevTables<T> tab, int lxi, int let, int nstart,
-             int nend, const T *__restrict__ recv, T *__restrict__ drva, int64_t F, Coeffs cf) {
-    using L = LineLayout<LT>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sm = reinterpret_cast<T *>(smem_raw);
-    const int n = tab.n;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t line0 = (int64_t)blockIdx.x * kPairLines;
-    pair_tile_io<LT, AXIS, T, false>(in, nullptr, sm, line0, F, n, lxi, let);
-    if (AXIS == 0) __syncwarp();
-    else __syncthreads();
-    const int64_t fidx0 = line0 + 2 * w;
-    if (fidx0 < F) {
-        T d[2][LT];
+// The fields one derivative launch covers (blockIdx.y): field f is
+// in[f * in_fs + .] -> out[f * out_fs + .], line-end values at drva + f F and
+// received sums at recv + 4 f F (either may be null).
+template <typename T>
+struct FieldSet {
+    const T *in;
+    T *out;
+    const T *recv;
+    T *drva;
+    int64_t in_fs, out_fs;
+};
+
+// Compact first derivative along x (deriv_kernel_1d/2d,
+// src/cuda/kernels/numerics_pc.hpp:124-249) of rows whose length and start are
+// multiples of VB bytes: a warp solves NV neighbouring lines, each lane loading
+// its own chunks with VB-byte vectors and storing the solution from the same
+// registers.  Neighbouring points come by shuffle, and only the eight points
+// at either end of a line pass through shared memory (the interface sums).
+template <int LT, int NV, int VB, typename T>
+__global__ void __launch_bounds__(kThreads, LT <= 8 ? 3 : 1)
+k_deriv_row(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, Coeffs cf) {
+    constexpr int VE = VB / (int)sizeof(T);
+    __shared__ T ends[kThreads / 32][NV][2 * kLmd + 1];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31, j0 = lane * LT;
+    const int64_t line0 = ((int64_t)blockIdx.x * (kThreads / 32) + w) * NV;
+    if (line0 >= F) return;
+    const T *in = fs.in + blockIdx.y * fs.in_fs + line0 * n + j0;
+    T *out = fs.out + blockIdx.y * fs.out_fs + line0 * n + j0;
+    T d[NV][LT];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int64_t fidx = fidx0 + h;
-            if (fidx < F) {
-                T r4[4];
-                const T *rp = nullptr;
-                if (recv && (nstart || nend)) {
+    for (int h = 0; h < NV; ++h)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) r4[k] = recv[k * F + fidx];
-                    rp = r4;
-                }
-                deriv_rhs<LT, T, T>(sm + (2 * w + h) * L::kSlot, n, lane, nstart, nend, rp, cf, d[h]);
+        for (int t = 0; t < LT; t += VE) {
+            if (line0 + h < F && j0 + t < n) {
+                load_vec<VB, T>(in + (int64_t)h * n + t, &d[h][t]);
             } else {
 #pragma unroll
-                for (int t = 0; t < LT; ++t) d[h][t] = T(0);
+                for (int k = 0; k < VE; ++k) d[h][t + k] = T(0);
             }
         }
-        warp_solve<LT, 2, T>(tab, d, lane);
-        __syncwarp();
+    T rows = T(0);  // lane 8 h + {0, 1, 4, 5}: interface rows 0, 1, n-1, n-2 of line h
+    if (nstart || nend) {
+        if (j0 < kLmd || j0 + LT > n - kLmd) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int64_t fidx = fidx0 + h;
-            if (fidx >= F) continue;
-            if (drva) {
-                if (lane == 0) drva[fidx] = d[h][0];
-                if (lane == (n - 1) / LT) drva[5 * F + fidx] = get_at<LT, T>(d[h], (n - 1) - lane * LT);
+            for (int h = 0; h < NV; ++h)
+#pragma unroll
+                for (int t = 0; t < LT; ++t) {
+                    const int j = j0 + t;
+                    if (j < kLmd) ends[w][h][j] = d[h][t];
+                    if (j < n && j >= n - kLmd) ends[w][h][kLmd + n - 1 - j] = d[h][t];
+                }
+        }
+        __syncwarp();
+        const int h = lane >> 3, k8 = lane & 7;
+        T dv = T(0);
+        if (h < NV) {
+            const bool bci = k8 < 2 || k8 == 4 || k8 == 5, asc = k8 < 2 || k8 >= 6, second = (k8 & 1) != 0;
+            if (fs.recv && (k8 & 2)) {
+                if (line0 + h < F)
+                    dv = fs.recv[((int64_t)blockIdx.y * 4 + ((k8 >> 1 & 2) | (k8 & 1))) * F + line0 + h];
+            } else {
+#pragma unroll
+                for (int k = 0; k < kLmd; ++k) {
+                    const double c = bci ? (second ? cf.pbci[kLmd + k] : cf.pbci[k])
+                                         : (second ? cf.pbco[kLmd + k] : cf.pbco[k]);
+                    dv += xmul(T(c), ends[w][h][asc ? k : kLmd + k]);
+                }
             }
-            store_line_regs<LT, T>(sm + (2 * w + h) * L::kSlot, d[h], lane, n);
+        }
+        rows = dv + __shfl_down_sync(0xffffffffu, dv, 2);
+    }
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        T x[LT + 4];
+        x[0] = __shfl_up_sync(0xffffffffu, d[h][LT - 2], 1);
+        x[1] = __shfl_up_sync(0xffffffffu, d[h][LT - 1], 1);
+        x[LT + 2] = __shfl_down_sync(0xffffffffu, d[h][0], 1);
+        x[LT + 3] = __shfl_down_sync(0xffffffffu, d[h][1], 1);
+#pragma unroll
+        for (int t = 0; t < LT; ++t) x[t + 2] = d[h][t];
+        T own2[2] = {T(0), T(0)};
+        if (nstart || nend) take_closure_rows(rows, h, lane, own2);
+        chunk_rhs<LT, T>(x, lane, n, nstart, nend, d[h]);
+        if (nstart && lane == 0) {
+            d[h][0] = own2[0];
+            d[h][1] = own2[1];
+        }
+        if (nend) {
+            if (lane == (n - 1) / LT) set_at<LT, T>(d[h], (n - 1) - j0, -own2[0]);
+            if (lane == (n - 2) / LT) set_at<LT, T>(d[h], (n - 2) - j0, -own2[1]);
         }
     }
-    if (AXIS == 0) __syncwarp();
-    else __syncthreads();
-    pair_tile_io<LT, AXIS, T, true>(nullptr, out, sm, line0, F, n, lxi, let);
+    warp_solve<LT, NV, T>(tab, d, lane);
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        if (line0 + h >= F) break;
+        if (fs.drva) {
+            T *dr = fs.drva + blockIdx.y * F + line0 + h;
+            if (lane == 0) dr[0] = d[h][0];
+            if (lane == (n - 1) / LT) dr[5 * F] = get_at<LT, T>(d[h], (n - 1) - j0);
+        }
+#pragma unroll
+        for (int t = 0; t < LT; t += VE)
+            if (j0 + t < n) store_vec<VB, T>(out + (int64_t)h * n + t, &d[h][t]);
+    }
+}
+
+// The same for x rows of any length and start: a warp stages NV lines in
+// shared memory (LineLayout) with 256-byte coalesced accesses and solves them
+// from there.
+template <int LT, int NV, typename T>
+__global__ void __launch_bounds__(kThreads, LT <= 8 ? 3 : 1)
+k_deriv_row_any(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, Coeffs cf) {
+    using L = LineLayout<LT>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    T *sm = reinterpret_cast<T *>(smem_raw) + w * NV * L::kSlot;
+    const int64_t line0 = ((int64_t)blockIdx.x * (kThreads / 32) + w) * NV;
+    if (line0 >= F) return;
+    const T *in = fs.in + blockIdx.y * fs.in_fs + line0 * n;
+    T *out = fs.out + blockIdx.y * fs.out_fs + line0 * n;
+    const int nl = F - line0 < NV ? (int)(F - line0) : NV;
+    for (int h = 0; h < nl; ++h)
+        for (int j = lane; j < n; j += 32) sm[h * L::kSlot + L::pos(j)] = in[(int64_t)h * n + j];
+    __syncwarp();
+    T d[NV][LT];
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        if (h < nl) {
+            T r4[4];
+            const T *rp = nullptr;
+            if (fs.recv && (nstart || nend)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r4[k] = fs.recv[((int64_t)blockIdx.y * 4 + k) * F + line0 + h];
+                rp = r4;
+            }
+            deriv_rhs<LT, T, T>(sm + h * L::kSlot, n, lane, nstart, nend, rp, cf, d[h]);
+        } else {
+#pragma unroll
+            for (int t = 0; t < LT; ++t) d[h][t] = T(0);
+        }
+    }
+    warp_solve<LT, NV, T>(tab, d, lane);
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        if (h >= nl) break;
+        if (fs.drva) {
+            T *dr = fs.drva + blockIdx.y * F + line0 + h;
+            if (lane == 0) dr[0] = d[h][0];
+            if (lane == (n - 1) / LT) dr[5 * F] = get_at<LT, T>(d[h], (n - 1) - lane * LT);
+        }
+        store_line_regs<LT, T>(sm + h * L::kSlot, d[h], lane, n);
+    }
+    __syncwarp();
+    for (int h = 0; h < nl; ++h)
+        for (int j = lane; j < n; j += 32) out[(int64_t)h * n + j] = sm[h * L::kSlot + L::pos(j)];
+}
+
+// The same along y and z: a column tile of TL lines (column.cuh).
+template <int LT, int AXIS, int TL, typename T>
+__global__ void __launch_bounds__(TL * 32, LT <= 8 ? 1024 / (TL * 32) : (LT == 16 ? 2 : 1))
+k_deriv_col(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int nend, int64_t F, Coeffs cf) {
+    using C = Column<LT, TL>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *V = reinterpret_cast<T *>(smem_raw), *rows = V + C::kField;
+    const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL, j0 = c * LT;
+    const int len = lane_len(c, LT, tab.p, tab.last_len);
+    const int64_t line0 = (int64_t)blockIdx.x * TL, fidx = line0 + l;
+    const bool ok = fidx < F;
+    const int64_t s = line_stride<AXIS>(lxi, let), base = line_base<AXIS>(fidx, lxi, let) + j0 * s;
+    const T *in = fs.in + blockIdx.y * fs.in_fs + base;
+    T d[1][LT];
+#pragma unroll
+    for (int t = 0; t < LT; ++t) d[0][t] = ok && t < len ? in[t * s] : T(0);
+    const bool near_end = j0 < kLmd || j0 + LT > n - kLmd;
+#pragma unroll
+    for (int t = 0; t < LT; ++t)
+        if (t < 2 || t >= LT - 2 || near_end) V[C::at(t, c, l)] = d[0][t];
+    __syncthreads();
+    if (nstart || nend)
+        column_closure_rows<LT, TL, 1, T>(V, rows, n, cf, fs.recv ? fs.recv + blockIdx.y * 4 * F : nullptr, F, line0);
+    column_rhs<LT, TL, T>(V, c, l, n, nstart, nend, d[0]);
+    __syncthreads();
+    column_take_rows<LT, T>(rows + 4 * l, c, n, nstart, nend, d[0]);
+    chunk_eliminate<LT, 1, T>(tab, d, c);
+    column_put_ends<LT, TL, T>(V, d[0], c, l, len);
+    __syncthreads();
+    column_reduced<LT, TL, 1, T>(V, tab, F, line0, nullptr);
+    __syncthreads();
+    column_finish<LT, TL, T>(V, tab, c, l, len, d[0]);
+    if (!ok) return;
+    if (fs.drva) {
+        T *dr = fs.drva + blockIdx.y * F + fidx;
+        if (c == 0) dr[0] = d[0][0];
+        if (c == (n - 1) / LT) dr[5 * F] = get_at<LT, T>(d[0], (n - 1) - j0);
+    }
+    T *out = fs.out + blockIdx.y * fs.out_fs + base;
+#pragma unroll
+    for (int t = 0; t < LT; ++t)
+        if (t < len) out[t * s] = d[0][t];
 }
 
 // Compact filter of one field along AXIS.
@@ -433,42 +539,61 @@ static int prep_smem(KernelT kern, size_t bytes) {
     return CS_OK;
 }
 
+#ifndef CSB_COL_TL
+#define CSB_COL_TL 8
+#endif
+
 template <int LT, int AXIS, typename T>
-static int launch_deriv_lt(const T *in, T *out, const DevTables<T> &tab, const cs_dcomp &d,
-                           int nstart, int nend, const T *recv, T *drva, const Coeffs &cf,
-                           cudaStream_t st) {
+static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d, int nstart,
+                           int nend, const Coeffs &cf, cudaStream_t st) {
     const int64_t F = face_size(d, AXIS);
-    if constexpr (LT <= 8) {
-        const size_t smem = (size_t)kPairLines * LineLayout<LT>::kSlot * sizeof(T);
-        auto kern = k_deriv_pair<LT, AXIS, T>;
+    if constexpr (AXIS == 0) {
+        constexpr int NV = LT <= 8 ? 2 : 1, WARPS = kThreads / 32;
+        const dim3 grid((unsigned)((F + NV * WARPS - 1) / (NV * WARPS)), (unsigned)nf);
+        auto aligned = [&](int vb) {
+            const int64_t ve = vb / (int)sizeof(T);
+            return LT % ve == 0 && d.lxi % ve == 0 && (nf == 1 || (fs.in_fs % ve == 0 && fs.out_fs % ve == 0)) &&
+                   reinterpret_cast<uintptr_t>(fs.in) % vb == 0 && reinterpret_cast<uintptr_t>(fs.out) % vb == 0;
+        };
+        if constexpr (LT * sizeof(T) >= 32) {
+            if (aligned(32)) {
+                k_deriv_row<LT, NV, 32, T><<<grid, kThreads, 0, st>>>(fs, tab, nstart, nend, F, cf);
+                CSB_CUDA(cudaGetLastError());
+                return CS_OK;
+            }
+        }
+        if constexpr (LT * sizeof(T) >= 16) {
+            if (aligned(16)) {
+                k_deriv_row<LT, NV, 16, T><<<grid, kThreads, 0, st>>>(fs, tab, nstart, nend, F, cf);
+                CSB_CUDA(cudaGetLastError());
+                return CS_OK;
+            }
+        }
+        const size_t smem = (size_t)NV * WARPS * LineLayout<LT>::kSlot * sizeof(T);
+        auto kern = k_deriv_row_any<LT, NV, T>;
         if (int rc = prep_smem(kern, smem)) return rc;
-        const int64_t blocks = (F + kPairLines - 1) / kPairLines;
-        kern<<<(unsigned)blocks, kThreads, smem, st>>>(in, out, tab, d.lxi, d.let, nstart, nend, recv, drva, F,
-                                                      cf);
-        CSB_CUDA(cudaGetLastError());
-        return CS_OK;
+        kern<<<grid, kThreads, smem, st>>>(fs, tab, nstart, nend, F, cf);
+    } else {
+        constexpr int TL = CSB_COL_TL;
+        const size_t smem = (size_t)(Column<LT, TL>::kField + 4 * TL) * sizeof(T);
+        auto kern = k_deriv_col<LT, AXIS, TL, T>;
+        if (int rc = prep_smem(kern, smem)) return rc;
+        kern<<<dim3((unsigned)((F + TL - 1) / TL), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
+            fs, tab, d.lxi, d.let, nstart, nend, F, cf);
     }
-    const size_t smem = (size_t)kTileLines * LineLayout<LT>::kSlot * sizeof(T);
-    auto kern = k_deriv<LT, AXIS, T>;
-    int rc = prep_smem(kern, smem);
-    if (rc) return rc;
-    const int64_t blocks = (F + kTileLines - 1) / kTileLines;
-    kern<<<(unsigned)blocks, kThreads, smem, st>>>(in, out, tab, d.lxi, d.let, nstart, nend, recv,
-                                                  drva, F, cf);
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
 }
 
 template <int AXIS, typename T>
-static int launch_deriv_axis(int lt, const T *in, T *out, const DevTables<T> &tab, const cs_dcomp &d,
-                             int nstart, int nend, const T *recv, T *drva, const Coeffs &cf,
-                             cudaStream_t st) {
+static int launch_deriv_axis(int lt, const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d,
+                             int nstart, int nend, const Coeffs &cf, cudaStream_t st) {
     switch (lt) {
-        case 2: return launch_deriv_lt<2, AXIS, T>(in, out, tab, d, nstart, nend, recv, drva, cf, st);
-        case 4: return launch_deriv_lt<4, AXIS, T>(in, out, tab, d, nstart, nend, recv, drva, cf, st);
-        case 8: return launch_deriv_lt<8, AXIS, T>(in, out, tab, d, nstart, nend, recv, drva, cf, st);
-        case 16: return launch_deriv_lt<16, AXIS, T>(in, out, tab, d, nstart, nend, recv, drva, cf, st);
-        case 32: return launch_deriv_lt<32, AXIS, T>(in, out, tab, d, nstart, nend, recv, drva, cf, st);
+        case 2: return launch_deriv_lt<2, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
+        case 4: return launch_deriv_lt<4, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
+        case 8: return launch_deriv_lt<8, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
+        case 16: return launch_deriv_lt<16, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
+        case 32: return launch_deriv_lt<32, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
     }
     return set_error(CS_ERR_UNSUPPORTED, "chunk length %d", lt);
 }
@@ -540,14 +665,13 @@ static int deriv_impl(cs_numerics *nm, int axis, const T *in, T *out, int nstart
     } else if (halo == CS_HALO_RECV && (nstart || nend)) {
         return set_error(CS_ERR_UNSUPPORTED, "FP32 derivative supports CS_HALO_SELF only");
     }
-    const T *src = in + (int64_t)comp * d.lmx;
-    T *dst = out + (int64_t)slot * d.lmx;
+    const FieldSet<T> fs{in + (int64_t)comp * d.lmx, out + (int64_t)slot * d.lmx, recv, drva, 0, 0};
     cudaStream_t st = (cudaStream_t)stream;
     const DevTables<T> &tab = pick_tables<T>(*dt);
     switch (axis) {
-        case 0: return launch_deriv_axis<0, T>(dt->lt, src, dst, tab, d, nstart, nend, recv, drva, nm->cf, st);
-        case 1: return launch_deriv_axis<1, T>(dt->lt, src, dst, tab, d, nstart, nend, recv, drva, nm->cf, st);
-        default: return launch_deriv_axis<2, T>(dt->lt, src, dst, tab, d, nstart, nend, recv, drva, nm->cf, st);
+        case 0: return launch_deriv_axis<0, T>(dt->lt, fs, 1, tab, d, nstart, nend, nm->cf, st);
+        case 1: return launch_deriv_axis<1, T>(dt->lt, fs, 1, tab, d, nstart, nend, nm->cf, st);
+        default: return launch_deriv_axis<2, T>(dt->lt, fs, 1, tab, d, nstart, nend, nm->cf, st);
     }
 }
 

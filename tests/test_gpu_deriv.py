@@ -105,6 +105,35 @@ def test_deriv2d_recv_path_and_drva(cuda, dims):
                           drva[5 * F + m * F:5 * F + (m + 1) * F]) < TOL
 
 
+@pytest.mark.parametrize("closure", [45, 10])
+@pytest.mark.parametrize("n", [8, 10, 12, 33, 34, 64, 66, 68, 127, 132, 255, 256, 260, 514, 1000, 1024])
+def test_deriv_row_and_column_lengths(cuda, n, closure):
+    """Line lengths around the chunk, tile and vector-access edges, along every
+    axis, with field starts on and off a 16-byte boundary (the x rows' vector
+    and staged paths): FP64 within the parity bar, FP32 within 2e-6."""
+    import torch
+    import compact_schemes_b200 as cs
+    nd = int(closure == 45)
+    coeffs = O.deriv_setup()
+    for axis in range(3):
+        dims = [9, 8, 10]
+        dims[axis] = n
+        nm = make(cuda, tuple(dims), [[closure] * 3] * 2)
+        f = field(dims, 3)
+        ref = O.deriv(f, dims, axis, nd, nd, coeffs=coeffs)
+        for off in (0, 1, 2):
+            for dt, tol in ((torch.float64, TOL), (torch.float32, 2e-6)):
+                buf = torch.zeros(f.size + off, dtype=dt, device=cuda)
+                out = torch.full((f.size + off + 5,), 7.0, dtype=dt, device=cuda)
+                buf[off:] = torch.from_numpy(f).to(cuda).to(dt)
+                want = ref if dt == torch.float64 else O.deriv(buf[off:].double().cpu().numpy(), dims, axis, nd, nd,
+                                                               coeffs=coeffs)
+                nm.deriv1d(axis, buf[off:], out[off:], nd, nd, nm.dcomp, 0, halo=cs.HALO_SELF)
+                assert relerr(out[off:off + f.size].double().cpu().numpy(), want) < tol, (axis, off, dt)
+                assert bool((out[:off] == 7.0).all()) and bool((out[off + f.size:] == 7.0).all())
+        nm.close()
+
+
 def test_deriv_fp32(cuda):
     import torch
     import compact_schemes_b200 as cs
