@@ -39,18 +39,19 @@ inline int column_threads(int tl, int p) { return (tl * p + 31) / 32 * 32; }
 // 1, n-1, n-2 of the right-hand side (the last two without their sign).  Eight
 // neighbouring threads form the eight 8-term sums of one line (interface_sum's
 // operations), then two of them are added.  recv != nullptr: the far-end sums
-// are received values recv[k F + line] instead.  All threads of the tile call
-// it; the caller synchronizes before the rows are read.
-template <int LT, int TL, int NF, typename T>
-__device__ __forceinline__ void column_closure_rows(const T *V, T *rows, int n, const Coeffs &cf, const T *recv,
-                                                    int64_t F, int64_t line0) {
+// are received values recv[k F + line0 + f TL + l] instead (the fields are then
+// TL-line groups of one field).  CT: type the sums are formed in.  All threads of the tile call it; the caller
+// synchronizes before the rows are read.
+template <int LT, int TL, int NF, typename T, typename CT = T>
+__device__ __forceinline__ void column_closure_rows(const T *V, CT *rows, int n, const Coeffs &cf, const CT *recv,
+                                                    int F, int line0) {
     using C = Column<LT, TL>;
     static_assert(NF * TL * 8 % 32 == 0, "whole warps");
     for (int i = threadIdx.x; i < NF * TL * 8; i += blockDim.x) {
         const int g = i >> 3, d = i & 7, f = g / TL, l = g % TL;
-        T dv = T(0);
+        CT dv = CT(0);
         if (recv && (d & 2)) {
-            if (line0 + l < F) dv = recv[(int64_t)((d >> 1 & 2) | (d & 1)) * F + line0 + l];
+            if (line0 + g < F) dv = recv[(int64_t)((d >> 1 & 2) | (d & 1)) * F + line0 + g];
         } else {
             const bool bci = d < 2 || d == 4 || d == 5, asc = d < 2 || d >= 6, second = (d & 1) != 0;
             const T *line = V + f * C::kField;
@@ -58,21 +59,37 @@ __device__ __forceinline__ void column_closure_rows(const T *V, T *rows, int n, 
             for (int k = 0; k < kLmd; ++k) {
                 const double w = bci ? (second ? cf.pbci[kLmd + k] : cf.pbci[k])
                                      : (second ? cf.pbco[kLmd + k] : cf.pbco[k]);
-                dv += xmul(T(w), line[C::pos(asc ? k : n - 1 - k, l)]);
+                dv += xmul(CT(w), CT(line[C::pos(asc ? k : n - 1 - k, l)]));
             }
         }
-        const T x = dv + __shfl_down_sync(0xffffffffu, dv, 2);
+        const CT x = dv + __shfl_down_sync(0xffffffffu, dv, 2);
         if (!(d & 2)) rows[g * 4 + ((d >> 2) * 2 | (d & 1))] = x;
     }
 }
 
-// Right-hand side of the compact derivative for this thread's chunk: d holds
-// its field values on entry; the two points on either side come from V.  Rows
-// of the physical closure are formed here; rows of the interface closure are
-// put in by column_take_rows once column_closure_rows has run.  Slots outside
-// the line are read but only reach rows that are replaced.
+// Write the rows of a chunk that other threads read: the two at either end
+// (the neighbours' stencils), all of them near the line's ends (the closure).
 template <int LT, int TL, typename T>
-__device__ __forceinline__ void column_rhs(const T *V, int c, int l, int n, int nstart, int nend, T (&d)[LT]) {
+__device__ __forceinline__ void column_put_raw(T *V, const T (&d)[LT], int c, int l, int n) {
+    using C = Column<LT, TL>;
+    V[C::at(0, c, l)] = d[0];
+    V[C::at(1, c, l)] = d[1];
+    if (LT > 2) V[C::at(LT - 2, c, l)] = d[LT - 2];
+    if (LT > 3) V[C::at(LT - 1, c, l)] = d[LT - 1];
+    if (LT > 4 && (c * LT < kLmd || (c + 1) * LT > n - kLmd)) {
+#pragma unroll
+        for (int t = 2; t < LT - 2; ++t) V[C::at(t, c, l)] = d[t];
+    }
+}
+
+// Right-hand side of the compact derivative for this thread's chunk (len rows):
+// d holds its field values on entry; the two points on either side come from V.
+// Rows of the physical closure are formed here; rows of the interface closure
+// are put in by column_take_rows once column_closure_rows has run.  Slots
+// outside the line are read but only reach rows that are replaced.
+template <int LT, int TL, typename T>
+__device__ __forceinline__ void column_rhs(const T *V, int c, int l, int len, int n, int nstart, int nend,
+                                           T (&d)[LT]) {
     using C = Column<LT, TL>;
     const int cm = c > 0 ? c - 1 : 0, cp = c < 31 ? c + 1 : 31;
     T w[LT + 4];
@@ -82,55 +99,46 @@ __device__ __forceinline__ void column_rhs(const T *V, int c, int l, int n, int 
     w[LT + 3] = V[C::at(1, cp, l)];
 #pragma unroll
     for (int t = 0; t < LT; ++t) w[t + 2] = d[t];
-    chunk_rhs<LT, T>(w, c, n, nstart, nend, d);
+    chunk_rhs<LT, T>(w, c, len, n, nstart, nend, d);
 }
 
-// Put the interface closure rows of line l (rows: its four entries) into d.
+// Put the interface closure rows of a line (rows: its four entries) into d.
 template <int LT, typename T>
 __device__ __forceinline__ void column_take_rows(const T *rows, int c, int n, int nstart, int nend, T (&d)[LT]) {
-    if (nstart && c == 0) {
-        d[0] = rows[0];
-        d[1] = rows[1];
-    }
-    if (nend) {
-        if (c == (n - 1) / LT) set_at<LT, T>(d, (n - 1) - c * LT, -rows[2]);
-        if (c == (n - 2) / LT) set_at<LT, T>(d, (n - 2) - c * LT, -rows[3]);
-    }
+    if (c == 0 || (c + 1) * LT >= n - 1)
+        chunk_take_rows<LT, T>(rows[0], rows[1], rows[2], rows[3], c, n, nstart, nend, d);
 }
 
 // Write an eliminated chunk's end rows where the line's warp reads them.
 template <int LT, int TL, typename T>
 __device__ __forceinline__ void column_put_ends(T *V, const T (&d)[LT], int c, int l, int len) {
     using C = Column<LT, TL>;
-    if (len == LT) {
-        V[C::at(0, c, l)] = d[0];
-        V[C::at(LT - 1, c, l)] = d[LT - 1];
-    } else if (len > 0) {
-        V[C::at(0, c, l)] = d[0];
-        if (len >= 2) V[C::at(len - 1, c, l)] = get_at<LT, T>(d, len - 1);
-    }
+    V[C::at(0, c, l)] = d[0];
+    if (len == LT) V[C::at(LT - 1, c, l)] = d[LT - 1];
+    else if (len >= 2) V[C::at(len - 1, c, l)] = get_at<LT, T>(d, len - 1);
 }
 
-// Solve the reduced systems of the tile's lines, one warp per line, in place
-// of the chunks' end rows.  beta != nullptr (cyclic systems): the factor of
-// the Sherman-Morrison correction per field and line.
+// Solve the reduced systems of the tile's lines, one warp per line (all NF
+// fields of it together), in place of the chunks' end rows.  beta != nullptr
+// (cyclic systems): the factor of the Sherman-Morrison correction per field and
+// line.
 template <int LT, int TL, int NF, typename T>
-__device__ __forceinline__ void column_reduced(T *V, const DevTables<T> &tab, int64_t F, int64_t line0, T *beta) {
+__device__ __forceinline__ void column_reduced(T *V, const DevTables<T> &tab, T *beta = nullptr) {
     using C = Column<LT, TL>;
     const int lane = threadIdx.x & 31, len = lane_len(lane, LT, tab.p, tab.last_len);
     for (int l = threadIdx.x >> 5; l < TL; l += blockDim.x >> 5) {
-        if (line0 + l >= F) break;
+        T *lo = V + C::at(0, lane, l), *hi = V + C::at(len >= 2 ? len - 1 : 0, lane, l);
         T y0[NF], y1[NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-            y0[f] = len >= 1 ? V[f * C::kField + C::at(0, lane, l)] : T(0);
-            y1[f] = len >= 2 ? V[f * C::kField + C::at(len - 1, lane, l)] : T(0);
+            y0[f] = len >= 1 ? lo[f * C::kField] : T(0);
+            y1[f] = len >= 2 ? hi[f * C::kField] : T(0);
         }
         reduced_solve<NF, T>(tab, y0, y1, lane);
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-            if (len >= 1) V[f * C::kField + C::at(0, lane, l)] = y0[f];
-            if (len >= 2) V[f * C::kField + C::at(len - 1, lane, l)] = y1[f];
+            if (len >= 1) lo[f * C::kField] = y0[f];
+            if (len >= 2) hi[f * C::kField] = y1[f];
             if (beta) {
                 const T ya = __shfl_sync(0xffffffffu, y0[f], 0);
                 const T yb = __shfl_sync(0xffffffffu, len >= 2 ? y1[f] : y0[f], tab.p - 1);
@@ -144,9 +152,65 @@ __device__ __forceinline__ void column_reduced(T *V, const DevTables<T> &tab, in
 template <int LT, int TL, typename T>
 __device__ __forceinline__ void column_finish(const T *V, const DevTables<T> &tab, int c, int l, int len, T (&d)[LT]) {
     using C = Column<LT, TL>;
-    const T X0 = len >= 1 ? V[C::at(0, c, l)] : T(0);
-    const T X1 = len >= 2 ? V[C::at(len - 1, c, l)] : T(0);
+    const T X0 = V[C::at(0, c, l)];
+    const T X1 = V[C::at(len >= 2 ? len - 1 : 0, c, l)];
     chunk_substitute<LT, T>(tab, d, X0, X1, c, len);
+}
+
+// ----------------------------------------------------------------------------
+// Lines of 65 to 128 points, one field at a time: four neighbouring lines per
+// warp, lane 4 c + l holding chunk c (16 rows, at most 8 chunks) of line l in
+// registers.  A row of the tile is one 32-byte sector; neighbours and the
+// reduced system go by shuffle, so a warp needs no other warp and no barrier,
+// and the reduced system takes 3 steps on an eighth of the rows.
+// ----------------------------------------------------------------------------
+constexpr int kWarpLines = 4;
+constexpr int kWarpChunk = 16;
+// Measured on B200 (transposed derivative, 4.5 fields of 128^3): 53 us against
+// 72 us for the column tiles.  Shorter lines leave too few rows per lane to pay
+// for its serial sweeps (64^3: 5.8 us against 4.9 us), longer ones need 32-row
+// chunks, whose registers allow only 16 warps per SM (256^3: 83 against 78 us).
+__host__ __device__ constexpr bool warp_column(int n) { return n > 64 && n <= 8 * kWarpChunk; }
+
+// Right-hand side of a lane's chunk from its field values d; ends: this warp's
+// [4][17] end points in shared memory; far: the received far-end sum that this
+// lane's closure sum uses instead (or null).
+template <int LT, typename T>
+__device__ __forceinline__ void warp_column_rhs(T (*ends)[2 * kLmd + 1], int lane, int len, int n, int nstart, int nend,
+                                                const Coeffs &cf, const T *far, T (&d)[1][LT]) {
+    const int c = lane / kWarpLines, l = lane % kWarpLines;
+    T rows = T(0);
+    if (nstart || nend) {
+        chunk_put_ends<LT, 1, T>(ends + l, d, c, len, n);
+        __syncwarp();
+        rows = ends_closure_row<T>(ends[lane >> 3], lane & 7, cf, far);
+    }
+    T x[LT + 4];
+    x[0] = __shfl_up_sync(0xffffffffu, d[0][LT - 2], kWarpLines);
+    x[1] = __shfl_up_sync(0xffffffffu, d[0][LT - 1], kWarpLines);
+    x[LT + 2] = __shfl_down_sync(0xffffffffu, d[0][0], kWarpLines);
+    x[LT + 3] = __shfl_down_sync(0xffffffffu, d[0][1], kWarpLines);
+#pragma unroll
+    for (int t = 0; t < LT; ++t) x[t + 2] = d[0][t];
+    chunk_rhs<LT, T>(x, c, len, n, nstart, nend, d[0]);
+    if (nstart || nend) {
+        // all four: a short line's first chunk can hold its last rows too
+        const T r0 = __shfl_sync(0xffffffffu, rows, 8 * l), r1 = __shfl_sync(0xffffffffu, rows, 8 * l + 1);
+        const T r2 = __shfl_sync(0xffffffffu, rows, 8 * l + 4), r3 = __shfl_sync(0xffffffffu, rows, 8 * l + 5);
+        chunk_take_rows<LT, T>(r0, r1, r2, r3, c, n, nstart, nend, d[0]);
+    }
+}
+
+// Solve the four lines of the warp in place.
+template <int LT, typename T>
+__device__ __forceinline__ void warp_column_solve(const DevTables<T> &tab, int lane, int len, T (&d)[1][LT]) {
+    const int c = lane / kWarpLines;
+    chunk_eliminate<LT, 1, T>(tab, d, c);
+    T y0[1] = {d[0][0]}, y1[1];
+    if (len == LT) y1[0] = d[0][LT - 1];
+    else y1[0] = len >= 2 ? get_at<LT, T>(d[0], len - 1) : T(0);
+    reduced_solve<1, T, 32, kWarpLines>(tab, y0, y1, c);
+    chunk_substitute<LT, T>(tab, d[0], y0[0], y1[0], c, len);
 }
 
 }  // namespace csb

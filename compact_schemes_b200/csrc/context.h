@@ -66,3 +66,27 @@ struct cs_numerics {
     double *recv[3] = {nullptr, nullptr, nullptr};
     csb::TableCache tables;
 };
+
+namespace csb {
+
+// sum[f] = (add0[f] + add1[f]) + the derivative of field f, formed by the
+// derivative's own launch (fields f add_fs / sum_fs apart).
+struct DerivSum {
+    const double *add0 = nullptr, *add1 = nullptr;
+    double *sum = nullptr;
+    int64_t add_fs = 0, sum_fs = 0;
+};
+
+// Several fields of a single-rank block at once (numerics.cu), with the face
+// closures, the received sums and the line-end buffers of the numerics object,
+// variables var .. var + nf - 1.
+// nf derivatives along `axis`: in + f in_fs -> out + f out_fs; sum (z only, may
+// be null) adds them up.
+int deriv_fields(cs_numerics *nm, int axis, const double *in, int64_t in_fs, double *out, int64_t out_fs, int nf,
+                 unsigned var, const DerivSum *sum, cudaStream_t st);
+// Interface sums of all faces into the send buffers and, exchanged, into the
+// receive buffers: variable f's field for axis a is in + f fs + a comp_fs.
+int exchange_self(cs_numerics *nm, const double *in, int64_t fs, int64_t comp_fs, int nf, unsigned var,
+                  cudaStream_t st);
+
+}  // namespace csb

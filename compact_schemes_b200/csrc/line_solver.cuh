@@ -193,15 +193,16 @@ __device__ __forceinline__ void chunk_eliminate(const DevTables<CT> &T, CT (&d)[
 // y0[v], y1[v] of chunk c and gets the solution there in their place.  All 32
 // lanes must call it (warp shuffles).  W < 32: every W lanes solve a line of
 // their own (lines with p <= W chunks and at most log2(W) + 1 PCR steps),
-// `lane` is the lane within its W-lane segment.
-template <int NV, typename CT, int W = 32>
+// `lane` is the lane within its W-lane segment.  S > 1: chunk c of line l sits
+// in warp lane c S + l (S lines of at most 32 / S chunks), `lane` is c.
+template <int NV, typename CT, int W = 32, int S = 1>
 __device__ __forceinline__ void reduced_solve(const DevTables<CT> &T, CT (&y0)[NV], CT (&y1)[NV], int lane) {
     {
         const CT ka = T.k1[lane], kb = T.k2[lane], kc = T.k1[32 + lane], kd = T.k2[32 + lane];
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            const CT up1 = __shfl_up_sync(0xffffffffu, y1[v], 1, W);
-            const CT dn0 = __shfl_down_sync(0xffffffffu, y0[v], 1, W);
+            const CT up1 = __shfl_up_sync(0xffffffffu, y1[v], S, W);
+            const CT dn0 = __shfl_down_sync(0xffffffffu, y0[v], S, W);
             const CT n0 = y0[v] - ka * up1 - kb * y1[v];
             const CT n1 = y1[v] - kc * y0[v] - kd * dn0;
             y0[v] = n0;
@@ -211,7 +212,7 @@ __device__ __forceinline__ void reduced_solve(const DevTables<CT> &T, CT (&y0)[N
 #pragma unroll
     for (int s = 1; s < kPcrSteps; ++s) {
         if (s >= T.pcr) break;
-        const int dl = 1 << (s - 1);
+        const int dl = S << (s - 1);
         const CT ka = T.k1[s * 64 + lane], kb = T.k2[s * 64 + lane];
         const CT kc = T.k1[s * 64 + 32 + lane], kd = T.k2[s * 64 + 32 + lane];
 #pragma unroll
@@ -253,6 +254,19 @@ __device__ __forceinline__ void chunk_substitute(const DevTables<CT> &T, CT (&d)
         if (t != 0 && t == len - 1) x = X1;
         d[t] = x;
     }
+}
+
+// The same one row at a time (t a compile-time constant of an unrolled loop).
+template <bool INTERIOR, int LT, typename CT>
+__device__ __forceinline__ CT chunk_row(const DevTables<CT> &T, int t, CT d, CT X0, CT X1, int c, int len) {
+    if (INTERIOR) {
+        const ChunkFactors<LT, CT> U = interior_factors<LT, CT>();
+        return t == 0 ? X0 : (t == LT - 1 ? X1 : cf_fma(U.nrc[t], X1, cf_fma(U.nra[t], X0, d)));
+    }
+    CT x = d - T.rca[t * 32 + c] * X0 - T.rcc[t * 32 + c] * X1;
+    if (t == 0) x = X0;
+    if (t != 0 && t == len - 1) x = X1;
+    return x;
 }
 
 // warp_solve for lines with ChunkFactors (all chunks full, no cyclic
@@ -515,24 +529,113 @@ __device__ __forceinline__ void deriv_rhs(const FT *f, int n, int lane, int nsta
 // w = f[c LT - 2 .. c LT + LT + 1]: interior rows, and the rows of the physical
 // closure where a face has it.  Window entries outside the line only reach
 // rows that are replaced (here, or by the caller for interface faces); rows
-// past the line's end are zero.
+// past the chunk's len are zero.
 template <int LT, typename CT>
-__device__ __forceinline__ void chunk_rhs(const CT (&w)[LT + 4], int c, int n, int nstart, int nend, CT (&d)[LT]) {
+__device__ __forceinline__ void chunk_rhs(const CT (&w)[LT + 4], int c, int len, int n, int nstart, int nend,
+                                          CT (&d)[LT]) {
     const int j0 = c * LT;
-#pragma unroll
-    for (int t = 0; t < LT; ++t)
-        d[t] = j0 + t < n ? xmul(CT(kAa), w[t + 3] - w[t + 1]) + xmul(CT(kBb), w[t + 4] - w[t]) : CT(0);
-    if (nstart == 0 && c == 0) {
-        d[0] = xmul(CT(kAb00), w[2]) + xmul(CT(kAb01), w[3]) + xmul(CT(kAb02), w[4]);
-        d[1] = xmul(CT(kAb10), w[4] - w[2]);
+    // physical rows first, so that no window value outlives its interior row
+    const bool lo = nstart == 0 && c == 0, hi = nend == 0 && j0 + LT >= n - 1;
+    CT r0 = CT(0), r1 = CT(0), e1 = CT(0), e2 = CT(0);
+    if (lo) {
+        r0 = xmul(CT(kAb00), w[2]) + xmul(CT(kAb01), w[3]) + xmul(CT(kAb02), w[4]);
+        r1 = xmul(CT(kAb10), w[4] - w[2]);
     }
-    if (nend == 0 && j0 + LT >= n - 1) {
+    if (hi) {
 #pragma unroll
         for (int t = 0; t < LT; ++t) {
             if (j0 + t == n - 1)
-                d[t] = -(xmul(CT(kAb00), w[t + 2]) + xmul(CT(kAb01), w[t + 1]) + xmul(CT(kAb02), w[t]));
-            if (j0 + t == n - 2) d[t] = xmul(-CT(kAb10), w[t + 1] - w[t + 3]);
+                e1 = -(xmul(CT(kAb00), w[t + 2]) + xmul(CT(kAb01), w[t + 1]) + xmul(CT(kAb02), w[t]));
+            if (j0 + t == n - 2) e2 = xmul(-CT(kAb10), w[t + 1] - w[t + 3]);
         }
+    }
+#pragma unroll
+    for (int t = 0; t < LT; ++t) d[t] = xmul(CT(kAa), w[t + 3] - w[t + 1]) + xmul(CT(kBb), w[t + 4] - w[t]);
+    if (len < LT) {
+#pragma unroll
+        for (int t = 0; t < LT; ++t)
+            if (t >= len) d[t] = CT(0);
+    }
+    if (lo) {
+        d[0] = r0;
+        d[1] = r1;
+    }
+    if (hi) {
+        set_at<LT, CT>(d, n - 1 - j0, e1);
+        set_at<LT, CT>(d, n - 2 - j0, e2);
+    }
+}
+
+// Put the interface closure rows r0, r1 (rows 0, 1) and r2, r3 (rows n-1, n-2,
+// without their sign) of a line into chunk c's right-hand side.
+template <int LT, typename T>
+__device__ __forceinline__ void chunk_take_rows(T r0, T r1, T r2, T r3, int c, int n, int nstart, int nend,
+                                                T (&d)[LT]) {
+    if (nstart && c == 0) {
+        d[0] = r0;
+        d[1] = r1;
+    }
+    if (nend && (c + 1) * LT >= n - 1) {
+        if (c == (n - 1) / LT) set_at<LT, T>(d, (n - 1) - c * LT, -r2);
+        if (c == (n - 2) / LT) set_at<LT, T>(d, (n - 2) - c * LT, -r3);
+    }
+}
+
+// Lines held in the registers of one warp (lane c = chunk c): the eight points
+// at either end of line v go to ends[v] ([k] = f[k], [8 + k] = f[n-1-k]), ...
+template <int LT, int NV, typename T>
+__device__ __forceinline__ void chunk_put_ends(T (*ends)[2 * kLmd + 1], const T (&d)[NV][LT], int c, int len, int n) {
+    const int j0 = c * LT;
+    if (j0 < kLmd) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (j0 + t < kLmd) ends[v][j0 + t] = d[v][t];
+    }
+    if (j0 + LT > n - kLmd) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len && j0 + t >= n - kLmd) ends[v][kLmd + n - 1 - (j0 + t)] = d[v][t];
+    }
+}
+// ... and lane 8 v + k forms closure sum k of line v from them (interface_sum's
+// operations; far != nullptr: the far-end sums k = 2, 3, 6, 7 are *far).  Lanes
+// 8 v + {0, 1, 4, 5} get rows 0, 1, n-1, n-2.  All 32 lanes must call it.
+template <typename T>
+__device__ __forceinline__ T ends_closure_row(const T *ends, int k8, const Coeffs &cf, const T *far = nullptr) {
+    const bool bci = k8 < 2 || k8 == 4 || k8 == 5, asc = k8 < 2 || k8 >= 6, second = (k8 & 1) != 0;
+    T dv = T(0);
+    if (far && (k8 & 2)) {
+        dv = *far;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kLmd; ++k) {
+            const double c = bci ? (second ? cf.pbci[kLmd + k] : cf.pbci[k])
+                                 : (second ? cf.pbco[kLmd + k] : cf.pbco[k]);
+            dv += xmul(T(c), ends[asc ? k : kLmd + k]);
+        }
+    }
+    return dv + __shfl_down_sync(0xffffffffu, dv, 2);
+}
+// Right-hand side of line v from the field values d; rows: ends_closure_row.
+template <int LT, typename T>
+__device__ __forceinline__ void chunk_warp_rhs(T rows, int v, int lane, int len, int n, int nstart, int nend,
+                                               T (&d)[LT]) {
+    T x[LT + 4];
+    x[0] = __shfl_up_sync(0xffffffffu, d[LT - 2], 1);
+    x[1] = __shfl_up_sync(0xffffffffu, d[LT - 1], 1);
+    x[LT + 2] = __shfl_down_sync(0xffffffffu, d[0], 1);
+    x[LT + 3] = __shfl_down_sync(0xffffffffu, d[1], 1);
+#pragma unroll
+    for (int t = 0; t < LT; ++t) x[t + 2] = d[t];
+    chunk_rhs<LT, T>(x, lane, len, n, nstart, nend, d);
+    if (nstart || nend) {
+        T own2[2];
+        take_closure_rows(rows, v, lane, own2);
+        chunk_take_rows<LT, T>(own2[0], own2[1], own2[0], own2[1], lane, n, nstart, nend, d);
     }
 }
 

@@ -238,39 +238,6 @@ __device__ __forceinline__ void store_line_regs(T *line, const T (&d)[LT], int l
         if (lane * LT + t < n) line[L::pos_ct(lane, t)] = d[t];
 }
 
-// Vector access of VB bytes (16 or 32) to a lane's own chunk.
-template <int VB, typename T>
-__device__ __forceinline__ void load_vec(const T *p, T *v) {
-    if constexpr (VB == 32 && sizeof(T) == 8) {
-        asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
-            : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p) : "memory");
-    } else if constexpr (VB == 32) {
-        asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-            : "l"(p) : "memory");
-    } else if constexpr (sizeof(T) == 8) {
-        const double2 x = *reinterpret_cast<const double2 *>(p);
-        v[0] = x.x; v[1] = x.y;
-    } else {
-        const float4 x = *reinterpret_cast<const float4 *>(p);
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    }
-}
-template <int VB, typename T>
-__device__ __forceinline__ void store_vec(T *p, const T *v) {
-    if constexpr (VB == 32 && sizeof(T) == 8) {
-        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
-                     : "memory");
-    } else if constexpr (VB == 32) {
-        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
-                     "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
-    } else if constexpr (sizeof(T) == 8) {
-        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
-    } else {
-        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    }
-}
-
 // The fields one derivative launch covers (blockIdx.y): field f is
 // in[f * in_fs + .] -> out[f * out_fs + .], line-end values at drva + f F and
 // received sums at recv + 4 f F (either may be null).
@@ -297,72 +264,36 @@ k_deriv_row(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, C
     const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31, j0 = lane * LT;
     const int64_t line0 = ((int64_t)blockIdx.x * (kThreads / 32) + w) * NV;
     if (line0 >= F) return;
+    const int len = lane_len(lane, LT, tab.p, tab.last_len);
     const T *in = fs.in + blockIdx.y * fs.in_fs + line0 * n + j0;
     T *out = fs.out + blockIdx.y * fs.out_fs + line0 * n + j0;
     T d[NV][LT];
 #pragma unroll
-    for (int h = 0; h < NV; ++h)
+    for (int h = 0; h < NV; ++h) {
+        // past the last line: the last line again, not stored
+        const T *src = in + (line0 + h < F ? h : 0) * (int64_t)n;
 #pragma unroll
         for (int t = 0; t < LT; t += VE) {
-            if (line0 + h < F && j0 + t < n) {
-                load_vec<VB, T>(in + (int64_t)h * n + t, &d[h][t]);
+            if (t < len) {
+                load_vec<VB, T>(src + t, &d[h][t]);
             } else {
 #pragma unroll
                 for (int k = 0; k < VE; ++k) d[h][t + k] = T(0);
             }
         }
+    }
     T rows = T(0);  // lane 8 h + {0, 1, 4, 5}: interface rows 0, 1, n-1, n-2 of line h
     if (nstart || nend) {
-        if (j0 < kLmd || j0 + LT > n - kLmd) {
-#pragma unroll
-            for (int h = 0; h < NV; ++h)
-#pragma unroll
-                for (int t = 0; t < LT; ++t) {
-                    const int j = j0 + t;
-                    if (j < kLmd) ends[w][h][j] = d[h][t];
-                    if (j < n && j >= n - kLmd) ends[w][h][kLmd + n - 1 - j] = d[h][t];
-                }
-        }
+        chunk_put_ends<LT, NV, T>(ends[w], d, lane, len, n);
         __syncwarp();
         const int h = lane >> 3, k8 = lane & 7;
-        T dv = T(0);
-        if (h < NV) {
-            const bool bci = k8 < 2 || k8 == 4 || k8 == 5, asc = k8 < 2 || k8 >= 6, second = (k8 & 1) != 0;
-            if (fs.recv && (k8 & 2)) {
-                if (line0 + h < F)
-                    dv = fs.recv[((int64_t)blockIdx.y * 4 + ((k8 >> 1 & 2) | (k8 & 1))) * F + line0 + h];
-            } else {
-#pragma unroll
-                for (int k = 0; k < kLmd; ++k) {
-                    const double c = bci ? (second ? cf.pbci[kLmd + k] : cf.pbci[k])
-                                         : (second ? cf.pbco[kLmd + k] : cf.pbco[k]);
-                    dv += xmul(T(c), ends[w][h][asc ? k : kLmd + k]);
-                }
-            }
-        }
-        rows = dv + __shfl_down_sync(0xffffffffu, dv, 2);
+        T far = T(0);
+        if (fs.recv && (k8 & 2) && h < NV && line0 + h < F)
+            far = fs.recv[((int64_t)blockIdx.y * 4 + ((k8 >> 1 & 2) | (k8 & 1))) * F + line0 + h];
+        rows = ends_closure_row<T>(ends[w][h < NV ? h : 0], k8, cf, fs.recv ? &far : nullptr);
     }
 #pragma unroll
-    for (int h = 0; h < NV; ++h) {
-        T x[LT + 4];
-        x[0] = __shfl_up_sync(0xffffffffu, d[h][LT - 2], 1);
-        x[1] = __shfl_up_sync(0xffffffffu, d[h][LT - 1], 1);
-        x[LT + 2] = __shfl_down_sync(0xffffffffu, d[h][0], 1);
-        x[LT + 3] = __shfl_down_sync(0xffffffffu, d[h][1], 1);
-#pragma unroll
-        for (int t = 0; t < LT; ++t) x[t + 2] = d[h][t];
-        T own2[2] = {T(0), T(0)};
-        if (nstart || nend) take_closure_rows(rows, h, lane, own2);
-        chunk_rhs<LT, T>(x, lane, n, nstart, nend, d[h]);
-        if (nstart && lane == 0) {
-            d[h][0] = own2[0];
-            d[h][1] = own2[1];
-        }
-        if (nend) {
-            if (lane == (n - 1) / LT) set_at<LT, T>(d[h], (n - 1) - j0, -own2[0]);
-            if (lane == (n - 2) / LT) set_at<LT, T>(d[h], (n - 2) - j0, -own2[1]);
-        }
-    }
+    for (int h = 0; h < NV; ++h) chunk_warp_rhs<LT, T>(rows, h, lane, len, n, nstart, nend, d[h]);
     warp_solve<LT, NV, T>(tab, d, lane);
 #pragma unroll
     for (int h = 0; h < NV; ++h) {
@@ -374,7 +305,7 @@ k_deriv_row(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, C
         }
 #pragma unroll
         for (int t = 0; t < LT; t += VE)
-            if (j0 + t < n) store_vec<VB, T>(out + (int64_t)h * n + t, &d[h][t]);
+            if (t < len) store_vec<VB, T>(out + (int64_t)h * n + t, &d[h][t]);
     }
 }
 
@@ -430,48 +361,136 @@ k_deriv_row_any(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t 
         for (int j = lane; j < n; j += 32) out[(int64_t)h * n + j] = sm[h * L::kSlot + L::pos(j)];
 }
 
-// The same along y and z: a column tile of TL lines (column.cuh).
-template <int LT, int AXIS, int TL, typename T>
-__global__ void __launch_bounds__(TL * 32, LT <= 8 ? 1024 / (TL * 32) : (LT == 16 ? 2 : 1))
-k_deriv_col(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int nend, int64_t F, Coeffs cf) {
-    using C = Column<LT, TL>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *V = reinterpret_cast<T *>(smem_raw), *rows = V + C::kField;
-    const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL, j0 = c * LT;
+// The same along y and z for the lines of warp_column (column.cuh): four lines
+// per warp.  SUM: also sum[f] = (add0[f] + add1[f]) +
+// derivative, the right-hand side of calc_fluxes from its last derivative.
+template <int LT, int AXIS, typename T, bool SUM>
+__global__ void __launch_bounds__(kThreads, 3)
+k_deriv_wcol(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int nend, int F, Coeffs cf,
+             DerivSum sum) {
+    __shared__ T ends[kThreads / 32][kWarpLines][2 * kLmd + 1];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int l = lane % kWarpLines, c = lane / kWarpLines;
     const int len = lane_len(c, LT, tab.p, tab.last_len);
-    const int64_t line0 = (int64_t)blockIdx.x * TL, fidx = line0 + l;
-    const bool ok = fidx < F;
-    const int64_t s = line_stride<AXIS>(lxi, let), base = line_base<AXIS>(fidx, lxi, let) + j0 * s;
-    const T *in = fs.in + blockIdx.y * fs.in_fs + base;
+    const int line0 = ((int)blockIdx.x * (kThreads / 32) + w) * kWarpLines, s = AXIS == 1 ? lxi : lxi * let;
+    if (line0 >= F) return;
+    const int fidx = min(line0 + l, F - 1);  // past the last line: the last line again, not stored
+    const int base = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + c * LT * s;
+    const T *in = fs.in + blockIdx.y * fs.in_fs;
     T d[1][LT];
 #pragma unroll
-    for (int t = 0; t < LT; ++t) d[0][t] = ok && t < len ? in[t * s] : T(0);
-    const bool near_end = j0 < kLmd || j0 + LT > n - kLmd;
+    for (int t = 0; t < LT; ++t) d[0][t] = t < len ? in[base + t * s] : T(0);
+    T far = T(0);
+    if (fs.recv && (lane & 2)) {
+        const int k = (lane & 7) >> 1 & 2 | (lane & 1), line = line0 + (lane >> 3);
+        if (line < F) far = fs.recv[((int64_t)blockIdx.y * 4 + k) * F + line];
+    }
+    warp_column_rhs<LT, T>(ends[w], lane, len, n, nstart, nend, cf, fs.recv ? &far : nullptr, d);
+    warp_column_solve<LT, T>(tab, lane, len, d);
+    if (len == 0 || line0 + l >= F) return;
+    if (fs.drva) {
+        T *dr = fs.drva + (int64_t)blockIdx.y * F + fidx;
+        if (c == 0) dr[0] = d[0][0];
+        if (c == (n - 1) / LT) dr[5 * (int64_t)F] = get_at<LT, T>(d[0], (n - 1) - c * LT);
+    }
+    T *out = fs.out + blockIdx.y * fs.out_fs;
+    if constexpr (SUM) {
+        const double *a0 = sum.add0 + blockIdx.y * sum.add_fs, *a1 = sum.add1 + blockIdx.y * sum.add_fs;
+        double *total = sum.sum + blockIdx.y * sum.sum_fs;
+        constexpr int B = 8;
+#pragma unroll
+        for (int t0 = 0; t0 < LT; t0 += B) {
+            double r[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                if (t0 + b < len) r[b] = a0[base + (t0 + b) * s] + a1[base + (t0 + b) * s];
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                if (t0 + b < len) total[base + (t0 + b) * s] = r[b] + d[0][t0 + b];
+        }
+    }
 #pragma unroll
     for (int t = 0; t < LT; ++t)
-        if (t < 2 || t >= LT - 2 || near_end) V[C::at(t, c, l)] = d[0][t];
+        if (t < len) out[base + t * s] = d[0][t];
+}
+
+// The same for all other y and z lines: column tiles (column.cuh) of two groups of TL lines,
+// thread (l, c) holding chunk c of lines l and l + TL, so that addresses, solver
+// constants, table loads and barriers serve two lines (and a row of the tile is
+// 128 bytes).  Bound by its instructions and load latency (24 warps per SM): one
+// 256^3 field 78 us, 3.4 TB/s, against 80 us with one line per thread, 87 us with
+// 16-line tiles, and 105 us staged through a transposing layout.
+template <int LT, int AXIS, int TL, typename T, bool SUM>
+__global__ void __launch_bounds__(TL * 32, LT <= 8 ? 768 / (TL * 32) : (LT == 16 ? 2 : 1))
+k_deriv_col(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int nend, int F, Coeffs cf,
+            DerivSum sum) {
+    using C = Column<LT, TL>;
+    constexpr int NL = 2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *V = reinterpret_cast<T *>(smem_raw), *rows = V + NL * C::kField;
+    const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL, j0 = c * LT;
+    const int len = lane_len(c, LT, tab.p, tab.last_len);
+    const int line0 = (int)blockIdx.x * (NL * TL) , s = AXIS == 1 ? lxi : lxi * let;
+    int base[NL];
+#pragma unroll
+    for (int h = 0; h < NL; ++h) {
+        // past the last line: the last line again, not stored
+        const int fidx = min(line0 + h * TL + l, F - 1);
+        base[h] = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + j0 * s;
+    }
+    const T *in = fs.in + blockIdx.y * fs.in_fs;
+    T d[NL][LT];
+#pragma unroll
+    for (int t = 0; t < LT; ++t)
+#pragma unroll
+        for (int h = 0; h < NL; ++h) d[h][t] = t < len ? in[base[h] + t * s] : T(0);
+#pragma unroll
+    for (int h = 0; h < NL; ++h) column_put_raw<LT, TL, T>(V + h * C::kField, d[h], c, l, n);
     __syncthreads();
     if (nstart || nend)
-        column_closure_rows<LT, TL, 1, T>(V, rows, n, cf, fs.recv ? fs.recv + blockIdx.y * 4 * F : nullptr, F, line0);
-    column_rhs<LT, TL, T>(V, c, l, n, nstart, nend, d[0]);
-    __syncthreads();
-    column_take_rows<LT, T>(rows + 4 * l, c, n, nstart, nend, d[0]);
-    chunk_eliminate<LT, 1, T>(tab, d, c);
-    column_put_ends<LT, TL, T>(V, d[0], c, l, len);
-    __syncthreads();
-    column_reduced<LT, TL, 1, T>(V, tab, F, line0, nullptr);
-    __syncthreads();
-    column_finish<LT, TL, T>(V, tab, c, l, len, d[0]);
-    if (!ok) return;
-    if (fs.drva) {
-        T *dr = fs.drva + blockIdx.y * F + fidx;
-        if (c == 0) dr[0] = d[0][0];
-        if (c == (n - 1) / LT) dr[5 * F] = get_at<LT, T>(d[0], (n - 1) - j0);
-    }
-    T *out = fs.out + blockIdx.y * fs.out_fs + base;
+        column_closure_rows<LT, TL, NL, T, T>(V, rows, n, cf, fs.recv ? fs.recv + (int64_t)blockIdx.y * 4 * F : nullptr,
+                                           F, line0);
 #pragma unroll
-    for (int t = 0; t < LT; ++t)
-        if (t < len) out[t * s] = d[0][t];
+    for (int h = 0; h < NL; ++h) column_rhs<LT, TL, T>(V + h * C::kField, c, l, len, n, nstart, nend, d[h]);
+    __syncthreads();
+    if (nstart || nend) {
+#pragma unroll
+        for (int h = 0; h < NL; ++h) column_take_rows<LT, T>(rows + 4 * (h * TL + l), c, n, nstart, nend, d[h]);
+    }
+    chunk_eliminate<LT, NL, T>(tab, d, c);
+#pragma unroll
+    for (int h = 0; h < NL; ++h) column_put_ends<LT, TL, T>(V + h * C::kField, d[h], c, l, len);
+    __syncthreads();
+    column_reduced<LT, TL, NL, T>(V, tab);
+    __syncthreads();
+    if (len == 0) return;
+#pragma unroll
+    for (int h = 0; h < NL; ++h) column_finish<LT, TL, T>(V + h * C::kField, tab, c, l, len, d[h]);
+    T *out = fs.out + blockIdx.y * fs.out_fs;
+#pragma unroll
+    for (int h = 0; h < NL; ++h) {
+        const int fidx = line0 + h * TL + l;
+        if (fidx >= F) break;
+        if (fs.drva) {
+            T *dr = fs.drva + (int64_t)blockIdx.y * F + fidx;
+            if (c == 0) dr[0] = d[h][0];
+            if (c == (n - 1) / LT) dr[5 * (int64_t)F] = get_at<LT, T>(d[h], (n - 1) - j0);
+        }
+        if constexpr (SUM) {
+            const double *a0 = sum.add0 + blockIdx.y * sum.add_fs, *a1 = sum.add1 + blockIdx.y * sum.add_fs;
+            double *total = sum.sum + blockIdx.y * sum.sum_fs;
+            double r[LT];
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len) r[t] = a0[base[h] + t * s] + a1[base[h] + t * s];
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len) total[base[h] + t * s] = r[t] + d[h][t];
+        }
+#pragma unroll
+        for (int t = 0; t < LT; ++t)
+            if (t < len) out[base[h] + t * s] = d[h][t];
+    }
 }
 
 // Compact filter of one field along AXIS.
@@ -539,13 +558,9 @@ static int prep_smem(KernelT kern, size_t bytes) {
     return CS_OK;
 }
 
-#ifndef CSB_COL_TL
-#define CSB_COL_TL 8
-#endif
-
 template <int LT, int AXIS, typename T>
 static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d, int nstart,
-                           int nend, const Coeffs &cf, cudaStream_t st) {
+                           int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
     const int64_t F = face_size(d, AXIS);
     if constexpr (AXIS == 0) {
         constexpr int NV = LT <= 8 ? 2 : 1, WARPS = kThreads / 32;
@@ -574,12 +589,28 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
         if (int rc = prep_smem(kern, smem)) return rc;
         kern<<<grid, kThreads, smem, st>>>(fs, tab, nstart, nend, F, cf);
     } else {
-        constexpr int TL = CSB_COL_TL;
-        const size_t smem = (size_t)(Column<LT, TL>::kField + 4 * TL) * sizeof(T);
-        auto kern = k_deriv_col<LT, AXIS, TL, T>;
-        if (int rc = prep_smem(kern, smem)) return rc;
-        kern<<<dim3((unsigned)((F + TL - 1) / TL), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
-            fs, tab, d.lxi, d.let, nstart, nend, F, cf);
+        const bool with_sum = AXIS == 2 && sizeof(T) == 8 && sum;
+        if (LT == kWarpChunk && warp_column(tab.n)) {
+            if constexpr (LT == kWarpChunk) {
+                constexpr int LINES = kThreads / 32 * kWarpLines;
+                auto kern = k_deriv_wcol<LT, AXIS, T, false>;
+                if constexpr (AXIS == 2 && sizeof(T) == 8) {
+                    if (with_sum) kern = k_deriv_wcol<LT, AXIS, T, true>;
+                }
+                kern<<<dim3((unsigned)((F + LINES - 1) / LINES), (unsigned)nf), kThreads, 0, st>>>(
+                    fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, with_sum ? *sum : DerivSum{});
+            }
+        } else {
+            constexpr int TL = 8;
+            const size_t smem = (size_t)2 * (Column<LT, TL>::kField + 4 * TL) * sizeof(T);
+            auto kern = k_deriv_col<LT, AXIS, TL, T, false>;
+            if constexpr (AXIS == 2 && sizeof(T) == 8) {
+                if (with_sum) kern = k_deriv_col<LT, AXIS, TL, T, true>;
+            }
+            if (int rc = prep_smem(kern, smem)) return rc;
+            kern<<<dim3((unsigned)((F + 2 * TL - 1) / (2 * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
+                fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, with_sum ? *sum : DerivSum{});
+        }
     }
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
@@ -587,13 +618,13 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
 
 template <int AXIS, typename T>
 static int launch_deriv_axis(int lt, const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d,
-                             int nstart, int nend, const Coeffs &cf, cudaStream_t st) {
+                             int nstart, int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
     switch (lt) {
-        case 2: return launch_deriv_lt<2, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
-        case 4: return launch_deriv_lt<4, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
-        case 8: return launch_deriv_lt<8, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
-        case 16: return launch_deriv_lt<16, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
-        case 32: return launch_deriv_lt<32, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, st);
+        case 2: return launch_deriv_lt<2, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
+        case 4: return launch_deriv_lt<4, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
+        case 8: return launch_deriv_lt<8, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
+        case 16: return launch_deriv_lt<16, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
+        case 32: return launch_deriv_lt<32, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
     }
     return set_error(CS_ERR_UNSUPPORTED, "chunk length %d", lt);
 }
@@ -642,6 +673,35 @@ const DevTables<double> &pick_tables<double>(const DeviceTables &dt) { return dt
 template <>
 const DevTables<float> &pick_tables<float>(const DeviceTables &dt) { return dt.t32; }
 
+// Shortest chunk of the tables of a derivative along `axis`.
+static int deriv_chunk(int axis, int n) { return axis > 0 && warp_column(n) ? kWarpChunk : 2; }
+
+// nf derivatives along `axis` in one launch: field f is in + f in_fs -> out +
+// f out_fs, with the numerics object's interface buffers of variable var + f.
+template <typename T>
+static int deriv_launch(cs_numerics *nm, int axis, const T *in, int64_t in_fs, T *out, int64_t out_fs, int nf,
+                        unsigned var, int nstart, int nend, int halo, const DerivSum *sum, cudaStream_t st) {
+    const cs_dcomp &d = nm->d;
+    const int n = line_len(d, axis);
+    if ((nstart || nend) && n < kLmd) return set_error(CS_ERR_UNSUPPORTED, "interface closure needs n >= 8");
+    const DeviceTables *dt = nm->tables.get(n, kDeriv, nstart, nend, 0.0, deriv_chunk(axis, n));
+    if (!dt) return CS_ERR_UNSUPPORTED;
+    const int64_t F = face_size(d, axis);
+    FieldSet<T> fs{in, out, nullptr, nullptr, in_fs, out_fs};
+    if (sizeof(T) == sizeof(double)) {
+        if (halo == CS_HALO_RECV) fs.recv = reinterpret_cast<const T *>(nm->recv[axis] + (int64_t)var * 4 * F);
+        fs.drva = reinterpret_cast<T *>(nm->drva[axis] + (int64_t)var * F);
+    } else if (halo == CS_HALO_RECV && (nstart || nend)) {
+        return set_error(CS_ERR_UNSUPPORTED, "FP32 derivative supports CS_HALO_SELF only");
+    }
+    const DevTables<T> &tab = pick_tables<T>(*dt);
+    switch (axis) {
+        case 0: return launch_deriv_axis<0, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, nullptr, st);
+        case 1: return launch_deriv_axis<1, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, nullptr, st);
+        default: return launch_deriv_axis<2, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, sum, st);
+    }
+}
+
 template <typename T>
 static int deriv_impl(cs_numerics *nm, int axis, const T *in, T *out, int nstart, int nend,
                       cs_dcomp d, unsigned var, unsigned comp, unsigned slot, int halo,
@@ -652,27 +712,92 @@ static int deriv_impl(cs_numerics *nm, int axis, const T *in, T *out, int nstart
     if (!same_dims(d, nm->d)) return set_error(CS_ERR_INVALID, "dims differ from the numerics object");
     if (axis < 0 || axis > 2 || var >= 5 || comp > 14 || slot > 14)
         return set_error(CS_ERR_INVALID, "axis %d var %u comp %u slot %u", axis, var, comp, slot);
-    const int n = line_len(d, axis);
-    if ((nstart || nend) && n < kLmd) return set_error(CS_ERR_UNSUPPORTED, "interface closure needs n >= 8");
-    const DeviceTables *dt = nm->tables.get(n, kDeriv, nstart, nend, 0.0);
-    if (!dt) return CS_ERR_UNSUPPORTED;
-    const int64_t F = face_size(d, axis);
-    const T *recv = nullptr;
-    T *drva = nullptr;
-    if (sizeof(T) == sizeof(double)) {
-        if (halo == CS_HALO_RECV) recv = reinterpret_cast<const T *>(nm->recv[axis] + (int64_t)var * 4 * F);
-        drva = reinterpret_cast<T *>(nm->drva[axis] + (int64_t)var * F);
-    } else if (halo == CS_HALO_RECV && (nstart || nend)) {
-        return set_error(CS_ERR_UNSUPPORTED, "FP32 derivative supports CS_HALO_SELF only");
+    return deriv_launch<T>(nm, axis, in + (int64_t)comp * d.lmx, 0, out + (int64_t)slot * d.lmx, 0, 1, var, nstart,
+                           nend, halo, nullptr, (cudaStream_t)stream);
+}
+
+int deriv_fields(cs_numerics *nm, int axis, const double *in, int64_t in_fs, double *out, int64_t out_fs, int nf,
+                 unsigned var, const DerivSum *sum, cudaStream_t st) {
+    if (!nm->setup_done) return set_error(CS_ERR_STATE, "cs_deriv before cs_deriv_setup");
+    return deriv_launch<double>(nm, axis, in, in_fs, out, out_fs, nf, var, nm->ndf[0][axis], nm->ndf[1][axis],
+                                CS_HALO_RECV, sum, st);
+}
+
+// Interface sums of every face of a single-rank block and their exchange
+// (fill_buffers, then the copy of cs_halo_exchange_self) for nf variables in
+// one launch (34 us for five variables at 256^3; face by face and copy by copy
+// it was 30 launches and 30 copies, about 180 us, and all latency on small
+// blocks): thread = (face, line), blockIdx.y = variable; the sums of face
+// ip go to its send buffer and to the receive buffer of face 1 - ip.
+struct ExchangeArgs {
+    const double *in;  // variable 0; variables fs apart, axis a's component comp_fs * a further
+    int64_t fs, comp_fs;
+    double *send[3], *recv[3];
+    int64_t F[3];
+    int n[3], on[3], lxi, let;
+    unsigned var;  // variable of the buffers that blockIdx.y = 0 fills
+};
+__global__ void k_exchange_self(ExchangeArgs x, Coeffs cf) {
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int a = 0;
+    for (; a < 3; ++a) {
+        const int64_t lines = x.on[a] ? 2 * x.F[a] : 0;
+        if (i < lines) break;
+        i -= lines;
     }
-    const FieldSet<T> fs{in + (int64_t)comp * d.lmx, out + (int64_t)slot * d.lmx, recv, drva, 0, 0};
-    cudaStream_t st = (cudaStream_t)stream;
-    const DevTables<T> &tab = pick_tables<T>(*dt);
-    switch (axis) {
-        case 0: return launch_deriv_axis<0, T>(dt->lt, fs, 1, tab, d, nstart, nend, nm->cf, st);
-        case 1: return launch_deriv_axis<1, T>(dt->lt, fs, 1, tab, d, nstart, nend, nm->cf, st);
-        default: return launch_deriv_axis<2, T>(dt->lt, fs, 1, tab, d, nstart, nend, nm->cf, st);
+    if (a == 3) return;
+    const int64_t F = x.F[a], fidx = i < F ? i : i - F;
+    const int ip = i < F ? 0 : 1;
+    const int64_t base = a == 0 ? line_base<0>(fidx, x.lxi, x.let)
+                                : (a == 1 ? line_base<1>(fidx, x.lxi, x.let) : line_base<2>(fidx, x.lxi, x.let));
+    const int64_t s = a == 0 ? 1 : (a == 1 ? (int64_t)x.lxi : (int64_t)x.lxi * x.let);
+    const double *in = x.in + blockIdx.y * x.fs + a * x.comp_fs + base + (ip ? (x.n[a] - 1) * s : 0);
+    const int64_t inc = ip ? -s : s;
+    double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+    for (int k = 0; k < kLmd; ++k) {
+        const double f = in[k * inc];
+        v0 += cf.pbco[k] * f;
+        v1 += cf.pbco[kLmd + k] * f;
     }
+    const int64_t o = (int64_t)(x.var + blockIdx.y) * 4 * F + fidx;
+    double *snd = x.send[a] + o + ip * 2 * F, *rcv = x.recv[a] + o + (1 - ip) * 2 * F;
+    snd[0] = v0;
+    snd[F] = v1;
+    rcv[0] = v0;
+    rcv[F] = v1;
+}
+
+int exchange_self(cs_numerics *nm, const double *in, int64_t fs, int64_t comp_fs, int nf, unsigned var,
+                  cudaStream_t st) {
+    if (!nm->setup_done) return set_error(CS_ERR_STATE, "cs_fill_buffers before cs_deriv_setup");
+    ExchangeArgs x{};
+    int64_t total = 0;
+    for (int a = 0; a < 3; ++a) {
+        x.n[a] = line_len(nm->d, a);
+        if ((nm->ndf[0][a] || nm->ndf[1][a]) && x.n[a] < kLmd)
+            return set_error(CS_ERR_UNSUPPORTED, "interface face needs n >= 8");
+    }
+    for (int a = 0; a < 3; ++a) {
+        if (nm->ndf[0][a] != nm->ndf[1][a])
+            return set_error(CS_ERR_UNSUPPORTED,
+                             "axis %d has one interface face: a single rank has no neighbour for it", a);
+        x.F[a] = face_size(nm->d, a);
+        x.on[a] = nm->ndf[0][a];
+        x.send[a] = nm->send[a];
+        x.recv[a] = nm->recv[a];
+        if (x.on[a]) total += 2 * x.F[a];
+    }
+    if (total == 0) return CS_OK;
+    x.in = in;
+    x.fs = fs;
+    x.comp_fs = comp_fs;
+    x.lxi = nm->d.lxi;
+    x.let = nm->d.let;
+    x.var = var;
+    k_exchange_self<<<dim3((unsigned)((total + 127) / 128), (unsigned)nf), 128, 0, st>>>(x, nm->cf);
+    CSB_CUDA(cudaGetLastError());
+    return CS_OK;
 }
 
 }  // namespace csb
@@ -736,7 +861,7 @@ int cs_deriv_setup(cs_numerics *nm) {
     for (int a = 0; a < 3; ++a) {
         const int n = line_len(nm->d, a);
         if (n < 5) continue;  // degenerate axis: derivative along it is rejected at call time
-        if (!nm->tables.get(n, kDeriv, nm->ndf[0][a], nm->ndf[1][a], 0.0)) return CS_ERR_UNSUPPORTED;
+        if (!nm->tables.get(n, kDeriv, nm->ndf[0][a], nm->ndf[1][a], 0.0, deriv_chunk(a, n))) return CS_ERR_UNSUPPORTED;
     }
     nm->setup_done = true;
     return CS_OK;

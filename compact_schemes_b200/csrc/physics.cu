@@ -20,7 +20,6 @@ struct cs_physics {
     double *buffer_deriv = nullptr;  // [5][3][lmx]
     double *tau = nullptr;           // [6][lmx] xx, yy, zz, xy, yz, zx
     double *heat = nullptr;          // [3][lmx]
-    double *ss = nullptr;            // [3][lmx] temperature gradient
     double *dt_acc = nullptr;        // [2]
 };
 
@@ -89,61 +88,62 @@ __global__ void k_visc_init(double *__restrict__ buf, const double *__restrict__
 }
 
 // calc_viscous_shear_stress_post_compute_kernel<m> (physics.hpp:228-283),
-// applied to the derivatives (the reference passes the underived buffer).
-__global__ void k_visc_post(double *__restrict__ tau, double *__restrict__ heat, double *__restrict__ ss,
-                            const double *__restrict__ bd, const double *__restrict__ xim,
-                            const double *__restrict__ etm, const double *__restrict__ zem, int64_t n) {
+// applied to the derivatives (the reference passes the underived buffer), and
+// calc_viscous_shear_stress_final_kernel (:285-333) in one pass, including its
+// side effects on de (de0 <- ssk, de4 <- 2/3 div).  The physical gradients
+// stay in registers between the two: bound by its 37 field reads and writes
+// per point (710 us at 256^3, 7.0 TB/s; two kernels with 61: 1175 us).
+__global__ void k_visc_stress(double *__restrict__ de, double *__restrict__ tau, double *__restrict__ heat,
+                              const double *__restrict__ bd, const double *__restrict__ ssk,
+                              const double *__restrict__ xim, const double *__restrict__ etm,
+                              const double *__restrict__ zem, const double *__restrict__ yaco, int64_t n) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double *out[5][3] = {{nullptr, nullptr, nullptr},
-                         {tau, heat + 2 * n, tau + 5 * n},
-                         {tau + 3 * n, tau + 1 * n, heat},
-                         {heat + 1 * n, tau + 4 * n, tau + 2 * n},
-                         {ss, ss + n, ss + 2 * n}};
+    double M[3][3], dx[4][3];  // dx[c][k]: d/dx_k of u, v, w, T, without the J factor
 #pragma unroll
-    for (int m = 1; m < 5; ++m) {
-        const double g0 = bd[(m * 3) * n + i], g1 = bd[(m * 3 + 1) * n + i], g2 = bd[(m * 3 + 2) * n + i];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            out[m][k][i] = xmul(xim[k * n + i], g0) + xmul(etm[k * n + i], g1) + xmul(zem[k * n + i], g2);
+    for (int k = 0; k < 3; ++k) {
+        M[0][k] = xim[k * n + i];
+        M[1][k] = etm[k * n + i];
+        M[2][k] = zem[k * n + i];
     }
-}
-
-// calc_viscous_shear_stress_final_kernel (physics.hpp:285-333), including its
-// side effects on de (de0 <- ssk, de4 <- 2/3 div).
-__global__ void k_visc_final(double *__restrict__ de, double *__restrict__ tau, double *__restrict__ heat,
-                             const double *__restrict__ ss, const double *__restrict__ ssk,
-                             const double *__restrict__ yaco, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double muj = xmul(ssk[i], yaco[i]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const double *g = bd + (3 + 3 * c) * n + i;
+        const double g0 = g[0], g1 = g[n], g2 = g[2 * n];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dx[c][k] = xmul(M[0][k], g0) + xmul(M[1][k], g1) + xmul(M[2][k], g2);
+    }
+    const double sk = ssk[i];
+    const double muj = xmul(sk, yaco[i]);
     const double kap = xmul(kGamm1Prndtli, muj);
-    const double ux = tau[i], vy = tau[n + i], wz = tau[2 * n + i];
-    const double vx = tau[3 * n + i], wy = tau[4 * n + i], uz = tau[5 * n + i];
-    const double vz = heat[i], wx = heat[n + i], uy = heat[2 * n + i];
-    const double div = xmul(2.0 / 3.0, ux + vy + wz);
-    const double txx = xmul(muj, xmul(2.0, ux) - div), tyy = xmul(muj, xmul(2.0, vy) - div);
-    const double tzz = xmul(muj, xmul(2.0, wz) - div);
-    const double txy = xmul(muj, vx + uy), tyz = xmul(muj, wy + vz), tzx = xmul(muj, uz + wx);
+    const double div = xmul(2.0 / 3.0, dx[0][0] + dx[1][1] + dx[2][2]);
+    const double txx = xmul(muj, xmul(2.0, dx[0][0]) - div), tyy = xmul(muj, xmul(2.0, dx[1][1]) - div);
+    const double tzz = xmul(muj, xmul(2.0, dx[2][2]) - div);
+    const double txy = xmul(muj, dx[1][0] + dx[0][1]), tyz = xmul(muj, dx[2][1] + dx[1][2]);
+    const double tzx = xmul(muj, dx[0][2] + dx[2][0]);
     const double u = de[n + i], v = de[2 * n + i], w = de[3 * n + i];
     tau[i] = txx; tau[n + i] = tyy; tau[2 * n + i] = tzz;
     tau[3 * n + i] = txy; tau[4 * n + i] = tyz; tau[5 * n + i] = tzx;
-    heat[i] = xmul(kap, ss[i]) + xmul(u, txx) + xmul(v, txy) + xmul(w, tzx);
-    heat[n + i] = xmul(kap, ss[n + i]) + xmul(u, txy) + xmul(v, tyy) + xmul(w, tyz);
-    heat[2 * n + i] = xmul(kap, ss[2 * n + i]) + xmul(u, tzx) + xmul(v, tyz) + xmul(w, tzz);
-    de[i] = ssk[i];
+    heat[i] = xmul(kap, dx[3][0]) + xmul(u, txx) + xmul(v, txy) + xmul(w, tzx);
+    heat[n + i] = xmul(kap, dx[3][1]) + xmul(u, txy) + xmul(v, tyy) + xmul(w, tyz);
+    heat[2 * n + i] = xmul(kap, dx[3][2]) + xmul(u, tzx) + xmul(v, tyz) + xmul(w, tzz);
+    de[i] = sk;
     de[4 * n + i] = div;
 }
 
-// calc_time_step_kernel (physics.hpp:335-427): two maxima, reduced with a
-// warp shuffle and an integer atomic max on the non-negative bit patterns.
+// calc_time_step_kernel (physics.hpp:335-427): two maxima, reduced per thread
+// over a grid-stride loop, then by warp shuffles and an integer atomic max on
+// the non-negative bit patterns.  A few atomics per block of a grid that fills
+// the chip once: one pair per warp of one point each (2 x 524288 at 256^3)
+// queued on two addresses for 1.45 ms; with 1184 blocks the 16 fields read take
+// 0.43 ms.
+constexpr int kTimeStepBlocks = 148 * 8;
 __global__ void k_time_step(const double *__restrict__ xim, const double *__restrict__ etm,
                             const double *__restrict__ zem, const double *__restrict__ de,
                             const double *__restrict__ yaco, const double *__restrict__ ssk,
                             double u0, double u1, double u2, unsigned long long *__restrict__ acc, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     double m1 = 0.0, m2 = 0.0;
-    if (i < n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double M[3][3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -162,8 +162,8 @@ __global__ void k_time_step(const double *__restrict__ xim, const double *__rest
             rr2 += fabs(xmul(M[a][0], de[n + i] + u0) + xmul(M[a][1], de[2 * n + i] + u1) +
                         xmul(M[a][2], de[3 * n + i] + u2));
         const double ssi = fabs(yaco[i]);
-        m1 = xmul(sqrt(xmul(de[4 * n + i], rr1)) + rr2, ssi);
-        m2 = de[i] * ssk[i] * rr1 * ssi * ssi;
+        m1 = fmax(m1, xmul(sqrt(xmul(de[4 * n + i], rr1)) + rr2, ssi));
+        m2 = fmax(m2, de[i] * ssk[i] * rr1 * ssi * ssi);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -326,33 +326,42 @@ __device__ __forceinline__ void gc_matvec(const double A[5][5], const double *x,
     }
 }
 
-// Face point fi of face ip along AXIS (the derivative's drva face index) and
+// The active faces of one cs_gcbc_apply call (blockIdx.y picks one): axis, side
+// and update kind, and per axis the buffers and the face size.
+struct GcFaces {
+    double *drva[3], *drvb[3];
+    const double *cm[3];
+    int64_t F[3];
+    int axis[6], ip[6], kind[6];
+    int lxi, let, lze;
+};
+
+// Face point fi of face ip along `axis` (the derivative's drva face index) and
 // the stride into the block.
-template <int AXIS>
-__device__ __forceinline__ int64_t gc_point(int64_t fi, int ip, int lxi, int let, int lze, int64_t &stride,
+__device__ __forceinline__ int64_t gc_point(int axis, int64_t fi, int ip, const GcFaces &g, int64_t &stride,
                                             int &dim) {
     int64_t base;
-    if (AXIS == 0) { base = fi * lxi; stride = 1; dim = lxi; }
-    else if (AXIS == 1) { base = (fi / lxi) * (int64_t)lxi * let + fi % lxi; stride = lxi; dim = let; }
-    else { base = fi; stride = (int64_t)lxi * let; dim = lze; }
+    if (axis == 0) { base = fi * g.lxi; stride = 1; dim = g.lxi; }
+    else if (axis == 1) { base = (fi / g.lxi) * (int64_t)g.lxi * g.let + fi % g.lxi; stride = g.lxi; dim = g.let; }
+    else { base = fi; stride = (int64_t)g.lxi * g.let; dim = g.lze; }
     return base + (int64_t)(ip ? dim - 1 : 0) * stride;
 }
 
-// gcbc_setup_kernel (src/cuda/kernels/gcbc.hpp:251-342): drva of face ip in
-// place into characteristic form, from drva (flag, non-reflective faces) or
+// gcbc_setup_kernel (src/cuda/kernels/gcbc.hpp:251-342): drva of every active
+// face in place into characteristic form, from drva (non-reflective faces) or
 // from the full right-hand side de (walls, curvilinear interfaces), times J.
-template <int AXIS>
-__global__ void k_gc_setup(double *__restrict__ drva, const double *__restrict__ cm, const double *__restrict__ qa,
-                           const double *__restrict__ de, const double *__restrict__ p,
-                           const double *__restrict__ yaco, double u0, double u1, double u2, int ip, int flag,
-                           int lxi, int let, int lze) {
-    const int64_t n = (int64_t)lxi * let * lze;
-    const int64_t F = AXIS == 0 ? (int64_t)let * lze : (AXIS == 1 ? (int64_t)lxi * lze : (int64_t)lxi * let);
-    const int64_t fi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_gc_setup(GcFaces gf, const double *__restrict__ qa, const double *__restrict__ de,
+                           const double *__restrict__ p, const double *__restrict__ yaco, double u0, double u1,
+                           double u2) {
+    const int64_t n = (int64_t)gf.lxi * gf.let * gf.lze;
+    const int axis = gf.axis[blockIdx.y], ip = gf.ip[blockIdx.y], flag = gf.kind[blockIdx.y] == 0;
+    const int64_t F = gf.F[axis], fi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (fi >= F) return;
+    double *drva = gf.drva[axis];
+    const double *cm = gf.cm[axis];
     int64_t stride;
     int dim;
-    const int64_t idx = gc_point<AXIS>(fi, ip, lxi, let, lze, stride, dim);
+    const int64_t idx = gc_point(axis, fi, ip, gf, stride, dim);
     const double c[3] = {cm[(ip * 3 + 0) * F + fi], cm[(ip * 3 + 1) * F + fi], cm[(ip * 3 + 2) * F + fi]};
     const GcPt g = gc_eleme(c, qa[idx], qa[n + idx], qa[2 * n + idx], qa[3 * n + idx], p[idx], u0, u1, u2);
     double L[5][5], src[5], cha[5];
@@ -364,26 +373,32 @@ __global__ void k_gc_setup(double *__restrict__ drva, const double *__restrict__
     for (int v = 0; v < 5; ++v) drva[(ip * 5 + v) * F + fi] = cha[v];
 }
 
-// The update kernels (src/cuda/kernels/gcbc.hpp:344-695) for one face:
-// kind 0 non-reflective (incoming acoustic waves zeroed), 1 wall (incoming
-// acoustic wave reflected from the outgoing one with the frame acceleration
-// and the normal velocity relaxed at rate dtwi), 2 curvilinear interface
-// (incoming waves from the neighbour's drvb).  de += sbcc xtr2q (cha - drva)
-// on kMbci planes; the wall update subtracts drva like the other two (the
-// reference's wall kernel adds xtr2q cha, the whole right-hand side).
-template <int AXIS>
-__global__ void k_gc_update(int kind, const double *__restrict__ drva, const double *__restrict__ drvb,
-                            const double *__restrict__ cm, const double *__restrict__ qa, double *__restrict__ de,
+// The update kernels (src/cuda/kernels/gcbc.hpp:344-695) for the faces f0 ..
+// f0 + gridDim.y - 1: kind 0 non-reflective (incoming acoustic waves zeroed), 1
+// wall (incoming acoustic wave reflected from the outgoing one with the frame
+// acceleration and the normal velocity relaxed at rate dtwi), 2 curvilinear
+// interface (incoming waves from the neighbour's drvb).  de += sbcc xtr2q (cha
+// - drva) on kMbci planes; the wall update subtracts drva like the other two
+// (the reference's wall kernel adds xtr2q cha, the whole right-hand side).
+// A thread handles one plane of one face point: the four planes in turn were
+// four dependent memory round trips (8 us a face however small the face).  On
+// x faces the planes of a point are neighbouring threads, on y and z faces
+// neighbouring warps, so that a warp's accesses stay together.
+__global__ void k_gc_update(GcFaces gf, int f0, const double *__restrict__ qa, double *__restrict__ de,
                             const double *__restrict__ p, const double *__restrict__ sbcc, double u0, double u1,
-                            double u2, double a0, double a1, double a2, double dtwi, int ip, int lxi, int let,
-                            int lze) {
-    const int64_t n = (int64_t)lxi * let * lze;
-    const int64_t F = AXIS == 0 ? (int64_t)let * lze : (AXIS == 1 ? (int64_t)lxi * lze : (int64_t)lxi * let);
-    const int64_t fi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                            double u2, double a0, double a1, double a2, double dtwi) {
+    static_assert(kMbci == 4, "128 threads: 32 face points by 4 planes");
+    const int64_t n = (int64_t)gf.lxi * gf.let * gf.lze;
+    const int face = f0 + blockIdx.y, axis = gf.axis[face], ip = gf.ip[face], kind = gf.kind[face];
+    const int ii = axis == 0 ? threadIdx.x & 3 : threadIdx.x >> 5;
+    const int64_t F = gf.F[axis];
+    const int64_t fi = (int64_t)blockIdx.x * 32 + (axis == 0 ? threadIdx.x >> 2 : threadIdx.x & 31);
     if (fi >= F) return;
     int64_t stride;
     int dim;
-    const int64_t idx = gc_point<AXIS>(fi, ip, lxi, let, lze, stride, dim);
+    const int64_t idx = gc_point(axis, fi, ip, gf, stride, dim);
+    if (ii >= dim) return;
+    const double *drva = gf.drva[axis], *drvb = gf.drvb[axis], *cm = gf.cm[axis];
     const double c[3] = {cm[(ip * 3 + 0) * F + fi], cm[(ip * 3 + 1) * F + fi], cm[(ip * 3 + 2) * F + fi]};
     const double rho = qa[idx];
     const GcPt g = gc_eleme(c, rho, qa[n + idx], qa[2 * n + idx], qa[3 * n + idx], p[idx], u0, u1, u2);
@@ -412,12 +427,13 @@ __global__ void k_gc_update(int kind, const double *__restrict__ drva, const dou
     double S[5][5], dq[5];
     gc_xtr2q(g, S);
     gc_matvec(S, cha, dq);
-    const int iq = 1 - 2 * ip;
-    for (int ii = 0; ii < kMbci && ii < dim; ++ii) {
-        const int64_t o = idx + (int64_t)ii * iq * stride;
+    const int64_t o = idx + (int64_t)ii * (1 - 2 * ip) * stride;
+    const double sb = sbcc[o];
+    double r[5];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) de[v * n + o] += xmul(sbcc[o], dq[v]);
-    }
+    for (int v = 0; v < 5; ++v) r[v] = de[v * n + o];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) de[v * n + o] = r[v] + xmul(sb, dq[v]);
 }
 
 // Primitive recovery into the reference's de slots (the empty slot of the
@@ -454,14 +470,20 @@ static int check_physics(const cs_physics *ph, const cs_numerics *nm, const cs_d
     if (!ph) return set_error(CS_ERR_INVALID, "null physics object");
     if (d.lmx != ph->d.lmx || d.lxi != ph->d.lxi || d.let != ph->d.let || d.lze != ph->d.lze)
         return set_error(CS_ERR_INVALID, "dims differ from the physics object");
-    if (nm) {
-        int ndf[2][3];
-        if (cs_get_ndf(nm, ndf)) return CS_ERR_INVALID;
-    }
+    if (nm && (d.lmx != nm->d.lmx || d.lxi != nm->d.lxi || d.let != nm->d.let || d.lze != nm->d.lze))
+        return set_error(CS_ERR_INVALID, "dims differ from the numerics object");
     return CS_OK;
 }
 
 inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
+
+// Zero derivatives along a degenerate axis for variables m0 .. 4.
+static int zero_deriv(cs_physics *ph, int m0, int axis, cudaStream_t st) {
+    const int64_t n = ph->d.lmx;
+    for (int m = m0; m < 5; ++m)
+        CSB_CUDA(cudaMemsetAsync(ph->buffer_deriv + (m * 3 + axis) * n, 0, n * sizeof(double), st));
+    return CS_OK;
+}
 
 }  // namespace csb
 
@@ -472,9 +494,12 @@ using namespace csb;
 // npex == 0 get, inviscid, rho E = rho^gamma / (gamma (gamma-1)) + |m|^2 / (2 rho)
 // (isentropic pressure, momentum kept); viscous, m = -rho umf and
 // rho E = rho / (gamma (gamma-1)) + |m|^2 / (2 rho) with the updated m
-// (isothermal wall, T = 1).  plane = ip * (n - 1).
+// (isothermal wall, T = 1).  plane = ip * (n - 1); code: the wall codes of the
+// axis' two faces (0: not a wall), one face per blockIdx.y.
 __global__ void k_wall_face(double *__restrict__ q, const int *__restrict__ npex, double u0, double u1, double u2,
-                            int lxi, int let, int64_t lmx, int axis, int plane, int viscous, int64_t nf) {
+                            int lxi, int let, int64_t lmx, int axis, int last, int2 code, int64_t nf) {
+    const int face = code.x && code.y ? (int)blockIdx.y : (code.x ? 0 : 1), plane = face * last;
+    const bool viscous = (face ? code.y : code.x) == CS_BC_WALL_VISCOUS;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nf) return;
     int64_t idx;
@@ -509,7 +534,6 @@ int cs_physics_create(cs_physics **out, cs_dcomp d, int viscous) {
               cudaMalloc(&ph->buffer_deriv, 15 * n * sizeof(double)) == cudaSuccess &&
               cudaMalloc(&ph->tau, 6 * n * sizeof(double)) == cudaSuccess &&
               cudaMalloc(&ph->heat, 3 * n * sizeof(double)) == cudaSuccess &&
-              cudaMalloc(&ph->ss, 3 * n * sizeof(double)) == cudaSuccess &&
               cudaMalloc(&ph->dt_acc, 2 * sizeof(double)) == cudaSuccess;
     if (!ok) {
         cs_physics_destroy(ph);
@@ -526,7 +550,7 @@ int cs_physics_create(cs_physics **out, cs_dcomp d, int viscous) {
 int cs_physics_destroy(cs_physics *ph) {
     if (!ph) return CS_OK;
     for (void *p : {(void *)ph->buffer, (void *)ph->buffer_deriv, (void *)ph->tau, (void *)ph->heat,
-                    (void *)ph->ss, (void *)ph->dt_acc})
+                    (void *)ph->dt_acc})
         if (p) cudaFree(p);
     delete ph;
     return CS_OK;
@@ -568,25 +592,24 @@ int cs_calc_fluxes(cs_physics *ph, cs_numerics *nm, const double *qa, const doub
     if (int rc = check_physics(ph, nm, d)) return rc;
     if (!nm) return set_error(CS_ERR_INVALID, "null numerics object");
     if (int rc = cs_calc_fluxes_pre(ph, qa, p, de, xim, etm, zem, stream)) return rc;
-    int ndf[2][3];
-    cs_get_ndf(nm, ndf);
-    if (int rc = cs_fill_buffers(nm, ph->buffer, 0, 5, 0, d, stream)) return rc;
     const int64_t n = d.lmx;
-    for (unsigned m = 0; m < 5; ++m) {
-        if (int rc = cs_halo_exchange_self(nm, m, stream)) return rc;
-        for (int a = 0; a < 3; ++a) {
-            if ((a == 0 ? d.lxi : (a == 1 ? d.let : d.lze)) == 1) {
-                CSB_CUDA(cudaMemsetAsync(ph->buffer_deriv + (m * 3 + a) * n, 0, n * sizeof(double),
-                                         (cudaStream_t)stream));
-                continue;
-            }
-            if (int rc = cs_deriv(nm, a, ph->buffer + m * 3 * n, ph->buffer_deriv + m * 3 * n, ndf[0][a],
-                                  ndf[1][a], d, m, a, a, CS_HALO_RECV, stream))
-                return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (int rc = exchange_self(nm, ph->buffer, 3 * n, n, 5, 0, st)) return rc;
+    const int dims[3] = {d.lxi, d.let, d.lze};
+    // de from the last derivative's launch, where z is not degenerate
+    const DerivSum sum{ph->buffer_deriv, ph->buffer_deriv + n, de, 3 * n, n};
+    for (int a = 0; a < 3; ++a) {
+        if (dims[a] == 1) {
+            if (int rc = zero_deriv(ph, 0, a, st)) return rc;
+        } else if (int rc = deriv_fields(nm, a, ph->buffer + a * n, 3 * n, ph->buffer_deriv + a * n, 3 * n, 5, 0,
+                                         a == 2 ? &sum : nullptr, st)) {
+            return rc;
         }
     }
-    k_fluxes_post<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(de, ph->buffer_deriv, n);
-    CSB_CUDA(cudaGetLastError());
+    if (d.lze == 1) {
+        k_fluxes_post<<<blocks_for(n, 256), 256, 0, st>>>(de, ph->buffer_deriv, n);
+        CSB_CUDA(cudaGetLastError());
+    }
     return CS_OK;
 }
 
@@ -599,23 +622,18 @@ int cs_calc_viscous_shear_stress(cs_physics *ph, cs_numerics *nm, double *de, co
     cudaStream_t st = (cudaStream_t)stream;
     k_visc_init<<<blocks_for(n, 256), 256, 0, st>>>(ph->buffer, de, n);
     CSB_CUDA(cudaGetLastError());
-    int ndf[2][3];
-    cs_get_ndf(nm, ndf);
-    if (int rc = cs_fill_buffers(nm, ph->buffer, 1, 5, 1, d, stream)) return rc;
-    for (unsigned m = 1; m < 5; ++m) {
-        if (int rc = cs_halo_exchange_self(nm, m, stream)) return rc;
-        for (int a = 0; a < 3; ++a) {
-            if ((a == 0 ? d.lxi : (a == 1 ? d.let : d.lze)) == 1) {
-                CSB_CUDA(cudaMemsetAsync(ph->buffer_deriv + (m * 3 + a) * n, 0, n * sizeof(double), st));
-                continue;
-            }
-            if (int rc = cs_deriv(nm, a, ph->buffer + m * 3 * n, ph->buffer_deriv + m * 3 * n, ndf[0][a],
-                                  ndf[1][a], d, m, 0, a, CS_HALO_RECV, stream))
-                return rc;
+    if (int rc = exchange_self(nm, ph->buffer + 3 * n, 3 * n, 0, 4, 1, st)) return rc;
+    const int dims[3] = {d.lxi, d.let, d.lze};
+    for (int a = 0; a < 3; ++a) {
+        if (dims[a] == 1) {
+            if (int rc = zero_deriv(ph, 1, a, st)) return rc;
+        } else if (int rc = deriv_fields(nm, a, ph->buffer + 3 * n, 3 * n, ph->buffer_deriv + (3 + a) * n, 3 * n, 4,
+                                         1, nullptr, st)) {
+            return rc;
         }
     }
-    k_visc_post<<<blocks_for(n, 256), 256, 0, st>>>(ph->tau, ph->heat, ph->ss, ph->buffer_deriv, xim, etm, zem, n);
-    k_visc_final<<<blocks_for(n, 256), 256, 0, st>>>(de, ph->tau, ph->heat, ph->ss, ssk, yaco, n);
+    k_visc_stress<<<blocks_for(n, 256), 256, 0, st>>>(de, ph->tau, ph->heat, ph->buffer_deriv, ssk, xim, etm, zem,
+                                                     yaco, n);
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
 }
@@ -627,9 +645,10 @@ int cs_calc_time_step(cs_physics *ph, const double *xim, const double *etm, cons
     if ((int64_t)size != ph->d.lmx) return set_error(CS_ERR_INVALID, "size %zu != lmx", size);
     cudaStream_t st = (cudaStream_t)stream;
     CSB_CUDA(cudaMemsetAsync(ph->dt_acc, 0, 2 * sizeof(double), st));
-    k_time_step<<<blocks_for((int64_t)size, 256), 256, 0, st>>>(xim, etm, zem, de, yaco, ssk, ph->umf[0],
-                                                               ph->umf[1], ph->umf[2],
-                                                               (unsigned long long *)ph->dt_acc, (int64_t)size);
+    const unsigned blocks = blocks_for((int64_t)size, 256);
+    k_time_step<<<blocks < kTimeStepBlocks ? blocks : kTimeStepBlocks, 256, 0, st>>>(
+        xim, etm, zem, de, yaco, ssk, ph->umf[0], ph->umf[1], ph->umf[2], (unsigned long long *)ph->dt_acc,
+        (int64_t)size);
     CSB_CUDA(cudaGetLastError());
     double h[2];
     CSB_CUDA(cudaMemcpyAsync(h, ph->dt_acc, sizeof h, cudaMemcpyDeviceToHost, st));
@@ -644,16 +663,24 @@ int cs_wall_condition_update(double *q, const int *npex, const double umf[3], cs
     if (!q || !npex || !umf || !nbc) return set_error(CS_ERR_INVALID, "null argument");
     if (d.lxi < 1 || d.let < 1 || d.lze < 1 || d.lmx != d.lxi * d.let * d.lze) return set_error(CS_ERR_INVALID, "dims");
     const int dims[3] = {d.lxi, d.let, d.lze};
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 3; ++a) {
+        int code[2];
         for (int ip = 0; ip < 2; ++ip) {
-            const int code = nbc[ip][a];
-            if (code != CS_BC_WALL_INVISCID && code != CS_BC_WALL_VISCOUS) continue;
-            const int64_t nf = (int64_t)d.lmx / dims[a];
-            k_wall_face<<<blocks_for(nf, 256), 256, 0, (cudaStream_t)stream>>>(
-                q, npex, umf[0], umf[1], umf[2], d.lxi, d.let, d.lmx, a, ip * (dims[a] - 1),
-                code == CS_BC_WALL_VISCOUS ? 1 : 0, nf);
+            const int np = nbc[ip][a];
+            code[ip] = np == CS_BC_WALL_INVISCID || np == CS_BC_WALL_VISCOUS ? np : 0;
+        }
+        if (!code[0] && !code[1]) continue;
+        const int64_t nf = (int64_t)d.lmx / dims[a];
+        // both faces in one launch; a one-point axis takes them in turn
+        const bool both = code[0] && code[1] && dims[a] > 1;
+        for (int ip = 0; ip < (both ? 1 : 2); ++ip) {
+            if (!both && !code[ip]) continue;
+            const int2 cd = both ? make_int2(code[0], code[1]) : make_int2(ip ? 0 : code[0], ip ? code[1] : 0);
+            k_wall_face<<<dim3(blocks_for(nf, 256), both ? 2u : 1u), 256, 0, (cudaStream_t)stream>>>(
+                q, npex, umf[0], umf[1], umf[2], d.lxi, d.let, d.lmx, a, dims[a] - 1, cd, nf);
             CSB_CUDA(cudaGetLastError());
         }
+    }
     return CS_OK;
 }
 
@@ -725,18 +752,31 @@ int cs_gcbc_apply(double *const drva[3], double *const cm[3], double *const drvb
             if (!drva[a] || !cm[a]) return set_error(CS_ERR_INVALID, "drva[%d] / cm[%d] is null", a, a);
             if (np == CS_BC_INTER_CURV && !drvb[a]) return set_error(CS_ERR_INVALID, "drvb[%d] is null", a);
         }
-    // 1. characteristic form of drva (gcbc_setup_kernel)
-    for (int a = 0; a < 3; ++a)
+    GcFaces gf{};
+    int nf = 0;
+    for (int a = 0; a < 3; ++a) {
+        gf.drva[a] = drva[a];
+        gf.drvb[a] = drvb[a];
+        gf.cm[a] = cm[a];
+        gf.F[a] = F[a];
         for (int ip = 0; ip < 2; ++ip) {
             const int np = nbc[ip][a];
             if (!gc_active(np)) continue;
-            const int flag = np == CS_BC_NON_REFLECTIVE;
-            const unsigned b = blocks_for(F[a], 128);
-            if (a == 0) k_gc_setup<0><<<b, 128, 0, st>>>(drva[a], cm[a], qa, de, p, yaco, umf[0], umf[1], umf[2], ip, flag, d.lxi, d.let, d.lze);
-            else if (a == 1) k_gc_setup<1><<<b, 128, 0, st>>>(drva[a], cm[a], qa, de, p, yaco, umf[0], umf[1], umf[2], ip, flag, d.lxi, d.let, d.lze);
-            else k_gc_setup<2><<<b, 128, 0, st>>>(drva[a], cm[a], qa, de, p, yaco, umf[0], umf[1], umf[2], ip, flag, d.lxi, d.let, d.lze);
-            CSB_CUDA(cudaGetLastError());
+            gf.axis[nf] = a;
+            gf.ip[nf] = ip;
+            gf.kind[nf++] = np == CS_BC_NON_REFLECTIVE ? 0 : (np == CS_BC_INTER_CURV ? 2 : 1);
         }
+    }
+    if (nf == 0) return CS_OK;
+    gf.lxi = d.lxi;
+    gf.let = d.let;
+    gf.lze = d.lze;
+    int64_t Fmax = 0;
+    for (int k = 0; k < nf; ++k) Fmax = F[gf.axis[k]] > Fmax ? F[gf.axis[k]] : Fmax;
+    // 1. characteristic form of drva (gcbc_setup_kernel): reads qa and de,
+    //    writes each face's own drva
+    k_gc_setup<<<dim3(blocks_for(Fmax, 128), (unsigned)nf), 128, 0, st>>>(gf, qa, de, p, yaco, umf[0], umf[1], umf[2]);
+    CSB_CUDA(cudaGetLastError());
     // 2. GCIC exchange (src/gcbc.hpp:132-157): the neighbour across face ip
     //    is the block itself, adjacent through its face 1 - ip
     for (int a = 0; a < 3; ++a)
@@ -744,19 +784,17 @@ int cs_gcbc_apply(double *const drva[3], double *const cm[3], double *const drvb
             if (nbc[ip][a] == CS_BC_INTER_CURV)
                 CSB_CUDA(cudaMemcpyAsync(drvb[a] + (int64_t)ip * 5 * F[a], drva[a] + (int64_t)(1 - ip) * 5 * F[a],
                                          5 * F[a] * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    // 3. update kernels
-    for (int a = 0; a < 3; ++a)
-        for (int ip = 0; ip < 2; ++ip) {
-            const int np = nbc[ip][a];
-            if (!gc_active(np)) continue;
-            const int kind = np == CS_BC_NON_REFLECTIVE ? 0 : (np == CS_BC_INTER_CURV ? 2 : 1);
-            const unsigned b = blocks_for(F[a], 128);
-            const double *db = drvb[a];
-            if (a == 0) k_gc_update<0><<<b, 128, 0, st>>>(kind, drva[a], db, cm[a], qa, de, p, sbcc, umf[0], umf[1], umf[2], dudtmf[0], dudtmf[1], dudtmf[2], dtwi, ip, d.lxi, d.let, d.lze);
-            else if (a == 1) k_gc_update<1><<<b, 128, 0, st>>>(kind, drva[a], db, cm[a], qa, de, p, sbcc, umf[0], umf[1], umf[2], dudtmf[0], dudtmf[1], dudtmf[2], dtwi, ip, d.lxi, d.let, d.lze);
-            else k_gc_update<2><<<b, 128, 0, st>>>(kind, drva[a], db, cm[a], qa, de, p, sbcc, umf[0], umf[1], umf[2], dudtmf[0], dudtmf[1], dudtmf[2], dtwi, ip, d.lxi, d.let, d.lze);
-            CSB_CUDA(cudaGetLastError());
-        }
+    // 3. update kernels, in the order of the faces: planes of different axes
+    //    share points, the two faces of one axis only on lines shorter than
+    //    their planes
+    for (int k = 0; k < nf;) {
+        const int a = gf.axis[k];
+        const int pair = k + 1 < nf && gf.axis[k + 1] == a && dims[a] >= 2 * kMbci ? 2 : 1;
+        k_gc_update<<<dim3(blocks_for(F[a], 32), (unsigned)pair), 128, 0, st>>>(
+            gf, k, qa, de, p, sbcc, umf[0], umf[1], umf[2], dudtmf[0], dudtmf[1], dudtmf[2], dtwi);
+        CSB_CUDA(cudaGetLastError());
+        k += pair;
+    }
     return CS_OK;
 }
 

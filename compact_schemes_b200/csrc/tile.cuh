@@ -121,6 +121,39 @@ __device__ __forceinline__ void tile_sync() {
     else __syncthreads();
 }
 
+// Vector access of VB bytes (16 or 32) to a lane's own chunk.
+template <int VB, typename T>
+__device__ __forceinline__ void load_vec(const T *p, T *v) {
+    if constexpr (VB == 32 && sizeof(T) == 8) {
+        asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p) : "memory");
+    } else if constexpr (VB == 32) {
+        asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+            : "l"(p) : "memory");
+    } else if constexpr (sizeof(T) == 8) {
+        const double2 x = *reinterpret_cast<const double2 *>(p);
+        v[0] = x.x; v[1] = x.y;
+    } else {
+        const float4 x = *reinterpret_cast<const float4 *>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    }
+}
+template <int VB, typename T>
+__device__ __forceinline__ void store_vec(T *p, const T *v) {
+    if constexpr (VB == 32 && sizeof(T) == 8) {
+        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                     : "memory");
+    } else if constexpr (VB == 32) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
+                     "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+    } else if constexpr (sizeof(T) == 8) {
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    } else {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
 }  // namespace csb
 
 namespace csb {

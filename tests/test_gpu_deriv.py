@@ -134,6 +134,31 @@ def test_deriv_row_and_column_lengths(cuda, n, closure):
         nm.close()
 
 
+@pytest.mark.parametrize("closure", [45, 10])
+@pytest.mark.parametrize("n", [7, 9, 16, 33, 34, 64, 66, 127, 132, 256, 260, 511, 1000])
+def test_filter_lengths(cuda, n, closure):
+    """The filter at lengths around the chunk, tile and vector-access edges,
+    along every axis, in place and out of place, on and off a 16-byte boundary."""
+    import torch
+    nd = int(closure == 45)
+    for axis in range(3):
+        dims = [9, 8, 10]
+        dims[axis] = n
+        nm = make(cuda, tuple(dims), [[closure] * 3] * 2)
+        f = field(dims, 4)
+        ref = O.filt(f, dims, axis, nd, nd, alpha_f=0.4)
+        for off in (0, 1):
+            buf = torch.zeros(f.size + off, dtype=torch.float64, device=cuda)
+            buf[off:] = torch.from_numpy(f).to(cuda)
+            out = torch.full((f.size + off + 5,), 7.0, dtype=torch.float64, device=cuda)
+            nm.filter(axis, buf[off:], out[off:], 0.4, nm.dcomp)
+            assert relerr(out[off:off + f.size].cpu().numpy(), ref) < TOL, (axis, off)
+            assert bool((out[:off] == 7.0).all()) and bool((out[off + f.size:] == 7.0).all())
+            nm.filter(axis, buf[off:], buf[off:], 0.4, nm.dcomp)
+            assert bool((buf[off:] == out[off:off + f.size]).all()), (axis, off)
+        nm.close()
+
+
 def test_deriv_fp32(cuda):
     import torch
     import compact_schemes_b200 as cs
