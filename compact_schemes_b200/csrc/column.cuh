@@ -22,10 +22,12 @@ namespace csb {
 // Shared-memory slots of one field of a tile: row t of chunk c of line l.  The
 // odd chunk stride lets a warp read one line's 32 chunk ends without bank
 // conflicts, and threads (l, c) write their rows with at most a 2-way one.
-template <int LT, int TL>
+// P: chunk slots per line (lines of at most P chunks).
+template <int LT, int TL, int P = 32>
 struct Column {
     static constexpr int kChunk = TL + 1;
-    static constexpr int kRow = 32 * kChunk;
+    static constexpr int kRow = P * kChunk;
+    static constexpr int kSlots = P;
     static constexpr int kField = LT * kRow;
     __device__ __forceinline__ static int at(int t, int c, int l) { return t * kRow + c * kChunk + l; }
     __device__ __forceinline__ static int pos(int j, int l) { return at(j % LT, j / LT, l); }
@@ -42,10 +44,9 @@ inline int column_threads(int tl, int p) { return (tl * p + 31) / 32 * 32; }
 // are received values recv[k F + line0 + f TL + l] instead (the fields are then
 // TL-line groups of one field).  CT: type the sums are formed in.  All threads of the tile call it; the caller
 // synchronizes before the rows are read.
-template <int LT, int TL, int NF, typename T, typename CT = T>
+template <int LT, int TL, int NF, typename T, typename CT = T, typename C = Column<LT, TL>>
 __device__ __forceinline__ void column_closure_rows(const T *V, CT *rows, int n, const Coeffs &cf, const CT *recv,
                                                     int F, int line0) {
-    using C = Column<LT, TL>;
     static_assert(NF * TL * 8 % 32 == 0, "whole warps");
     for (int i = threadIdx.x; i < NF * TL * 8; i += blockDim.x) {
         const int g = i >> 3, d = i & 7, f = g / TL, l = g % TL;
@@ -69,9 +70,8 @@ __device__ __forceinline__ void column_closure_rows(const T *V, CT *rows, int n,
 
 // Write the rows of a chunk that other threads read: the two at either end
 // (the neighbours' stencils), all of them near the line's ends (the closure).
-template <int LT, int TL, typename T>
+template <int LT, int TL, typename T, typename C = Column<LT, TL>>
 __device__ __forceinline__ void column_put_raw(T *V, const T (&d)[LT], int c, int l, int n) {
-    using C = Column<LT, TL>;
     V[C::at(0, c, l)] = d[0];
     V[C::at(1, c, l)] = d[1];
     if (LT > 2) V[C::at(LT - 2, c, l)] = d[LT - 2];
@@ -87,11 +87,10 @@ __device__ __forceinline__ void column_put_raw(T *V, const T (&d)[LT], int c, in
 // Rows of the physical closure are formed here; rows of the interface closure
 // are put in by column_take_rows once column_closure_rows has run.  Slots
 // outside the line are read but only reach rows that are replaced.
-template <int LT, int TL, typename T>
+template <int LT, int TL, typename T, typename C = Column<LT, TL>>
 __device__ __forceinline__ void column_rhs(const T *V, int c, int l, int len, int n, int nstart, int nend,
                                            T (&d)[LT]) {
-    using C = Column<LT, TL>;
-    const int cm = c > 0 ? c - 1 : 0, cp = c < 31 ? c + 1 : 31;
+    const int cm = c > 0 ? c - 1 : 0, cp = c < C::kSlots - 1 ? c + 1 : C::kSlots - 1;
     T w[LT + 4];
     w[0] = V[C::at(LT - 2, cm, l)];
     w[1] = V[C::at(LT - 1, cm, l)];
@@ -110,9 +109,8 @@ __device__ __forceinline__ void column_take_rows(const T *rows, int c, int n, in
 }
 
 // Write an eliminated chunk's end rows where the line's warp reads them.
-template <int LT, int TL, typename T>
+template <int LT, int TL, typename T, typename C = Column<LT, TL>>
 __device__ __forceinline__ void column_put_ends(T *V, const T (&d)[LT], int c, int l, int len) {
-    using C = Column<LT, TL>;
     V[C::at(0, c, l)] = d[0];
     if (len == LT) V[C::at(LT - 1, c, l)] = d[LT - 1];
     else if (len >= 2) V[C::at(len - 1, c, l)] = get_at<LT, T>(d, len - 1);
@@ -122,9 +120,8 @@ __device__ __forceinline__ void column_put_ends(T *V, const T (&d)[LT], int c, i
 // fields of it together), in place of the chunks' end rows.  beta != nullptr
 // (cyclic systems): the factor of the Sherman-Morrison correction per field and
 // line.
-template <int LT, int TL, int NF, typename T>
+template <int LT, int TL, int NF, typename T, typename C = Column<LT, TL>>
 __device__ __forceinline__ void column_reduced(T *V, const DevTables<T> &tab, T *beta = nullptr) {
-    using C = Column<LT, TL>;
     const int lane = threadIdx.x & 31, len = lane_len(lane, LT, tab.p, tab.last_len);
     for (int l = threadIdx.x >> 5; l < TL; l += blockDim.x >> 5) {
         T *lo = V + C::at(0, lane, l), *hi = V + C::at(len >= 2 ? len - 1 : 0, lane, l);
@@ -149,9 +146,8 @@ __device__ __forceinline__ void column_reduced(T *V, const DevTables<T> &tab, T 
 }
 
 // The solution of this thread's chunk from its end values in V.
-template <int LT, int TL, typename T>
+template <int LT, int TL, typename T, typename C = Column<LT, TL>>
 __device__ __forceinline__ void column_finish(const T *V, const DevTables<T> &tab, int c, int l, int len, T (&d)[LT]) {
-    using C = Column<LT, TL>;
     const T X0 = V[C::at(0, c, l)];
     const T X1 = V[C::at(len >= 2 ? len - 1 : 0, c, l)];
     chunk_substitute<LT, T>(tab, d, X0, X1, c, len);

@@ -156,6 +156,7 @@ struct cs_solver {
     int can[2][3] = {{0, 0, 0}, {0, 0, 0}};    // feasible schedules: 1 tile 8, 2 tile 16, 4 pipelined,
                                                // 8 TMA-staged (gradient passes)
     int tma[3] = {0, 0, 0};                    // gradient pass along each axis stages its pencils by TMA
+    int merge = 1;                             // x gradient and flux in one launch where it applies
     int *err = nullptr;                        // device word: nonzero if a TMA staging copy timed out
     const DeviceTables *ftab[3] = {nullptr, nullptr, nullptr};  // filter tables (cfg.filter)
     int nsm = 0;
@@ -319,14 +320,23 @@ static bool gcbc_on(const cs_solver *s) {
            (s->cfg.nbc[0][0] == CS_BC_NON_REFLECTIVE || s->cfg.nbc[1][0] == CS_BC_NON_REFLECTIVE);
 }
 
+// Whether a stage's x gradient and flux passes run as one launch: both
+// one-phase, another axis to finish the stage, rows that k_gradflux_row takes.
+static bool merged_x(cs_solver *s, const double *q, const double *rhs) {
+    if (!s->merge || !s->active[0] || !(s->active[1] || s->active[2]) || s->pl[0][0] || s->pl[1][0] || s->tma[0])
+        return false;
+    return gradflux_vec(pass_args(s, 0, 1), q, rhs) != 0;
+}
+
 // RHS of one state (rk == nullptr) or one full RK stage.
 static int run_stage(cs_solver *s, const double *qin, const double *qn, double *qout, double *rhs_out,
                      const RkParams *rk, bool dtred, cudaStream_t st) {
     int axes[3], na = 0;
     for (int a = 0; a < 3; ++a)
         if (s->active[a]) axes[na++] = a;
+    const bool merged = merged_x(s, qin, rhs_out ? rhs_out : s->rhs);
     if (s->cfg.viscous)
-        for (int i = 0; i < na; ++i)
+        for (int i = merged ? 1 : 0; i < na; ++i)
             if (int rc = grad_pass(s, axes[i], qin, dtred && i == 0, st)) return rc;
     if (dtred && !s->cfg.viscous) {
         // inviscid: the CFL maxima come from a gradient-free reduction; reuse
@@ -343,7 +353,13 @@ static int run_stage(cs_solver *s, const double *qin, const double *qn, double *
         else if (na == 1) mode = kWriteRk;
         else mode = i == 0 ? kWrite : (i == na - 1 ? kAccumRk : kAccum);
         double *drva = (a == 0 && gcbc_on(s)) ? s->drva : nullptr;
-        int rc = flux_pass(s, a, mode, qin, qn, qout, drva, rk ? *rk : none, st);
+        int rc;
+        if (merged && i == 0) {
+            PassTimer pt(s, st, kPassFluxX);
+            rc = launch_gradflux_x(pass_args(s, 0, 1), qin, drva, dtred, st);
+        } else {
+            rc = flux_pass(s, a, mode, qin, qn, qout, drva, rk ? *rk : none, st);
+        }
         if (rc) { s->rhs = saved_rhs; return rc; }
         if (drva && (mode == kWrite || mode == kAccum) && !(rk && na == 1)) {
             PassTimer pt(s, st, kPassGcbc);
@@ -638,11 +654,16 @@ int cs_solver_autotune(cs_solver *s, const double *q, int reps, int choice[2][3]
         cs_solver_last_dt(s, &dt);
     }
     // per-point metrics run the one-phase kernels, or the TMA gradient passes
-    // (the metric-reading CFL reduction of the first then stays one-phase)
+    // (the metric-reading CFL reduction of the first then stays one-phase); the
+    // fifth candidate is the x gradient and flux in one launch, against the
+    // fastest two launches
     const int allowed = s->fm.xim ? 11 : 15;
-    for (int c = 0; c < 4 && rc == CS_OK && dt > 0.0; ++c) {
+    const int saved_merge = s->merge;
+    double merged_ms = 1e300;
+    for (int c = 0; c < 5 && rc == CS_OK && dt > 0.0; ++c) {
         const int bit = 1 << c;
-        if (!(allowed & bit)) continue;
+        if (c < 4 && !(allowed & bit)) continue;
+        s->merge = c == 4;
         for (int k = 0; k < 2; ++k)
             for (int a = 0; a < 3; ++a) {
                 const bool ok = (s->can[k][a] & bit) != 0;
@@ -653,6 +674,7 @@ int cs_solver_autotune(cs_solver *s, const double *q, int reps, int choice[2][3]
             }
         // one untimed step first: the first launch of a kernel may load its
         // module (lazy loading), which must not count against the schedule
+        if (c == 4 && (s->mixed || !merged_x(s, scratch, s->rhs))) break;
         rc = run_step(s, scratch, dt, st);
         if (rc) break;
         cs_solver_profile_begin(s);
@@ -661,6 +683,10 @@ int cs_solver_autotune(cs_solver *s, const double *q, int reps, int choice[2][3]
         int n[kPassKinds];
         if (rc == CS_OK) rc = cs_solver_profile_end(s, ms, n);
         if (rc) break;
+        if (c == 4) {
+            if (n[kPassFluxX] && !n[kPassGradX]) merged_ms = ms[kPassFluxX] / n[kPassFluxX];
+            break;
+        }
         for (int k = 0; k < 2; ++k)
             for (int a = 0; a < 3; ++a) {
                 const int kind = (k == 0 ? kPassGradX : kPassFluxX) + a;
@@ -671,6 +697,7 @@ int cs_solver_autotune(cs_solver *s, const double *q, int reps, int choice[2][3]
     }
     cudaFree(scratch);
     if (rc || !(dt > 0.0)) {
+        s->merge = saved_merge;
         for (int k = 0; k < 2; ++k)
             for (int a = 0; a < 3; ++a) {
                 s->tile[k][a] = saved_tile[k][a];
@@ -679,6 +706,8 @@ int cs_solver_autotune(cs_solver *s, const double *q, int reps, int choice[2][3]
             }
         return rc ? rc : set_error(CS_ERR_STATE, "autotune: no time step from the state");
     }
+    s->merge = merged_ms < best[0][0] + best[1][0];
+    if (s->merge) pick[0][0] = pick[1][0] = 8;
     for (int k = 0; k < 2; ++k)
         for (int a = 0; a < 3; ++a) {
             s->pl[k][a] = pick[k][a] == 0;

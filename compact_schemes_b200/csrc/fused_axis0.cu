@@ -17,4 +17,12 @@ int launch_flux<0>(const PassArgs &a, int mode, const double *q, const double *q
     return launch_flux_tl<0, 8>(a, mode, q, qn, qout, drva, rk, st);
 }
 
+int launch_gradflux_x(const PassArgs &a, const double *q, double *drva, bool dtred, cudaStream_t st) {
+    switch (a.tab->lt) {
+        case 2: return launch_gradflux_t<2>(a, q, drva, dtred, st);
+        case 4: return launch_gradflux_t<4>(a, q, drva, dtred, st);
+    }
+    return set_error(CS_ERR_UNSUPPORTED, "chunk length");
+}
+
 }  // namespace csb

@@ -5,9 +5,10 @@
 #include <cuda.h>
 
 #include <cmath>
+#include <type_traits>
 
+#include "column.cuh"
 #include "context.h"
-#include "tile.cuh"
 
 // Tuning knobs (compile-time; defaults chosen by measurement on B200):
 // points per thread loaded together in the load phase of the gradient / flux
@@ -33,6 +34,9 @@
 #endif
 #ifndef CSB_GRAD_SOLVE_GROUP
 #define CSB_GRAD_SOLVE_GROUP CSB_SOLVE_GROUP
+#endif
+#ifndef CSB_COL_BATCH
+#define CSB_COL_BATCH 2     // points per thread loaded together by the column gradient pass
 #endif
 #ifndef CSB_RMW_CHUNK
 #define CSB_RMW_CHUNK 4     // points per chunk when only R is read back
@@ -271,6 +275,54 @@ __device__ __forceinline__ void solve_fields(double *sm, int w, int lane, const 
     if constexpr (REM > 0) solve_field_group<LT, TL, NF, REM, ROWS>(sm, w, lane, tab, nstart, nend, cf, NFULL);
 }
 
+// The two maxima of calc_time_step_kernel (src/cuda/kernels/physics.hpp:335-427)
+// at one point.
+template <bool FM>
+__device__ __forceinline__ void cfl_terms(const Prim &s, const Phys &ph, const FieldMet &fm, int64_t lmx, int64_t gi,
+                                          double &m1, double &m2) {
+    const double uu = s.u + ph.umf[0], vv = s.v + ph.umf[1], ww = s.w + ph.umf[2];
+    const PointMet pm = point_met<FM>(ph, fm, lmx, gi);
+    double rr1 = ph.rr1;
+    if (FM) {
+        rr1 = 0.0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) rr1 += xmul(pm.M[a][c], pm.M[a][c]);
+    }
+    double rr2 = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) rr2 += fabs(xmul(pm.M[a][0], uu) + xmul(pm.M[a][1], vv) + xmul(pm.M[a][2], ww));
+    const double ssi = fabs(pm.J);
+    m1 = fmax(m1, xmul(sqrt(xmul(s.T, rr1)) + rr2, ssi));
+    m2 = fmax(m2, s.ri * ph.mu * rr1 * ssi * ssi);
+}
+
+// Reduce the block's CFL maxima into dtacc (all threads call it): one pair of
+// atomics per block, and none where a larger value is already there (the
+// accumulators only grow, so a stale read costs an atomic and nothing else).
+// Same-address atomics take 1.4 ns each on B200.
+__device__ __forceinline__ void cfl_reduce(double m1, double m2, unsigned long long *dtacc) {
+    __shared__ double red[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+        m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    }
+    if (lane == 0) {
+        red[0][w] = m1;
+        red[1][w] = m2;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double m = 0.0;
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) m = fmax(m, red[threadIdx.x][k]);
+        const unsigned long long b = (unsigned long long)__double_as_longlong(m);
+        if (b > __ldcg(dtacc + threadIdx.x)) atomicMax(dtacc + threadIdx.x, b);
+    }
+}
+
 // One tile of the gradient pass: lines line0 .. line0+TL-1 (TL * 32 threads;
 // sm holds 4 * TL line slots).  SG: fields per warp solve (0: the pass
 // default); ROWS: periodic closure rows formed lane-parallel (solve_fields).
@@ -293,26 +345,7 @@ __device__ __forceinline__ void grad_tile(double *sm, int64_t line0, const doubl
         field_line<LT, TL>(sm, 2, l)[pj] = s.w;
         field_line<LT, TL>(sm, 3, l)[pj] = s.T;
         if (DTRED) {
-            // calc_time_step_kernel (src/cuda/kernels/physics.hpp:335-427)
-            const double uu = s.u + ph.umf[0], vv = s.v + ph.umf[1], ww = s.w + ph.umf[2];
-            const PointMet pm = point_met<FM>(ph, fm, lmx, gi);
-            double rr1 = ph.rr1;
-            if (FM) {
-                rr1 = 0.0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) rr1 += xmul(pm.M[a][c], pm.M[a][c]);
-            }
-            double rr2 = 0.0;
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-                rr2 += fabs(xmul(pm.M[a][0], uu) + xmul(pm.M[a][1], vv) + xmul(pm.M[a][2], ww));
-            const double ssi = fabs(pm.J);
-            const double v1 = xmul(sqrt(xmul(s.T, rr1)) + rr2, ssi);
-            const double v2 = s.ri * ph.mu * rr1 * ssi * ssi;
-            m1 = fmax(m1, v1);
-            m2 = fmax(m2, v2);
+            cfl_terms<FM>(s, ph, fm, lmx, gi, m1, m2);
         }
     });
     tile_sync<AXIS, TL>();
@@ -350,6 +383,151 @@ k_grad(const double *__restrict__ q, double *__restrict__ g, DevTables<double> t
     extern __shared__ __align__(16) unsigned char smem_raw[];
     grad_tile<LT, AXIS, TL, DTRED, FM>(reinterpret_cast<double *>(smem_raw), (int64_t)blockIdx.x * TL, q, g, tab,
                                        lxi, let, lmx, F, nstart, nend, cf, ph, dtacc, fm);
+}
+
+// The gradient pass along y and z for lines of up to 256 points: column tiles
+// (column.cuh), thread (l, c) holding chunk c of line l for all four fields.
+// Bound by load latency at 16 warps per SM (128 registers): 256^3 0.37 ms, 3.3
+// TB/s, 128^3 68 us (a warp per line staged in shared memory: 82 us).
+// The tile of lines line0 .. line0 + TL - 1 (those below F); V holds 4 (kField +
+// 4 TL) values.
+template <int LT, int AXIS, int TL, int P, bool DTRED, bool FM>
+__device__ __forceinline__ void grad_col_tile(double *V, int line0, int F, const double *__restrict__ q,
+                                              double *__restrict__ g, const DevTables<double> &tab, int lxi, int let,
+                                              int64_t lmx, int nstart, int nend, const Coeffs &cf, const Phys &ph,
+                                              double &m1, double &m2, const FieldMet &fm = FieldMet{}) {
+    using C = Column<LT, TL, P>;
+    double *rows = V + 4 * C::kField;
+    const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL;
+    const int len = lane_len(c, LT, tab.p, tab.last_len);
+    const int s = AXIS == 1 ? lxi : lxi * let;
+    const int fidx = min(line0 + l, F - 1);  // past the last line: the last line again, not stored
+    const int base = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + c * LT * s;
+    double d[4][LT];
+    if (len > 0) {
+        constexpr int B = LT < 4 ? LT : CSB_COL_BATCH;  // points whose loads are in flight together
+#pragma unroll
+        for (int t0 = 0; t0 < LT; t0 += B) {
+            double qv[B][5];
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                const double *p = q + (base + min(t0 + b, len - 1) * s);  // past the chunk's end: its last point again
+#pragma unroll
+                for (int m = 0; m < 5; ++m) qv[b][m] = __ldg(p + m * lmx);
+            }
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                const Prim pr = primitives(qv[b][0], qv[b][1], qv[b][2], qv[b][3], qv[b][4]);
+                d[0][t0 + b] = pr.u;
+                d[1][t0 + b] = pr.v;
+                d[2][t0 + b] = pr.w;
+                d[3][t0 + b] = pr.T;
+                if (DTRED) cfl_terms<FM>(pr, ph, fm, lmx, base + min(t0 + b, len - 1) * s, m1, m2);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+#pragma unroll
+            for (int t = 0; t < LT; ++t) d[f][t] = 0.0;
+    }
+#pragma unroll
+    for (int f = 0; f < 4; ++f) column_put_raw<LT, TL, double, C>(V + f * C::kField, d[f], c, l, n);
+    __syncthreads();
+    if (nstart || nend) column_closure_rows<LT, TL, 4, double, double, C>(V, rows, n, cf, nullptr, F, line0);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) column_rhs<LT, TL, double, C>(V + f * C::kField, c, l, len, n, nstart, nend, d[f]);
+    __syncthreads();
+    if (nstart || nend) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) column_take_rows<LT, double>(rows + 4 * (f * TL + l), c, n, nstart, nend, d[f]);
+    }
+    chunk_eliminate<LT, 4, double>(tab, d, c);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) column_put_ends<LT, TL, double, C>(V + f * C::kField, d[f], c, l, len);
+    __syncthreads();
+    column_reduced<LT, TL, 4, double, C>(V, tab);
+    __syncthreads();
+    if (len > 0 && line0 + l < F) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            column_finish<LT, TL, double, C>(V + f * C::kField, tab, c, l, len, d[f]);
+            double *o = g + f * lmx + base;
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len) o[t * s] = d[f][t];
+        }
+    }
+}
+
+template <int LT, int AXIS, int TL, bool DTRED, bool FM>
+__global__ void __launch_bounds__(TL * 32, 512 / (TL * 32))
+k_grad_col(const double *__restrict__ q, double *__restrict__ g, DevTables<double> tab, int lxi, int let,
+           int64_t lmx, int F, int nstart, int nend, Coeffs cf, Phys ph, unsigned long long *__restrict__ dtacc,
+           FieldMet fm) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double m1 = 0.0, m2 = 0.0;
+    grad_col_tile<LT, AXIS, TL, 32, DTRED, FM>(reinterpret_cast<double *>(smem_raw), (int)blockIdx.x * TL, F, q, g,
+                                               tab, lxi, let, lmx, nstart, nend, cf, ph, m1, m2, fm);
+    if (DTRED) cfl_reduce(m1, m2, dtacc);
+}
+
+// The gradient pass along x for lines of up to 256 points whose rows are
+// multiples of VB bytes (k_deriv_row's form): a warp per line, each lane
+// loading its chunk of the five state fields with VB-byte vectors, the four
+// fields solved together, stored from the same registers (256^3 0.264 ms, 4.6
+// TB/s; staged in shared memory: 0.34 ms).
+template <int LT, int VB, bool DTRED, bool FM>
+__global__ void __launch_bounds__(256, 2)
+k_grad_row(const double *__restrict__ q, double *__restrict__ g, DevTables<double> tab, int64_t lmx, int F,
+           int nstart, int nend, Coeffs cf, Phys ph, unsigned long long *__restrict__ dtacc, FieldMet fm) {
+    constexpr int VE = VB / 8;
+    __shared__ double ends[8][4][2 * kLmd + 1];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int len = lane_len(lane, LT, tab.p, tab.last_len);
+    const int line = (int)blockIdx.x * 8 + w;
+    double m1 = 0.0, m2 = 0.0;
+    if (line < F) {
+        const int64_t base = (int64_t)line * n + lane * LT;
+        double d[4][LT];
+#pragma unroll
+        for (int t0 = 0; t0 < LT; t0 += VE) {
+            if (t0 < len) {
+                double qv[5][VE];
+#pragma unroll
+                for (int m = 0; m < 5; ++m) load_vec<VB, double>(q + m * lmx + base + t0, qv[m]);
+#pragma unroll
+                for (int b = 0; b < VE; ++b) {
+                    const Prim pr = primitives(qv[0][b], qv[1][b], qv[2][b], qv[3][b], qv[4][b]);
+                    d[0][t0 + b] = pr.u;
+                    d[1][t0 + b] = pr.v;
+                    d[2][t0 + b] = pr.w;
+                    d[3][t0 + b] = pr.T;
+                    if (DTRED) cfl_terms<FM>(pr, ph, fm, lmx, base + t0 + b, m1, m2);
+                }
+            } else {
+#pragma unroll
+                for (int f = 0; f < 4; ++f)
+#pragma unroll
+                    for (int b = 0; b < VE; ++b) d[f][t0 + b] = 0.0;
+            }
+        }
+        double rows = 0.0;  // lane 8 f + {0, 1, 4, 5}: interface rows 0, 1, n-1, n-2 of field f
+        if (nstart || nend) {
+            chunk_put_ends<LT, 4, double>(ends[w], d, lane, len, n);
+            __syncwarp();
+            rows = ends_closure_row<double>(ends[w][lane >> 3], lane & 7, cf);
+        }
+#pragma unroll
+        for (int f = 0; f < 4; ++f) chunk_warp_rhs<LT, double>(rows, f, lane, len, n, nstart, nend, d[f]);
+        warp_solve<LT, 4, double>(tab, d, lane);
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+#pragma unroll
+            for (int t = 0; t < LT; t += VE)
+                if (t < len) store_vec<VB, double>(g + f * lmx + base + t, &d[f][t]);
+    }
+    if (DTRED) cfl_reduce(m1, m2, dtacc);
 }
 
 // ----------------------------------------------------------------------------
@@ -544,6 +722,276 @@ k_flux(const double *__restrict__ q, const double *__restrict__ g, double *__res
 }
 
 
+// The store phase of a column flux tile: the derivative's rows from the
+// eliminated rows in V and the chunk's end values, P points at a time whose
+// read-modify-write loads are in flight together.
+template <bool INTERIOR, int LT, typename C, int MODE, bool FM, bool CG>
+__device__ __forceinline__ void flux_col_store(const double *V, const DevTables<double> &tab, int c, int l, int len,
+                                               int base, int s, int64_t lmx, double *rhs, const double *qn,
+                                               double *qout, double dtd, double dtk, const FieldMet &fm) {
+    constexpr int PW = CG || MODE == kWrite ? 1 : (MODE == kAccumRk ? CSB_RMW_CHUNK_RK : CSB_RMW_CHUNK);
+    constexpr int P = PW < LT ? PW : LT;
+    double X0[5], X1[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+        X0[m] = V[m * C::kField + C::at(0, c, l)];
+        X1[m] = V[m * C::kField + C::at(len >= 2 ? len - 1 : 0, c, l)];
+    }
+#pragma unroll
+    for (int t0 = 0; t0 < LT; t0 += P) {
+        double rv[P][5], qv[P][5], jv[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int gi = base + (t0 + p) * s;
+            if (t0 + p < len) {
+                if (FM && MODE >= kAccumRk) jv[p] = xmul(dtd, __ldg(fm.yaco + gi));
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    if (MODE == kAccum || MODE == kAccumRk) rv[p][m] = CG ? __ldcg(rhs + m * lmx + gi) : rhs[m * lmx + gi];
+                    if (MODE >= kAccumRk) qv[p][m] = qn[m * lmx + gi];
+                }
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int t = t0 + p, gi = base + t * s;
+            if (t < len) {
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    const double dfv = chunk_row<INTERIOR, LT, double>(tab, t, V[m * C::kField + C::at(t, c, l)],
+                                                                       X0[m], X1[m], c, len);
+                    if (MODE == kWrite) {
+                        rhs[m * lmx + gi] = dfv;
+                    } else if (MODE == kAccum) {
+                        rhs[m * lmx + gi] = rv[p][m] + dfv;
+                    } else {
+                        const double r = MODE == kAccumRk ? rv[p][m] + dfv : dfv;
+                        qout[m * lmx + gi] = qv[p][m] - xmul(FM ? jv[p] : dtk, r);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// The flux pass along y and z for lines of up to 128 points: column tiles
+// (column.cuh).  Thread (l, c) evaluates the fluxes of its chunk into its own
+// shared-memory rows, eliminates the five fields of the chunk in registers,
+// and reads the eliminated rows back for the read-modify-write.
+// The tile of lines line0 .. line0 + TL - 1 (those below F); V holds 5 (kField +
+// 4 TL) values.  CG as flux_tile.
+template <int LT, int AXIS, int TL, int P, int MODE, bool VISC, bool FM, bool CG>
+__device__ __forceinline__ void flux_col_tile(double *V, int line0, int F, const double *__restrict__ q,
+                                              const double *__restrict__ g, double *__restrict__ rhs,
+                                              const double *__restrict__ qn, double *__restrict__ qout,
+                                              const DevTables<double> &tab, int lxi, int let, int64_t lmx, int nstart,
+                                              int nend, const Coeffs &cf, const Phys &ph, const RkParams &rk,
+                                              const FieldMet &fm = FieldMet{}) {
+    using C = Column<LT, TL, P>;
+    double *rows = V + 5 * C::kField;
+    const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL;
+    const int len = lane_len(c, LT, tab.p, tab.last_len);
+    const int s = AXIS == 1 ? lxi : lxi * let;
+    const int fidx = min(line0 + l, F - 1);  // past the last line: the last line again, not stored
+    const int base = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + c * LT * s;
+    if (len > 0) {
+        constexpr int U = FM ? 1 : CSB_FLUX_UNROLL;
+#pragma unroll U
+        for (int t = 0; t < LT; ++t) {
+            double fl[5];
+            // past the chunk's end: its last point again
+            point_flux<AXIS, VISC, CG, FM>(q, g, lmx, base + min(t, len - 1) * s, ph, fl, fm);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) V[m * C::kField + C::at(t, c, l)] = fl[m];
+        }
+    }
+    __syncthreads();
+    if (nstart || nend) column_closure_rows<LT, TL, 5, double, double, C>(V, rows, n, cf, nullptr, F, line0);
+    {
+        double d[5][LT];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+#pragma unroll
+            for (int t = 0; t < LT; ++t) d[m][t] = V[m * C::kField + C::at(t, c, l)];
+            column_rhs<LT, TL, double, C>(V + m * C::kField, c, l, len, n, nstart, nend, d[m]);
+        }
+        __syncthreads();
+        if (nstart || nend) {
+#pragma unroll
+            for (int m = 0; m < 5; ++m) column_take_rows<LT, double>(rows + 4 * (m * TL + l), c, n, nstart, nend, d[m]);
+        }
+        chunk_eliminate<LT, 5, double>(tab, d, c);
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+#pragma unroll
+            for (int t = 0; t < LT; ++t) V[m * C::kField + C::at(t, c, l)] = d[m][t];
+    }
+    __syncthreads();
+    column_reduced<LT, TL, 5, double, C>(V, tab);
+    __syncthreads();
+    double dtk = 0.0, dtd = 0.0;
+    if (MODE >= kAccumRk) {
+        const double dt = rk_dt<CG>(rk);
+        dtd = dt / rk.div;
+        dtk = xmul(dtd, ph.J);
+        if (rk.dt_out && line0 == 0 && threadIdx.x == 0) *rk.dt_out = dt;
+    }
+    if (len == 0 || line0 + l >= F) return;
+    if (tab.interior)
+        flux_col_store<true, LT, C, MODE, FM, CG>(V, tab, c, l, len, base, s, lmx, rhs, qn, qout, dtd, dtk, fm);
+    else
+        flux_col_store<false, LT, C, MODE, FM, CG>(V, tab, c, l, len, base, s, lmx, rhs, qn, qout, dtd, dtk, fm);
+}
+
+template <int LT, int AXIS, int TL, int MODE, bool VISC, bool FM>
+__global__ void __launch_bounds__(TL * 32, 512 / (TL * 32))
+k_flux_col(const double *__restrict__ q, const double *__restrict__ g, double *__restrict__ rhs,
+           const double *__restrict__ qn, double *__restrict__ qout, DevTables<double> tab, int lxi, int let,
+           int64_t lmx, int F, int nstart, int nend, Coeffs cf, Phys ph, RkParams rk, FieldMet fm) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    flux_col_tile<LT, AXIS, TL, 32, MODE, VISC, FM, false>(reinterpret_cast<double *>(smem_raw),
+                                                           (int)blockIdx.x * TL, F, q, g, rhs, qn, qout, tab, lxi, let,
+                                                           lmx, nstart, nend, cf, ph, rk, fm);
+}
+
+// Gradient and flux pass along x in one kernel, for the viscous right-hand side
+// on the uniform grid (rows of up to 128 points, starting on multiples of their
+// chunk, which is one vector; mode kWrite).  A warp holds one line, each lane its chunk: the x gradients of (u,
+// v, w, T) are solved first, those the other flux passes read (u, v, w) are
+// stored, and the fluxes are formed from them while the line's state is still
+// in the caches, so the separate gradient pass's read of q and both passes'
+// traffic of its own gradients (80 of 216 bytes per point) never reach HBM.
+// The y and z gradients must be current.  Arithmetic as k_grad / k_flux.
+template <int LT, bool DTRED>
+__global__ void __launch_bounds__(256, 2)
+k_gradflux_row(const double *__restrict__ q, double *__restrict__ g, double *__restrict__ rhs,
+               double *__restrict__ drva, DevTables<double> tab, int64_t lmx, int F, int nstart, int nend, Coeffs cf,
+               Phys ph, unsigned long long *__restrict__ dtacc) {
+    constexpr int VE = LT, VB = 8 * LT;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31, j0 = lane * LT;
+    // this lane's slots [5][LT] (stride 32) and the warp's line ends [4][17]
+    double *slot = reinterpret_cast<double *>(smem_raw) + w * (5 * LT * 32) + lane;
+    double(*ends)[2 * kLmd + 1] =
+        reinterpret_cast<double(*)[2 * kLmd + 1]>(reinterpret_cast<double *>(smem_raw) + 8 * 5 * LT * 32) + w * 4;
+    const int len = lane_len(lane, LT, tab.p, tab.last_len);
+    const int line = (int)blockIdx.x * 8 + w;
+    double m1 = 0.0, m2 = 0.0;
+    if (line < F) {
+        const int64_t base = (int64_t)line * n + j0;
+        const bool sums = nstart || nend;
+        {
+            double d[4][LT];
+#pragma unroll
+            for (int t0 = 0; t0 < LT; t0 += VE) {
+                if (t0 < len) {
+                    double qv[5][VE];
+#pragma unroll
+                    for (int m = 0; m < 5; ++m) load_vec<VB, double>(q + m * lmx + base + t0, qv[m]);
+#pragma unroll
+                    for (int b = 0; b < VE; ++b) {
+                        const Prim pr = primitives(qv[0][b], qv[1][b], qv[2][b], qv[3][b], qv[4][b]);
+                        d[0][t0 + b] = pr.u;
+                        d[1][t0 + b] = pr.v;
+                        d[2][t0 + b] = pr.w;
+                        d[3][t0 + b] = pr.T;
+                        if (DTRED) cfl_terms<false>(pr, ph, FieldMet{}, lmx, base + t0 + b, m1, m2);
+                    }
+                } else {
+#pragma unroll
+                    for (int f = 0; f < 4; ++f)
+#pragma unroll
+                        for (int b = 0; b < VE; ++b) d[f][t0 + b] = 0.0;
+                }
+            }
+            double rows = 0.0;
+            if (sums) {
+                chunk_put_ends<LT, 4, double>(ends, d, lane, len, n);
+                __syncwarp();
+                rows = ends_closure_row<double>(ends[lane >> 3], lane & 7, cf);
+                __syncwarp();
+            }
+#pragma unroll
+            for (int f = 0; f < 4; ++f) chunk_warp_rhs<LT, double>(rows, f, lane, len, n, nstart, nend, d[f]);
+            warp_solve<LT, 4, double>(tab, d, lane);
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+#pragma unroll
+                for (int t = 0; t < LT; t += VE)
+                    if (f < 3 && t < len) store_vec<VB, double>(g + f * lmx + base + t, &d[f][t]);
+#pragma unroll
+                for (int t = 0; t < LT; ++t) slot[(f * LT + t) * 32] = d[f][t];
+            }
+        }
+        // fluxes: y and z gradients this axis needs are u_y, v_y and u_z, w_z
+#pragma unroll
+        for (int t0 = 0; t0 < LT; t0 += VE) {
+            if (t0 < len) {
+                double qv[5][VE], uy[VE], vy[VE], uz[VE], wz[VE];
+#pragma unroll
+                for (int m = 0; m < 5; ++m) load_vec<VB, double>(q + m * lmx + base + t0, qv[m]);
+                load_vec<VB, double>(g + 4 * lmx + base + t0, uy);
+                load_vec<VB, double>(g + 5 * lmx + base + t0, vy);
+                load_vec<VB, double>(g + 8 * lmx + base + t0, uz);
+                load_vec<VB, double>(g + 10 * lmx + base + t0, wz);
+                PointMet pm = point_met<false>(ph, FieldMet{}, lmx, 0);
+#pragma unroll
+                for (int b = 0; b < VE; ++b) {
+                    double gr[12] = {};
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) gr[f] = slot[(f * LT + t0 + b) * 32];
+                    gr[4] = uy[b];
+                    gr[5] = vy[b];
+                    gr[8] = uz[b];
+                    gr[10] = wz[b];
+                    double fl[5];
+                    flux_values<0, true, true>(qv[0][b], qv[1][b], qv[2][b], qv[3][b], qv[4][b], gr, pm, ph, fl);
+#pragma unroll
+                    for (int m = 0; m < 5; ++m) slot[(m * LT + t0 + b) * 32] = fl[m];
+                }
+            } else {
+#pragma unroll
+                for (int m = 0; m < 5; ++m)
+#pragma unroll
+                    for (int b = 0; b < VE; ++b) slot[(m * LT + t0 + b) * 32] = 0.0;
+            }
+        }
+        auto solve = [&](auto nf, int m0) {
+            constexpr int G = decltype(nf)::value;
+            double d[G][LT];
+#pragma unroll
+            for (int f = 0; f < G; ++f)
+#pragma unroll
+                for (int t = 0; t < LT; ++t) d[f][t] = slot[((m0 + f) * LT + t) * 32];
+            double rows = 0.0;
+            if (sums) {
+                chunk_put_ends<LT, G, double>(ends, d, lane, len, n);
+                __syncwarp();
+                rows = ends_closure_row<double>(ends[(lane >> 3) < G ? lane >> 3 : 0], lane & 7, cf);
+                __syncwarp();
+            }
+#pragma unroll
+            for (int f = 0; f < G; ++f) chunk_warp_rhs<LT, double>(rows, f, lane, len, n, nstart, nend, d[f]);
+            warp_solve<LT, G, double>(tab, d, lane);
+#pragma unroll
+            for (int f = 0; f < G; ++f) {
+#pragma unroll
+                for (int t = 0; t < LT; t += VE)
+                    if (t < len) store_vec<VB, double>(rhs + (m0 + f) * lmx + base + t, &d[f][t]);
+                if (drva) {
+                    // line-end derivatives for the characteristic boundary closure
+                    if (lane == 0) drva[(int64_t)(m0 + f) * F + line] = d[f][0];
+                    if (lane == (n - 1) / LT)
+                        drva[(int64_t)(5 + m0 + f) * F + line] = get_at<LT, double>(d[f], n - 1 - j0);
+                }
+            }
+        };
+        solve(std::integral_constant<int, 3>{}, 0);
+        solve(std::integral_constant<int, 2>{}, 3);
+    }
+    if (DTRED) cfl_reduce(m1, m2, dtacc);
+}
+
 // Derivative closure of a boundary code: 0 physical, 1 interface / periodic, -1 unknown.
 int bc_ndf(int code);
 // Metrics, Jacobian and viscosity of the uniform grid of a solver configuration.
@@ -625,31 +1073,112 @@ FluxPrefetch flux_prefetch(const PassArgs &b, const RT *rhs, const double *qn, C
     return pf;
 }
 
-template <int LT, int AXIS, int TL>
-int launch_grad_t(const PassArgs &a, const double *q, bool dtred, cudaStream_t st) {
-    const size_t smem = (size_t)4 * TL * LineLayout<LT>::kSlot * sizeof(double);
-    auto kern = dtred ? k_grad<LT, AXIS, TL, true> : k_grad<LT, AXIS, TL, false>;
-    if (dtred && a.fm.xim) kern = k_grad<LT, AXIS, TL, true, true>;
-    if (int rc = set_smem(kern, smem)) return rc;
-    const unsigned blocks = (unsigned)((a.F + TL - 1) / TL);
-    kern<<<blocks, TL * 32, smem, st>>>(q, a.grad + (int64_t)AXIS * 4 * a.lmx, a.tab->t64, a.lxi, a.let,
-                                        a.lmx, a.F, a.nstart, a.nend, a.cf, a.ph, a.dtacc, a.fm);
+template <int LT, int VB>
+int launch_grad_row(const PassArgs &a, const double *q, bool dtred, cudaStream_t st) {
+    auto kern = dtred ? k_grad_row<LT, VB, true, false> : k_grad_row<LT, VB, false, false>;
+    if (dtred && a.fm.xim) kern = k_grad_row<LT, VB, true, true>;
+    kern<<<(unsigned)((a.F + 7) / 8), 256, 0, st>>>(q, a.grad, a.tab->t64, a.lmx, (int)a.F, a.nstart, a.nend, a.cf,
+                                                    a.ph, a.dtacc, a.fm);
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
 }
 
+// Vector bytes of the merged x pass (k_gradflux_row) on this state, 0 where it
+// does not apply.  Lines of up to 128 points only: measured against the two
+// passes, 64^3 30 against 43 us, 128^3 126 against 146 us, but 192^3 592 against
+// 420 us (eight-row chunks: 82 KB of slots per CTA leave too little L1 for
+// chunk-wise loads of nine fields).
+constexpr int kMergeMaxLt = 4;
+inline int gradflux_vec(const PassArgs &a, const double *q, const double *rhs) {
+    if (a.tab->lt > kMergeMaxLt || !a.viscous || a.fm.xim) return 0;
+    const int vb = a.tab->lt * 8;  // a whole chunk
+    const uintptr_t p = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(a.grad) |
+                        reinterpret_cast<uintptr_t>(rhs);
+    return a.lxi % a.tab->lt == 0 && a.lmx % a.tab->lt == 0 && p % vb == 0 ? vb : 0;
+}
+// Gradient and flux pass along x in one launch (rhs written); a.rhs receives it.
+int launch_gradflux_x(const PassArgs &a, const double *q, double *drva, bool dtred, cudaStream_t st);
+
+template <int LT>
+int launch_gradflux_t(const PassArgs &a, const double *q, double *drva, bool dtred, cudaStream_t st) {
+    const size_t smem = (size_t)(8 * 5 * LT * 32 + 8 * 4 * (2 * kLmd + 1)) * sizeof(double);
+    auto kern = dtred ? k_gradflux_row<LT, true> : k_gradflux_row<LT, false>;
+    if (int rc = set_smem(kern, smem)) return rc;
+    kern<<<(unsigned)((a.F + 7) / 8), 256, smem, st>>>(q, a.grad, a.rhs, drva, a.tab->t64, a.lmx, (int)a.F, a.nstart,
+                                                       a.nend, a.cf, a.ph, a.dtacc);
+    CSB_CUDA(cudaGetLastError());
+    return CS_OK;
+}
+
+template <int LT, int AXIS, int TL>
+int launch_grad_col(const PassArgs &a, const double *q, bool dtred, cudaStream_t st) {
+    const size_t smem = (size_t)4 * (Column<LT, TL>::kField + 4 * TL) * sizeof(double);
+    auto kern = dtred ? k_grad_col<LT, AXIS, TL, true, false> : k_grad_col<LT, AXIS, TL, false, false>;
+    if (dtred && a.fm.xim) kern = k_grad_col<LT, AXIS, TL, true, true>;
+    if (int rc = set_smem(kern, smem)) return rc;
+    kern<<<(unsigned)((a.F + TL - 1) / TL), column_threads(TL, a.tab->t64.p), smem, st>>>(
+        q, a.grad + (int64_t)AXIS * 4 * a.lmx, a.tab->t64, a.lxi, a.let, a.lmx, (int)a.F, a.nstart, a.nend, a.cf,
+        a.ph, a.dtacc, a.fm);
+    CSB_CUDA(cudaGetLastError());
+    return CS_OK;
+}
+
+template <int LT, int AXIS, int TL>
+int launch_grad_t(const PassArgs &a, const double *q, bool dtred, cudaStream_t st) {
+    if constexpr (LT <= 8 && AXIS > 0) return launch_grad_col<LT, AXIS, TL>(a, q, dtred, st);
+    if constexpr (LT <= 8 && AXIS == 0) {
+        auto aligned = [&](int vb) {
+            return LT * 8 >= vb && a.lxi % (vb / 8) == 0 && a.lmx % (vb / 8) == 0 &&
+                   (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(a.grad)) % vb == 0;
+        };
+        if constexpr (LT >= 4) {
+            if (aligned(32)) return launch_grad_row<LT, 32>(a, q, dtred, st);
+        }
+        if (aligned(16)) return launch_grad_row<LT, 16>(a, q, dtred, st);
+    }
+    if constexpr (LT > 8 || AXIS == 0) {
+        const size_t smem = (size_t)4 * TL * LineLayout<LT>::kSlot * sizeof(double);
+        auto kern = dtred ? k_grad<LT, AXIS, TL, true> : k_grad<LT, AXIS, TL, false>;
+        if (dtred && a.fm.xim) kern = k_grad<LT, AXIS, TL, true, true>;
+        if (int rc = set_smem(kern, smem)) return rc;
+        const unsigned blocks = (unsigned)((a.F + TL - 1) / TL);
+        kern<<<blocks, TL * 32, smem, st>>>(q, a.grad + (int64_t)AXIS * 4 * a.lmx, a.tab->t64, a.lxi, a.let,
+                                            a.lmx, a.F, a.nstart, a.nend, a.cf, a.ph, a.dtacc, a.fm);
+        CSB_CUDA(cudaGetLastError());
+        return CS_OK;
+    }
+}
+
+// The flux passes along y and z run column tiles for lines of up to 128 points
+// (y / z + RK: 128^3 115 / 143 against 131 / 156 us with a warp per line, 64^3 23
+// / 25 against 29 / 31 us); with eight-row chunks they are no faster (256^3 785 /
+// 866 against 732 / 889 us, 192^3 424 / 450 against 369 / 452 us).
+constexpr int kFluxColMaxLt = 4;
 template <int LT, int AXIS, int TL, int MODE>
 int launch_flux_t(const PassArgs &a, const double *q, const double *qn, double *qout, double *drva,
                   const RkParams &rk, cudaStream_t st) {
-    const size_t smem = (size_t)5 * TL * LineLayout<LT>::kSlot * sizeof(double);
-    auto kern = a.viscous ? k_flux<LT, AXIS, TL, MODE, true> : k_flux<LT, AXIS, TL, MODE, false>;
-    if (a.fm.xim) kern = a.viscous ? k_flux<LT, AXIS, TL, MODE, true, true> : k_flux<LT, AXIS, TL, MODE, false, true>;
-    if (int rc = set_smem(kern, smem)) return rc;
-    const unsigned blocks = (unsigned)((a.F + TL - 1) / TL);
-    kern<<<blocks, TL * 32, smem, st>>>(q, a.grad, a.rhs, qn, qout, drva, a.tab->t64, a.lxi, a.let, a.lmx,
-                                        a.F, a.nstart, a.nend, a.cf, a.ph, rk, a.fm);
-    CSB_CUDA(cudaGetLastError());
-    return CS_OK;
+    if constexpr (LT <= kFluxColMaxLt && AXIS > 0) {
+        const size_t csm = (size_t)5 * (Column<LT, TL>::kField + 4 * TL) * sizeof(double);
+        auto ck = a.viscous ? k_flux_col<LT, AXIS, TL, MODE, true, false> : k_flux_col<LT, AXIS, TL, MODE, false, false>;
+        if (a.fm.xim)
+            ck = a.viscous ? k_flux_col<LT, AXIS, TL, MODE, true, true> : k_flux_col<LT, AXIS, TL, MODE, false, true>;
+        if (int rc = set_smem(ck, csm)) return rc;
+        ck<<<(unsigned)((a.F + TL - 1) / TL), column_threads(TL, a.tab->t64.p), csm, st>>>(
+            q, a.grad, a.rhs, qn, qout, a.tab->t64, a.lxi, a.let, a.lmx, (int)a.F, a.nstart, a.nend, a.cf, a.ph, rk,
+            a.fm);
+        CSB_CUDA(cudaGetLastError());
+        return CS_OK;
+    } else {
+        const size_t smem = (size_t)5 * TL * LineLayout<LT>::kSlot * sizeof(double);
+        auto kern = a.viscous ? k_flux<LT, AXIS, TL, MODE, true> : k_flux<LT, AXIS, TL, MODE, false>;
+        if (a.fm.xim) kern = a.viscous ? k_flux<LT, AXIS, TL, MODE, true, true> : k_flux<LT, AXIS, TL, MODE, false, true>;
+        if (int rc = set_smem(kern, smem)) return rc;
+        const unsigned blocks = (unsigned)((a.F + TL - 1) / TL);
+        kern<<<blocks, TL * 32, smem, st>>>(q, a.grad, a.rhs, qn, qout, drva, a.tab->t64, a.lxi, a.let, a.lmx,
+                                            a.F, a.nstart, a.nend, a.cf, a.ph, rk, a.fm);
+        CSB_CUDA(cudaGetLastError());
+        return CS_OK;
+    }
 }
 
 template <int AXIS, int TL>

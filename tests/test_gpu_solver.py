@@ -69,6 +69,40 @@ def test_rhs_periodic(cuda, dims, viscous):
     assert rhs_err(out.cpu().numpy(), ref, scale) < 1e-12
 
 
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("dims", [(8, 9, 10), (12, 33, 66), (66, 8, 129), (68, 127, 8), (130, 10, 255), (260, 12, 9),
+                                  (9, 256, 17), (10, 17, 300)])
+def test_rhs_chunk_and_tile_edges(cuda, dims, periodic):
+    """Line lengths and line counts around the chunk, tile and vector-access
+    edges of every gradient and flux pass, both closures, the state on and off
+    a 16-byte boundary, and the same with the metrics given as arrays."""
+    import torch
+    import compact_schemes_b200 as cs
+    b = cs.BC_PERIODIC if periodic else cs.BC_NON_REFLECTIVE
+    nbc = [[b] * 3] * 2
+    n = int(np.prod(dims))
+    mm = O.uniform_metrics(*dims)
+    s = solver(dims, nbc=nbc)
+    q = O.tgv_init(dims, 0.2, 1e-3, 7)
+    ref, scale = O.rhs(q, s.cfg.mu, mm, dims, [[int(periodic)] * 3] * 2, with_scale=True)
+    for off in (0, 1):
+        buf = torch.zeros(5 * n + off, dtype=torch.float64, device=cuda)
+        buf[off:] = dev(q)
+        out = torch.zeros(5 * n + 8, dtype=torch.float64, device=cuda)
+        s.rhs(buf[off:], out)
+        assert rhs_err(out[:5 * n].cpu().numpy(), ref, scale) < 1e-12
+        assert not bool(out[5 * n:].any())
+    h = [2 * math.pi / d for d in dims]
+    diag = [torch.zeros(3, n, dtype=torch.float64, device=cuda) for _ in range(3)]
+    for a, v in enumerate((h[1] * h[2], h[0] * h[2], h[0] * h[1])):
+        diag[a][a] = v
+    s.set_metrics(*(d.reshape(-1) for d in diag),
+                  torch.full((n,), 1.0 / (h[0] * h[1] * h[2]), dtype=torch.float64, device=cuda))
+    out.zero_()
+    s.rhs(dev(q), out)
+    assert rhs_err(out[:5 * n].cpu().numpy(), ref, scale) < 1e-12
+
+
 def test_rhs_random_state(cuda):
     """A non-smooth state exercises every term (all gradients, all fluxes)."""
     import torch
