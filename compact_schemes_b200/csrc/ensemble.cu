@@ -26,7 +26,7 @@ struct cs_ensemble {
     double *dt = nullptr;
     int *ctl = nullptr;  // [0] error word, [1] queue head, [2..] done[nbox][kEnsPhases]
     csb::Coeffs *cf_dev = nullptr;
-    int lt_max = 2;
+    int lt_max = 4;
     int nsm = 1;
     cs_ensemble_tuning tune{0, 8, 0, 4};
     // work lists of the current tuning: [0] stage 0, [1] stages 1-3
@@ -114,7 +114,12 @@ static int ens_build_lists(cs_ensemble *e) {
     return CS_OK;
 }
 
-static int ens_tile_doubles(const cs_ensemble *e) { return 5 * e->tune.tile * (32 * e->lt_max + 1); }
+// Tile buffer of five fields: whole lines (x items) or column tiles (y and z),
+// which pad every chunk slot row and keep their closure rows.
+static int ens_tile_doubles(int tile, int lt) {
+    return 5 * std::max(tile * (32 * lt + 1), lt * (32 * tile + 32) + 16 * tile);
+}
+static int ens_tile_doubles(const cs_ensemble *e) { return ens_tile_doubles(e->tune.tile, e->lt_max); }
 
 // tile buffer, then the segment starts of the larger of the two work lists
 static size_t ens_smem(const cs_ensemble *e) {
@@ -164,7 +169,7 @@ static int ens_check_tuning(const cs_ensemble *e, const cs_ensemble_tuning &t) {
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         smem_max = 227 * 1024;
-    const size_t need = (size_t)5 * t.tile * (32 * e->lt_max + 1) * sizeof(double) + kEnsSmemStarts * sizeof(int);
+    const size_t need = (size_t)ens_tile_doubles(t.tile, e->lt_max) * sizeof(double) + kEnsSmemStarts * sizeof(int);
     if (need > (size_t)smem_max) return set_error(CS_ERR_UNSUPPORTED, "ensemble tile %d needs %zu bytes", t.tile, need);
     return CS_OK;
 }

@@ -85,18 +85,7 @@ constexpr int kEnsMaxBoxes = 96;
 static __constant__ EnsBox c_ens_boxes[kEnsMaxBoxes];
 static __constant__ Coeffs c_ens_cf;
 
-// Points per read-modify-write chunk in the ensemble's flux items (fewer than
-// the per-box passes: the items have fewer registers to spare; measured on
-// the 64-box set, one point beats two or four).
-#ifndef CSB_ENS_RMW
-#define CSB_ENS_RMW 1
-#endif
-#ifndef CSB_ENS_RMW_RK
-#define CSB_ENS_RMW_RK 1
-#endif
-constexpr int kEnsRmwChunk = CSB_ENS_RMW, kEnsRmwChunkRk = CSB_ENS_RMW_RK;
-
-// Line solves of the work items: fields per warp solve for lines of up to 128
+// Line solves of the x items: fields per warp solve for lines of up to 128
 // points (LT <= 4), and whether the periodic closure rows are formed
 // lane-parallel (8 lanes per field line) instead of by the two owner lanes.
 // Short lines make the serial closure sums a large share of the solve, which
@@ -112,31 +101,46 @@ constexpr int ens_solve_group() {
     return LT <= 4 ? CSB_ENS_SG : 2;
 }
 
-// One work item of pass KIND for chunk length LT, inlined into the stage
-// kernel (with the box parameters in constant memory the combined body spills
-// little; separate functions measured slower by their call overhead).
+// Tiles [t0, t1) of TL lines of pass KIND for chunk length LT.  Each pass is a
+// function of its own, called once per work item: inlined into the stage kernel
+// the column passes spilled 5.7 KB per thread, as functions nothing for lines of
+// up to 128 points (one point per read-modify-write; two spill 640 bytes).
+// x passes run one tile at a time with a warp per line (grad_tile / flux_tile);
+// y and z passes run column tiles (grad_col_tile / flux_col_tile) of TL, 2 TL or
+// 4 TL lines, whichever fills the CTA's threads for lines of 32, 16 or 8 chunks.
 template <int TL, bool VISC, int LT, int KIND>
-__device__ __forceinline__ void ens_item(const EnsArgs &a, int b, int64_t line0, double *sm) {
+__device__ __noinline__ void ens_item_x(const EnsArgs &a, int b, int64_t t0, int64_t t1, double *sm) {
     const EnsBox &bx = c_ens_boxes[b];
     const int stage = a.stage;
     const double *qin = (stage == 0 ? a.q : a.q1) + bx.qoff;
     double *g = a.grad + bx.goff;
-    constexpr int AX = KIND % 3;
-    const Phys &ph = bx.ph;
-    const DevTables<double> &tab = bx.tab[AX];
-    if (KIND < 3) {
-        constexpr int SG = ens_solve_group<LT>();
-        constexpr bool ROWS = CSB_ENS_ROWS != 0;
+    const DevTables<double> &tab = bx.tab[0];
+    constexpr int SG = ens_solve_group<LT>();
+    constexpr bool ROWS = CSB_ENS_ROWS != 0;
+    for (int64_t t = t0; t < t1; ++t) {
+        if (t > t0) __syncthreads();  // the tile buffer is reused
         if (KIND == 0 && stage == 0)
-            grad_tile<LT, 0, TL, true, false, SG, ROWS>(sm, line0, qin, g, tab, bx.lxi, bx.let, bx.lmx, bx.F[0],
-                                                        bx.nstart[0], bx.nend[0], c_ens_cf, ph, a.dtacc + 2 * b);
+            grad_tile<LT, 0, TL, true, false, SG, ROWS>(sm, t * TL, qin, g, tab, bx.lxi, bx.let, bx.lmx, bx.F[0],
+                                                        bx.nstart[0], bx.nend[0], c_ens_cf, bx.ph, a.dtacc + 2 * b);
+        else if (KIND == 0)
+            grad_tile<LT, 0, TL, false, false, SG, ROWS>(sm, t * TL, qin, g, tab, bx.lxi, bx.let, bx.lmx, bx.F[0],
+                                                         bx.nstart[0], bx.nend[0], c_ens_cf, bx.ph, nullptr);
         else
-            grad_tile<LT, AX, TL, false, false, SG, ROWS>(sm, line0, qin, g + 4 * AX * bx.lmx, tab, bx.lxi, bx.let,
-                                                          bx.lmx, bx.F[AX], bx.nstart[AX], bx.nend[AX], c_ens_cf, ph,
-                                                          nullptr);
-        return;
+            flux_tile<LT, 0, TL, kWrite, VISC, true, 1, false, SG, ROWS>(
+                sm, t * TL, qin, g, a.rhs + bx.roff, nullptr, nullptr, nullptr, tab, bx.lxi, bx.let, bx.lmx, bx.F[0],
+                bx.nstart[0], bx.nend[0], c_ens_cf, bx.ph, RkParams{});
     }
-    double *rhs = a.rhs + bx.roff;
+}
+
+template <int TL, int TLC, bool VISC, int LT, int KIND>
+__device__ __noinline__ void ens_item_col(const EnsArgs &a, int b, int line0, int line1, double *sm) {
+    const EnsBox &bx = c_ens_boxes[b];
+    const int stage = a.stage;
+    const double *qin = (stage == 0 ? a.q : a.q1) + bx.qoff;
+    double *g = a.grad + bx.goff;
+    constexpr int AX = KIND % 3, P = 32 * TL / TLC;
+    constexpr int MODE = KIND == 4 ? kAccum : kAccumRk;
+    const DevTables<double> &tab = bx.tab[AX];
     RkParams rk{};
     if (KIND == 5) {
         rk.div = 4 - stage;
@@ -145,33 +149,47 @@ __device__ __forceinline__ void ens_item(const EnsArgs &a, int b, int64_t line0,
         rk.dtacc = a.dtacc + 2 * b;
         rk.dt_out = stage == 0 ? a.dt + b : nullptr;
     }
-    const double *qn = a.q + bx.qoff;
-    double *qout = (stage == 3 ? a.q : a.q1) + bx.qoff;
-    constexpr int MODE = KIND == 3 ? kWrite : (KIND == 4 ? kAccum : kAccumRk);
-    constexpr int P = MODE == kAccum ? kEnsRmwChunk : kEnsRmwChunkRk;
-    flux_tile<LT, AX, TL, MODE, VISC, true, P, false, ens_solve_group<LT>(), CSB_ENS_ROWS != 0>(
-        sm, line0, qin, g, rhs, qn, qout, nullptr, tab, bx.lxi, bx.let, bx.lmx, bx.F[AX], bx.nstart[AX], bx.nend[AX],
-        c_ens_cf, ph, rk);
-}
-
-template <int TL, bool VISC, int LT>
-__device__ __forceinline__ void ens_run_lt(const EnsArgs &a, int b, int kind, int64_t line0, double *sm) {
-    switch (kind) {
-        case 0: ens_item<TL, VISC, LT, 0>(a, b, line0, sm); break;
-        case 1: ens_item<TL, VISC, LT, 1>(a, b, line0, sm); break;
-        case 2: ens_item<TL, VISC, LT, 2>(a, b, line0, sm); break;
-        case 3: ens_item<TL, VISC, LT, 3>(a, b, line0, sm); break;
-        case 4: ens_item<TL, VISC, LT, 4>(a, b, line0, sm); break;
-        default: ens_item<TL, VISC, LT, 5>(a, b, line0, sm); break;
+    for (int l = line0; l < line1; l += TLC) {
+        if (l > line0) __syncthreads();  // the tile buffer is reused
+        if (KIND < 3) {
+            double m1 = 0.0, m2 = 0.0;
+            grad_col_tile<LT, AX, TLC, P, false, false>(sm, l, line1, qin, g + 4 * AX * bx.lmx, tab, bx.lxi, bx.let,
+                                                        bx.lmx, bx.nstart[AX], bx.nend[AX], c_ens_cf, bx.ph, m1, m2);
+        } else {
+            flux_col_tile<LT, AX, TLC, P, MODE, VISC, false, true>(
+                sm, l, line1, qin, g, a.rhs + bx.roff, a.q + bx.qoff, (stage == 3 ? a.q : a.q1) + bx.qoff, tab, bx.lxi,
+                bx.let, bx.lmx, bx.nstart[AX], bx.nend[AX], c_ens_cf, bx.ph, rk);
+        }
     }
 }
 
+template <int TL, int TLC, bool VISC, int LT>
+__device__ __forceinline__ void ens_run_col(const EnsArgs &a, int b, int kind, int line0, int line1, double *sm) {
+    if (kind == 1) ens_item_col<TL, TLC, VISC, LT, 1>(a, b, line0, line1, sm);
+    else if (kind == 2) ens_item_col<TL, TLC, VISC, LT, 2>(a, b, line0, line1, sm);
+    else if (kind == 4) ens_item_col<TL, TLC, VISC, LT, 4>(a, b, line0, line1, sm);
+    else ens_item_col<TL, TLC, VISC, LT, 5>(a, b, line0, line1, sm);
+}
+
+// The ensemble's tables have chunks of 4 points (lines of up to 128 points) or 8.
 template <int TL, bool VISC>
-__device__ __forceinline__ void ens_run_item(const EnsArgs &a, int b, int kind, int64_t line0, double *sm) {
+__device__ __forceinline__ void ens_run_item(const EnsArgs &a, int b, int kind, int t0, int t1, double *sm) {
     const int lt = c_ens_boxes[b].lt[kind % 3];
-    if (lt == 2) ens_run_lt<TL, VISC, 2>(a, b, kind, line0, sm);
-    else if (lt == 4) ens_run_lt<TL, VISC, 4>(a, b, kind, line0, sm);
-    else ens_run_lt<TL, VISC, 8>(a, b, kind, line0, sm);
+    if (kind % 3 == 0) {
+        if (lt == 4) {
+            if (kind == 0) ens_item_x<TL, VISC, 4, 0>(a, b, t0, t1, sm);
+            else ens_item_x<TL, VISC, 4, 3>(a, b, t0, t1, sm);
+        } else {
+            if (kind == 0) ens_item_x<TL, VISC, 8, 0>(a, b, t0, t1, sm);
+            else ens_item_x<TL, VISC, 8, 3>(a, b, t0, t1, sm);
+        }
+        return;
+    }
+    const int line0 = t0 * TL, line1 = min(t1 * TL, (int)c_ens_boxes[b].F[kind % 3]), p = c_ens_boxes[b].tab[kind % 3].p;
+    if (lt == 8) ens_run_col<TL, TL, VISC, 8>(a, b, kind, line0, line1, sm);
+    else if (p > 16) ens_run_col<TL, TL, VISC, 4>(a, b, kind, line0, line1, sm);
+    else if (p > 8) ens_run_col<TL, 2 * TL, VISC, 4>(a, b, kind, line0, line1, sm);
+    else ens_run_col<TL, 4 * TL, VISC, 4>(a, b, kind, line0, line1, sm);
 }
 
 __device__ __forceinline__ int ens_load_acquire(const int *p) {
@@ -222,10 +240,7 @@ __global__ void __launch_bounds__(TL * 32, TL == 8 ? 2 : 4) k_ensemble_stage(con
         if (s_ok) {
             const int t0 = (it - sg.start) * a.chunk;
             const int t1 = min(t0 + a.chunk, sg.ntiles);
-            for (int t = t0; t < t1; ++t) {
-                if (t > t0) __syncthreads();  // the tile buffer is reused
-                ens_run_item<TL, VISC>(a, sg.box, sg.kind, (int64_t)t * TL, sm);
-            }
+            ens_run_item<TL, VISC>(a, sg.box, sg.kind, t0, t1, sm);
         }
         __syncthreads();  // the item's stores are issued by every thread
         if (threadIdx.x == 0) {
