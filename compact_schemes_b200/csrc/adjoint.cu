@@ -28,6 +28,8 @@ struct cs_adjoint {
     int nsm = 1;
     csb::TableCache tables;
     const csb::DeviceTables *tab[3] = {nullptr, nullptr, nullptr};
+    // tables of the line operators D and D^T (the gradient passes use tab)
+    const csb::DeviceTables *ltab[3] = {nullptr, nullptr, nullptr};
     const csb::DeviceTables *tabT[3] = {nullptr, nullptr, nullptr};
     csb::Coeffs cf{};
     csb::Phys ph{};
@@ -35,6 +37,7 @@ struct cs_adjoint {
     // scratch: G, dG / Gbar [12], phi4 [4], F15 [15], qbar [5], t1, t2, t3 [5], partial sums
     double *G = nullptr, *G2 = nullptr, *phi4 = nullptr, *F15 = nullptr, *qbar = nullptr;
     double *t1 = nullptr, *t2 = nullptr, *t3 = nullptr, *partial = nullptr;
+    double *bcol = nullptr;  // closure columns of B^T per axis [3][16][4] (closure_columns)
     unsigned long long *dtacc = nullptr;
     // non-reflective GCBC on the x faces: face mask, forward / tangent x-derivative
     // terms at the faces [2][5][F], face adjoint of q, lambda for the x solve [5][lmx]
@@ -49,37 +52,61 @@ namespace csb {
 
 constexpr int kPointBlocks = 148 * 8;
 
-static int lines(cs_adjoint *a, int axis, bool trans, const double *in, int64_t in_fs, double *out, int64_t out_fs,
-                 int nf, bool accum, double scale, cudaStream_t st) {
-    const DeviceTables *t = trans ? a->tabT[axis] : a->tab[axis];
-    const dim3 grid((unsigned)((a->F[axis] + 7) / 8), (unsigned)nf);
-    const int nstart = a->ndf[0][axis], nend = a->ndf[1][axis];
-#define CSB_LINES(LT, AX)                                                                                    \
-    do {                                                                                                     \
-        if (trans)                                                                                           \
-            k_lines<LT, AX, true><<<grid, 256, 0, st>>>(in, in_fs, out, out_fs, accum, scale, t->t64,         \
-                                                        a->d.lxi, a->d.let, a->F[AX], nstart, nend, a->cf); \
-        else                                                                                                 \
-            k_lines<LT, AX, false><<<grid, 256, 0, st>>>(in, in_fs, out, out_fs, accum, scale, t->t64,        \
-                                                         a->d.lxi, a->d.let, a->F[AX], nstart, nend, a->cf); \
-    } while (0)
-#define CSB_LINES_AX(LT)                       \
-    do {                                       \
-        if (axis == 0) CSB_LINES(LT, 0);       \
-        else if (axis == 1) CSB_LINES(LT, 1);  \
-        else CSB_LINES(LT, 2);                 \
-    } while (0)
-    switch (t->lt) {
-        case 2: CSB_LINES_AX(2); break;
-        case 4: CSB_LINES_AX(4); break;
-        case 8: CSB_LINES_AX(8); break;
-        case 16: CSB_LINES_AX(16); break;
-        default: return set_error(CS_ERR_UNSUPPORTED, "adjoint: lines of more than 512 points");
+template <int LT, int AXIS, bool TRANS>
+static int lines_t(cs_adjoint *a, const LineSet &ls, int nf, const DevTables<double> &tab, cudaStream_t st) {
+    const int F = (int)a->F[AXIS], nstart = a->ndf[0][AXIS], nend = a->ndf[1][AXIS];
+    const double *bcol = a->bcol + AXIS * 64;
+    if constexpr (AXIS == 0) {
+        constexpr int NV = LT <= 8 ? 2 : 1;
+        const dim3 grid((unsigned)((F + 8 * NV - 1) / (8 * NV)), (unsigned)nf);
+        auto aligned = [&](int vb) {
+            const int64_t ve = vb / 8;
+            return LT % ve == 0 && a->d.lxi % ve == 0 && ls.in_fs % ve == 0 && ls.out_fs % ve == 0 &&
+                   (reinterpret_cast<uintptr_t>(ls.in) | reinterpret_cast<uintptr_t>(ls.out)) % vb == 0;
+        };
+        if (LT >= 4 && aligned(32))
+            k_lines_row<LT, NV, (LT >= 4 ? 32 : 16), TRANS><<<grid, 256, 0, st>>>(ls, tab, F, nstart, nend, a->cf, bcol);
+        else if (aligned(16))
+            k_lines_row<LT, NV, 16, TRANS><<<grid, 256, 0, st>>>(ls, tab, F, nstart, nend, a->cf, bcol);
+        else
+            k_lines<LT, 0, TRANS><<<dim3((unsigned)((F + 7) / 8), (unsigned)nf), 256, 0, st>>>(
+                ls.in, ls.in_fs, ls.out, ls.out_fs, ls.accum, tab, a->d.lxi, a->d.let, F, nstart, nend, a->cf);
+    } else {
+        if (LT == kWarpChunk && warp_column(tab.n)) {
+            if constexpr (LT == kWarpChunk)
+                k_lines_wcol<LT, AXIS, TRANS><<<dim3((unsigned)((F + 31) / 32), (unsigned)nf), 256, 0, st>>>(
+                    ls, tab, a->d.lxi, a->d.let, F, nstart, nend, a->cf, bcol);
+        } else {
+            constexpr int TL = 8;
+            const size_t smem = (size_t)2 * (Column<LT, TL>::kField + 16 * TL) * sizeof(double);
+            auto kern = k_lines_col<LT, AXIS, TL, TRANS>;
+            if (int rc = set_smem(kern, smem)) return rc;
+            kern<<<dim3((unsigned)((F + 2 * TL - 1) / (2 * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
+                ls, tab, a->d.lxi, a->d.let, F, nstart, nend, a->cf, bcol);
+        }
     }
-#undef CSB_LINES_AX
-#undef CSB_LINES
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
+}
+
+template <int LT, bool TRANS>
+static int lines_ax(cs_adjoint *a, int axis, const LineSet &ls, int nf, const DevTables<double> &tab, cudaStream_t st) {
+    if (axis == 0) return lines_t<LT, 0, TRANS>(a, ls, nf, tab, st);
+    if (axis == 1) return lines_t<LT, 1, TRANS>(a, ls, nf, tab, st);
+    return lines_t<LT, 2, TRANS>(a, ls, nf, tab, st);
+}
+
+static int lines(cs_adjoint *a, int axis, bool trans, const double *in, int64_t in_fs, double *out, int64_t out_fs,
+                 int nf, bool accum, cudaStream_t st) {
+    const DeviceTables *t = trans ? a->tabT[axis] : a->ltab[axis];
+    const LineSet ls{in, out, in_fs, out_fs, accum ? 1 : 0};
+    switch (t->lt) {
+        case 2: return trans ? lines_ax<2, true>(a, axis, ls, nf, t->t64, st) : lines_ax<2, false>(a, axis, ls, nf, t->t64, st);
+        case 4: return trans ? lines_ax<4, true>(a, axis, ls, nf, t->t64, st) : lines_ax<4, false>(a, axis, ls, nf, t->t64, st);
+        case 8: return trans ? lines_ax<8, true>(a, axis, ls, nf, t->t64, st) : lines_ax<8, false>(a, axis, ls, nf, t->t64, st);
+        case 16: return trans ? lines_ax<16, true>(a, axis, ls, nf, t->t64, st) : lines_ax<16, false>(a, axis, ls, nf, t->t64, st);
+    }
+    return set_error(CS_ERR_UNSUPPORTED, "adjoint: lines of more than 512 points");
 }
 
 // The compact filter (Gaitonde-Visbal, filter_rhs) or its transpose along axis.
@@ -94,10 +121,10 @@ static int filter_lines(cs_adjoint *a, int axis, bool trans, double af, const do
 #define CSB_FLINES(LT, AX)                                                                                      \
     do {                                                                                                        \
         if (trans)                                                                                              \
-            k_lines<LT, AX, true, true><<<grid, 256, 0, st>>>(in, lmx, out, lmx, accum, 1.0, t->t64, a->d.lxi,   \
+            k_lines<LT, AX, true, true><<<grid, 256, 0, st>>>(in, lmx, out, lmx, accum, t->t64, a->d.lxi,   \
                                                               a->d.let, a->F[AX], nstart, nend, a->cf, af);     \
         else                                                                                                    \
-            k_lines<LT, AX, false, true><<<grid, 256, 0, st>>>(in, lmx, out, lmx, accum, 1.0, t->t64, a->d.lxi,  \
+            k_lines<LT, AX, false, true><<<grid, 256, 0, st>>>(in, lmx, out, lmx, accum, t->t64, a->d.lxi,  \
                                                                a->d.let, a->F[AX], nstart, nend, a->cf, af);    \
     } while (0)
 #define CSB_FLINES_AX(LT)                       \
@@ -154,7 +181,7 @@ static int gcbc_forward_faces(cs_adjoint *a, const double *q, cudaStream_t st) {
     if (a->cfg.viscous) k_flux_x_eval<true><<<kPointBlocks, 256, 0, st>>>(q, a->G, a->F15, a->ap);
     else k_flux_x_eval<false><<<kPointBlocks, 256, 0, st>>>(q, nullptr, a->F15, a->ap);
     CSB_CUDA(cudaGetLastError());
-    if (int rc = lines(a, 0, false, a->F15, lmx, a->F15 + 5 * lmx, lmx, 5, false, 1.0, st)) return rc;
+    if (int rc = lines(a, 0, false, a->F15, lmx, a->F15 + 5 * lmx, lmx, 5, false, st)) return rc;
     k_xface_extract<<<face_blocks(a), 128, 0, st>>>(a->F15 + 5 * lmx, a->rf, a->d.lxi, lmx, a->F[0]);
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
@@ -169,7 +196,7 @@ static int rhs_jvp(cs_adjoint *a, const double *q, const double *dq, double *dR,
         CSB_CUDA(cudaGetLastError());
         for (int b = 0; b < 3; ++b)
             if (a->active[b])
-                if (int rc = lines(a, b, false, a->phi4, lmx, a->G2 + 4 * b * lmx, lmx, 4, false, 1.0, st)) return rc;
+                if (int rc = lines(a, b, false, a->phi4, lmx, a->G2 + 4 * b * lmx, lmx, 4, false, st)) return rc;
         k_flux_tan<true><<<kPointBlocks, 256, 0, st>>>(q, a->G, dq, a->G2, a->F15, a->ap, a->amask);
     } else {
         k_flux_tan<false><<<kPointBlocks, 256, 0, st>>>(q, nullptr, dq, nullptr, a->F15, a->ap, a->amask);
@@ -178,7 +205,7 @@ static int rhs_jvp(cs_adjoint *a, const double *q, const double *dq, double *dR,
     bool first = true;
     for (int ax = 0; ax < 3; ++ax) {
         if (!a->active[ax]) continue;
-        if (int rc = lines(a, ax, false, a->F15 + 5 * ax * lmx, lmx, dR, lmx, 5, !first, 1.0, st)) return rc;
+        if (int rc = lines(a, ax, false, a->F15 + 5 * ax * lmx, lmx, dR, lmx, 5, !first, st)) return rc;
         if (ax == 0 && a->gcbc_mask) {
             k_xface_extract<<<face_blocks(a), 128, 0, st>>>(dR, a->drf, a->d.lxi, lmx, a->F[0]);
             CSB_CUDA(cudaGetLastError());
@@ -214,7 +241,7 @@ static int rhs_vjp(cs_adjoint *a, const double *q, const double *lam, double *ou
     }
     for (int ax = 0; ax < 3; ++ax)
         if (a->active[ax])
-            if (int rc = lines(a, ax, true, ax == 0 ? lam_x : lam, lmx, a->F15 + 5 * ax * lmx, lmx, 5, false, 1.0, st))
+            if (int rc = lines(a, ax, true, ax == 0 ? lam_x : lam, lmx, a->F15 + 5 * ax * lmx, lmx, 5, false, st))
                 return rc;
     if (visc) k_flux_adj<true><<<kPointBlocks, 256, 0, st>>>(q, a->G, a->F15, a->qbar, a->G2, a->ap, a->amask);
     else k_flux_adj<false><<<kPointBlocks, 256, 0, st>>>(q, nullptr, a->F15, a->qbar, nullptr, a->ap, a->amask);
@@ -227,7 +254,7 @@ static int rhs_vjp(cs_adjoint *a, const double *q, const double *lam, double *ou
     if (visc) {
         for (int b = 0; b < 3; ++b) {
             if (!a->active[b]) continue;
-            if (int rc = lines(a, b, true, a->G2 + 4 * b * lmx, lmx, a->phi4, lmx, 4, have_pb, 1.0, st)) return rc;
+            if (int rc = lines(a, b, true, a->G2 + 4 * b * lmx, lmx, a->phi4, lmx, 4, have_pb, st)) return rc;
             have_pb = true;
         }
     }
@@ -249,7 +276,7 @@ extern "C" {
 int cs_adjoint_destroy(cs_adjoint *a) {
     if (!a) return set_error(CS_ERR_INVALID, "null argument");
     if (a->fwd) cs_solver_destroy(a->fwd);
-    for (double *p : {a->G, a->G2, a->phi4, a->F15, a->qbar, a->t1, a->t2, a->t3, a->partial, a->rf, a->drf, a->qbf,
+    for (double *p : {a->G, a->G2, a->phi4, a->F15, a->qbar, a->t1, a->t2, a->t3, a->partial, a->bcol, a->rf, a->drf, a->qbf,
                       a->lamx, a->sweep})
         cudaFree(p);
     cudaFree(a->dtacc);
@@ -279,8 +306,10 @@ int cs_adjoint_create(cs_adjoint **out, const cs_solver_config *cfg) {
         if (n[ax] == 1) continue;
         if (n[ax] > 512) { cs_adjoint_destroy(a); return set_error(CS_ERR_UNSUPPORTED, "adjoint: lines of at most 512 points"); }
         a->tab[ax] = a->tables.get(n[ax], kDeriv, a->ndf[0][ax], a->ndf[1][ax], 0.0);
-        a->tabT[ax] = a->tables.get(n[ax], kDerivT, a->ndf[0][ax], a->ndf[1][ax], 0.0);
-        if (!a->tab[ax] || !a->tabT[ax]) { cs_adjoint_destroy(a); return CS_ERR_UNSUPPORTED; }
+        const int min_lt = ax > 0 && warp_column(n[ax]) ? kWarpChunk : 2;
+        a->ltab[ax] = a->tables.get(n[ax], kDeriv, a->ndf[0][ax], a->ndf[1][ax], 0.0, min_lt);
+        a->tabT[ax] = a->tables.get(n[ax], kDerivT, a->ndf[0][ax], a->ndf[1][ax], 0.0, min_lt);
+        if (!a->tab[ax] || !a->ltab[ax] || !a->tabT[ax]) { cs_adjoint_destroy(a); return CS_ERR_UNSUPPORTED; }
         a->active[ax] = 1;
         a->amask |= 1 << ax;
     }
@@ -300,12 +329,20 @@ int cs_adjoint_create(cs_adjoint **out, const cs_solver_config *cfg) {
     const bool ok = alloc(&a->G, 12) && alloc(&a->G2, 12) && alloc(&a->phi4, 4) && alloc(&a->F15, 15) &&
                     alloc(&a->qbar, 5) && alloc(&a->t1, 5) && alloc(&a->t2, 5) && alloc(&a->t3, 5) &&
                     cudaMalloc(&a->partial, kPointBlocks * sizeof(double)) == cudaSuccess &&
+                    cudaMalloc(&a->bcol, 3 * 64 * sizeof(double)) == cudaSuccess &&
                     cudaMalloc(&a->dtacc, 2 * sizeof(unsigned long long)) == cudaSuccess;
     if (!ok) {
         cs_adjoint_destroy(a);
         return set_error(CS_ERR_ALLOC, "adjoint scratch allocation failed");
     }
     cudaMemset(a->G, 0, 12 * lmx * sizeof(double));
+    double bcol[3 * 64] = {};
+    for (int ax = 0; ax < 3; ++ax)
+        if (a->active[ax]) closure_columns(n[ax], a->ndf[0][ax], a->ndf[1][ax], a->cf, bcol + ax * 64);
+    if (cudaMemcpy(a->bcol, bcol, sizeof bcol, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cs_adjoint_destroy(a);
+        return set_error(CS_ERR_CUDA, "adjoint closure columns upload failed");
+    }
     if (cfg->gcbc && a->active[0])
         a->gcbc_mask = (cfg->nbc[0][0] == CS_BC_NON_REFLECTIVE ? 1 : 0) | (cfg->nbc[1][0] == CS_BC_NON_REFLECTIVE ? 2 : 0);
     if (a->gcbc_mask) {
@@ -324,7 +361,7 @@ int cs_adjoint_deriv(cs_adjoint *a, int axis, int transpose, const double *in, d
                      int accumulate, void *stream) {
     if (!a || !in || !out || axis < 0 || axis > 2 || nfields < 1) return set_error(CS_ERR_INVALID, "bad argument");
     if (!a->active[axis]) return set_error(CS_ERR_INVALID, "axis %d has a single point", axis);
-    return lines(a, axis, transpose != 0, in, a->lmx, out, a->lmx, nfields, accumulate != 0, 1.0,
+    return lines(a, axis, transpose != 0, in, a->lmx, out, a->lmx, nfields, accumulate != 0,
                  (cudaStream_t)stream);
 }
 

@@ -15,20 +15,20 @@
 namespace csb {
 
 // Column j of the closure rows 0, 1, n-2, n-1 of B.
-__device__ __forceinline__ double brow0(int j, int n, int nstart, const Coeffs &cf) {
+__host__ __device__ inline double brow0(int j, int n, int nstart, const Coeffs &cf) {
     if (nstart) return (j < kLmd ? cf.pbci[j] : 0.0) + (n - 1 - j < kLmd ? cf.pbco[n - 1 - j] : 0.0);
     return j == 0 ? kAb00 : (j == 1 ? kAb01 : (j == 2 ? kAb02 : 0.0));
 }
-__device__ __forceinline__ double brow1(int j, int n, int nstart, const Coeffs &cf) {
+__host__ __device__ inline double brow1(int j, int n, int nstart, const Coeffs &cf) {
     if (nstart)
         return (j < kLmd ? cf.pbci[kLmd + j] : 0.0) + (n - 1 - j < kLmd ? cf.pbco[kLmd + n - 1 - j] : 0.0);
     return j == 0 ? -kAb10 : (j == 2 ? kAb10 : 0.0);
 }
-__device__ __forceinline__ double browm1(int j, int n, int nend, const Coeffs &cf) {
+__host__ __device__ inline double browm1(int j, int n, int nend, const Coeffs &cf) {
     if (nend) return -((n - 1 - j < kLmd ? cf.pbci[n - 1 - j] : 0.0) + (j < kLmd ? cf.pbco[j] : 0.0));
     return j == n - 1 ? -kAb00 : (j == n - 2 ? -kAb01 : (j == n - 3 ? -kAb02 : 0.0));
 }
-__device__ __forceinline__ double browm2(int j, int n, int nend, const Coeffs &cf) {
+__host__ __device__ inline double browm2(int j, int n, int nend, const Coeffs &cf) {
     if (nend)
         return -((n - 1 - j < kLmd ? cf.pbci[kLmd + n - 1 - j] : 0.0) + (j < kLmd ? cf.pbco[kLmd + j] : 0.0));
     return j == n - 3 ? -kAb10 : (j == n - 1 ? kAb10 : 0.0);
@@ -94,12 +94,315 @@ __device__ __forceinline__ void filter_stencil_t(const double *z, int n, int lan
     }
 }
 
-// out[f] (=|+=) scale * D (or D^T) in[f] along AXIS, field f = blockIdx.y, or
-// the compact filter (FILTER) and its transpose; one warp per line, 8 lines
-// per CTA.
+// The closure columns of B^T for the eight points at either end of a line: the
+// weights of z[0], z[1], z[n-2], z[n-1] in column k (k < 8: point k; else point
+// n-1-(k-8)), w[k * 4 + .].  Built on the host once per axis.
+inline void closure_columns(int n, int nstart, int nend, const Coeffs &cf, double *w) {
+    for (int k = 0; k < 2 * kLmd; ++k) {
+        const int j = k < kLmd ? k : n - 1 - (k - kLmd);
+        w[k * 4 + 0] = brow0(j, n, nstart, cf);
+        w[k * 4 + 1] = brow1(j, n, nstart, cf);
+        w[k * 4 + 2] = browm2(j, n, nend, cf);
+        w[k * 4 + 3] = browm1(j, n, nend, cf);
+    }
+}
+
+// Interior part of o = B^T z for chunk c from its window w = z[c LT - 2 .. c LT
+// + LT + 1]: rows i in [2, n-3] have B[i][i+-1] = +-a, B[i][i+-2] = +-b.
+template <int LT>
+__device__ __forceinline__ void chunk_stencil_t(const double (&w)[LT + 4], int c, int n, double (&o)[LT]) {
+    const int j0 = c * LT;
+    if (j0 >= 4 && j0 + LT <= n - 4) {
+#pragma unroll
+        for (int t = 0; t < LT; ++t) o[t] = kAa * (w[t + 1] - w[t + 3]) + kBb * (w[t] - w[t + 4]);
+        return;
+    }
+    double m[LT + 4];
+#pragma unroll
+    for (int k = 0; k < LT + 4; ++k) {
+        const int i = j0 + k - 2;
+        m[k] = i >= 2 && i <= n - 3 ? w[k] : 0.0;
+    }
+#pragma unroll
+    for (int t = 0; t < LT; ++t)
+        o[t] = j0 + t < n ? kAa * (m[t + 1] - m[t + 3]) + kBb * (m[t] - m[t + 4]) : 0.0;
+}
+
+// One launch's fields: out[f] = or += D (D^T) in[f], f = blockIdx.y.
+struct LineSet {
+    const double *in;
+    double *out;
+    int64_t in_fs, out_fs;
+    int accum;
+};
+
+// D or D^T along x (k_deriv_row's form, numerics.cu): a warp solves NV lines,
+// each lane loading its chunks with VB-byte vectors.  The transposed closure
+// columns are formed by 16 lanes and handed to the chunks that hold them.
+template <int LT, int NV, int VB, bool TRANS>
+__global__ void __launch_bounds__(256, LT <= 8 ? 3 : 1)
+k_lines_row(LineSet ls, DevTables<double> tab, int F, int nstart, int nend, Coeffs cf, const double *__restrict__ bcol) {
+    constexpr int VE = VB / 8;
+    __shared__ double ends[8][NV][2 * kLmd + 1];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31, j0 = lane * LT;
+    const int len = lane_len(lane, LT, tab.p, tab.last_len);
+    const int line0 = ((int)blockIdx.x * 8 + w) * NV;
+    if (line0 >= F) return;
+    const int64_t base = (int64_t)line0 * n + j0;
+    const double *in = ls.in + blockIdx.y * ls.in_fs + base;
+    double d[NV][LT];
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        const double *src = in + (line0 + h < F ? h : 0) * (int64_t)n;
+#pragma unroll
+        for (int t = 0; t < LT; t += VE) {
+            if (t < len) {
+                load_vec<VB, double>(src + t, &d[h][t]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < VE; ++k) d[h][t + k] = 0.0;
+            }
+        }
+    }
+    if (!TRANS) {
+        double rows = 0.0;
+        if (nstart || nend) {
+            chunk_put_ends<LT, NV, double>(ends[w], d, lane, len, n);
+            __syncwarp();
+            rows = ends_closure_row<double>(ends[w][(lane >> 3) < NV ? lane >> 3 : 0], lane & 7, cf);
+        }
+#pragma unroll
+        for (int h = 0; h < NV; ++h) chunk_warp_rhs<LT, double>(rows, h, lane, len, n, nstart, nend, d[h]);
+    }
+    warp_solve<LT, NV, double>(tab, d, lane);
+    if (TRANS) {
+        double cw[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) cw[k] = bcol[(lane & 15) * 4 + k];
+#pragma unroll
+        for (int h = 0; h < NV; ++h) {
+            double x[LT + 4];
+            x[0] = __shfl_up_sync(0xffffffffu, d[h][LT - 2], 1);
+            x[1] = __shfl_up_sync(0xffffffffu, d[h][LT - 1], 1);
+            x[LT + 2] = __shfl_down_sync(0xffffffffu, d[h][0], 1);
+            x[LT + 3] = __shfl_down_sync(0xffffffffu, d[h][1], 1);
+#pragma unroll
+            for (int t = 0; t < LT; ++t) x[t + 2] = d[h][t];
+            const double z0 = __shfl_sync(0xffffffffu, d[h][0], 0), z1 = __shfl_sync(0xffffffffu, d[h][1], 0);
+            const double zm1 = __shfl_sync(0xffffffffu, get_at<LT, double>(d[h], (n - 1) % LT), (n - 1) / LT);
+            const double zm2 = __shfl_sync(0xffffffffu, get_at<LT, double>(d[h], (n - 2) % LT), (n - 2) / LT);
+            if (lane < 16) ends[w][h][lane] = z0 * cw[0] + z1 * cw[1] + zm2 * cw[2] + zm1 * cw[3];
+            chunk_stencil_t<LT>(x, lane, n, d[h]);
+        }
+        __syncwarp();
+        if (j0 < kLmd || j0 + LT > n - kLmd) {
+#pragma unroll
+            for (int h = 0; h < NV; ++h)
+#pragma unroll
+                for (int t = 0; t < LT; ++t) {
+                    const int j = j0 + t;
+                    if (j < kLmd) d[h][t] += ends[w][h][j];
+                    else if (t < len && j >= n - kLmd) d[h][t] += ends[w][h][kLmd + n - 1 - j];
+                }
+        }
+    }
+    double *out = ls.out + blockIdx.y * ls.out_fs + base;
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        if (line0 + h >= F) break;
+#pragma unroll
+        for (int t = 0; t < LT; t += VE)
+            if (t < len) {
+                double *o = out + (int64_t)h * n + t;
+                if (ls.accum) {
+                    double r[VE];
+                    load_vec<VB, double>(o, r);
+#pragma unroll
+                    for (int k = 0; k < VE; ++k) d[h][t + k] += r[k];
+                }
+                store_vec<VB, double>(o, &d[h][t]);
+            }
+    }
+}
+
+// D or D^T along y and z for the lines of warp_column (k_deriv_wcol's form): four
+// lines per warp.
+template <int LT, int AXIS, bool TRANS>
+__global__ void __launch_bounds__(256, 3)
+k_lines_wcol(LineSet ls, DevTables<double> tab, int lxi, int let, int F, int nstart, int nend, Coeffs cf,
+             const double *__restrict__ bcol) {
+    __shared__ double ends[8][kWarpLines][2 * kLmd + 1];
+    const int n = tab.n, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int l = lane % kWarpLines, c = lane / kWarpLines, j0 = c * LT;
+    const int len = lane_len(c, LT, tab.p, tab.last_len);
+    const int line0 = ((int)blockIdx.x * 8 + w) * kWarpLines, s = AXIS == 1 ? lxi : lxi * let;
+    if (line0 >= F) return;
+    const int fidx = min(line0 + l, F - 1);  // past the last line: the last line again, not stored
+    const int base = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + j0 * s;
+    const double *in = ls.in + blockIdx.y * ls.in_fs;
+    double d[1][LT];
+#pragma unroll
+    for (int t = 0; t < LT; ++t) d[0][t] = t < len ? in[base + t * s] : 0.0;
+    if (!TRANS) warp_column_rhs<LT, double>(ends[w], lane, len, n, nstart, nend, cf, nullptr, d);
+    warp_column_solve<LT, double>(tab, lane, len, d);
+    if (TRANS) {
+        const double z0 = __shfl_sync(0xffffffffu, d[0][0], l), z1 = __shfl_sync(0xffffffffu, d[0][1], l);
+        const double zm1 = __shfl_sync(0xffffffffu, get_at<LT, double>(d[0], (n - 1) % LT), (n - 1) / LT * kWarpLines + l);
+        const double zm2 = __shfl_sync(0xffffffffu, get_at<LT, double>(d[0], (n - 2) % LT), (n - 2) / LT * kWarpLines + l);
+        // the 16 closure columns of line l: two per lane
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double *cw = bcol + 4 * (c + 8 * k);
+            ends[w][l][c + 8 * k] = z0 * cw[0] + z1 * cw[1] + zm2 * cw[2] + zm1 * cw[3];
+        }
+        double x[LT + 4];
+        x[0] = __shfl_up_sync(0xffffffffu, d[0][LT - 2], kWarpLines);
+        x[1] = __shfl_up_sync(0xffffffffu, d[0][LT - 1], kWarpLines);
+        x[LT + 2] = __shfl_down_sync(0xffffffffu, d[0][0], kWarpLines);
+        x[LT + 3] = __shfl_down_sync(0xffffffffu, d[0][1], kWarpLines);
+#pragma unroll
+        for (int t = 0; t < LT; ++t) x[t + 2] = d[0][t];
+        chunk_stencil_t<LT>(x, c, n, d[0]);
+        __syncwarp();
+        if (j0 < kLmd || j0 + LT > n - kLmd) {
+#pragma unroll
+            for (int t = 0; t < LT; ++t) {
+                const int j = j0 + t;
+                if (j < kLmd) d[0][t] += ends[w][l][j];
+                else if (t < len && j >= n - kLmd) d[0][t] += ends[w][l][kLmd + n - 1 - j];
+            }
+        }
+    }
+    if (len == 0 || line0 + l >= F) return;
+    double *out = ls.out + blockIdx.y * ls.out_fs;
+    if (ls.accum) {
+        constexpr int B = 8;
+#pragma unroll
+        for (int t0 = 0; t0 < LT; t0 += B) {
+            double r[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                if (t0 + b < len) r[b] = out[base + (t0 + b) * s];
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                if (t0 + b < len) out[base + (t0 + b) * s] = r[b] + d[0][t0 + b];
+        }
+    } else {
+#pragma unroll
+        for (int t = 0; t < LT; ++t)
+            if (t < len) out[base + t * s] = d[0][t];
+    }
+}
+
+// The same for all other y and z lines (k_deriv_col's form): column tiles of two groups of
+// TL lines.
+template <int LT, int AXIS, int TL, bool TRANS>
+__global__ void __launch_bounds__(TL * 32, LT <= 8 ? 768 / (TL * 32) : 2)
+k_lines_col(LineSet ls, DevTables<double> tab, int lxi, int let, int F, int nstart, int nend, Coeffs cf,
+            const double *__restrict__ bcol) {
+    using C = Column<LT, TL>;
+    constexpr int NL = 2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *V = reinterpret_cast<double *>(smem_raw), *rows = V + NL * C::kField;  // rows: [NL][TL][16]
+    const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL, j0 = c * LT;
+    const int len = lane_len(c, LT, tab.p, tab.last_len);
+    const int line0 = (int)blockIdx.x * (NL * TL), s = AXIS == 1 ? lxi : lxi * let;
+    int base[NL];
+#pragma unroll
+    for (int h = 0; h < NL; ++h) {
+        const int fidx = min(line0 + h * TL + l, F - 1);  // past the last line: the last line again, not stored
+        base[h] = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + j0 * s;
+    }
+    const double *in = ls.in + blockIdx.y * ls.in_fs;
+    double d[NL][LT];
+#pragma unroll
+    for (int t = 0; t < LT; ++t)
+#pragma unroll
+        for (int h = 0; h < NL; ++h) d[h][t] = t < len ? in[base[h] + t * s] : 0.0;
+    if (!TRANS) {
+#pragma unroll
+        for (int h = 0; h < NL; ++h) column_put_raw<LT, TL, double>(V + h * C::kField, d[h], c, l, n);
+        __syncthreads();
+        if (nstart || nend) column_closure_rows<LT, TL, NL, double, double>(V, rows, n, cf, nullptr, F, line0);
+#pragma unroll
+        for (int h = 0; h < NL; ++h) column_rhs<LT, TL, double>(V + h * C::kField, c, l, len, n, nstart, nend, d[h]);
+        __syncthreads();
+        if (nstart || nend) {
+#pragma unroll
+            for (int h = 0; h < NL; ++h) column_take_rows<LT, double>(rows + 4 * (h * TL + l), c, n, nstart, nend, d[h]);
+        }
+    }
+    chunk_eliminate<LT, NL, double>(tab, d, c);
+#pragma unroll
+    for (int h = 0; h < NL; ++h) column_put_ends<LT, TL, double>(V + h * C::kField, d[h], c, l, len);
+    __syncthreads();
+    column_reduced<LT, TL, NL, double>(V, tab);
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < NL; ++h) column_finish<LT, TL, double>(V + h * C::kField, tab, c, l, len, d[h]);
+    if (TRANS) {
+        // the end rows read by column_finish are this thread's own
+#pragma unroll
+        for (int h = 0; h < NL; ++h) column_put_raw<LT, TL, double>(V + h * C::kField, d[h], c, l, n);
+        __syncthreads();
+        for (int i = threadIdx.x; i < NL * TL * 16; i += blockDim.x) {
+            const int ll = i % TL, h = i / TL % NL, k = i / (TL * NL);
+            const double *z = V + h * C::kField, *cw = bcol + 4 * k;
+            rows[(h * TL + ll) * 16 + k] = z[C::pos(0, ll)] * cw[0] + z[C::pos(1, ll)] * cw[1] +
+                                           z[C::pos(n - 2, ll)] * cw[2] + z[C::pos(n - 1, ll)] * cw[3];
+        }
+        const int cm = c > 0 ? c - 1 : 0, cp = c < 31 ? c + 1 : 31;
+#pragma unroll
+        for (int h = 0; h < NL; ++h) {
+            const double *z = V + h * C::kField;
+            double x[LT + 4];
+            x[0] = z[C::at(LT - 2, cm, l)];
+            x[1] = z[C::at(LT - 1, cm, l)];
+            x[LT + 2] = z[C::at(0, cp, l)];
+            x[LT + 3] = z[C::at(1, cp, l)];
+#pragma unroll
+            for (int t = 0; t < LT; ++t) x[t + 2] = d[h][t];
+            chunk_stencil_t<LT>(x, c, n, d[h]);
+        }
+        __syncthreads();
+        if (j0 < kLmd || j0 + LT > n - kLmd) {
+#pragma unroll
+            for (int h = 0; h < NL; ++h)
+#pragma unroll
+                for (int t = 0; t < LT; ++t) {
+                    const int j = j0 + t;
+                    const double *e = rows + (h * TL + l) * 16;
+                    if (j < kLmd) d[h][t] += e[j];
+                    else if (t < len && j >= n - kLmd) d[h][t] += e[kLmd + n - 1 - j];
+                }
+        }
+    }
+    double *out = ls.out + blockIdx.y * ls.out_fs;
+#pragma unroll
+    for (int h = 0; h < NL; ++h) {
+        if (line0 + h * TL + l >= F) break;
+        if (ls.accum) {
+            double r[LT];
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len) r[t] = out[base[h] + t * s];
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len) out[base[h] + t * s] = r[t] + d[h][t];
+        } else {
+#pragma unroll
+            for (int t = 0; t < LT; ++t)
+                if (t < len) out[base[h] + t * s] = d[h][t];
+        }
+    }
+}
+
+// The same for x rows of any length and start, and the compact filter (FILTER)
+// and its transpose along AXIS: one warp per line, 8 lines per CTA, staged in
+// shared memory.
 template <int LT, int AXIS, bool TRANS, bool FILTER = false>
 __global__ void __launch_bounds__(256) k_lines(const double *__restrict__ in, int64_t in_fs,
-                                               double *__restrict__ out, int64_t out_fs, int accum, double scale,
+                                               double *__restrict__ out, int64_t out_fs, int accum,
                                                DevTables<double> tab, int lxi, int let, int64_t F, int nstart,
                                                int nend, Coeffs cf, double af = 0.0) {
     constexpr int TL = 8;
@@ -139,7 +442,7 @@ __global__ void __launch_bounds__(256) k_lines(const double *__restrict__ in, in
     }
     tile_sync<AXIS, TL>();
     tile_for_each<AXIS, TL>(line0, F, n, lxi, let, [&](int l, int j, int64_t gi) {
-        const double v = scale * sm[l * L::kSlot + L::pos(j)];
+        const double v = sm[l * L::kSlot + L::pos(j)];
         dst[gi] = accum ? dst[gi] + v : v;
     });
 }
@@ -165,9 +468,10 @@ __global__ void k_prim_tan(const double *__restrict__ q, const double *__restric
     }
 }
 
-// dF[a][m] = (dF_a/dq) dq + (dF_a/dG) dG for every active axis a
+// dF[a][m] = (dF_a/dq) dq + (dF_a/dG) dG for every active axis a (the adjoint
+// runs on the uniform grid, whose metric matrix is diagonal)
 template <bool VISC>
-__global__ void k_flux_tan(const double *__restrict__ q, const double *__restrict__ G, const double *__restrict__ dq,
+__global__ void __launch_bounds__(256, 2) k_flux_tan(const double *__restrict__ q, const double *__restrict__ G, const double *__restrict__ dq,
                            const double *__restrict__ dG, double *__restrict__ dF, AdjPoint ap, int amask) {
     const int64_t lmx = ap.lmx;
     CSB_GRID_STRIDE(i, lmx) {
@@ -177,9 +481,10 @@ __global__ void k_flux_tan(const double *__restrict__ q, const double *__restric
             g[k] = VISC ? G[k * lmx + i] : 0.0;
             dg[k] = VISC ? dG[k * lmx + i] : 0.0;
         }
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
             if (!(amask >> a & 1)) continue;
-            flux_tan<VISC>(a, qq, g, d, dg, ap.ph, o);
+            flux_tan<VISC, true>(a, qq, g, d, dg, ap.ph, o);
             for (int m = 0; m < 5; ++m) dF[(a * 5 + m) * lmx + i] = o[m];
         }
     }
@@ -187,7 +492,7 @@ __global__ void k_flux_tan(const double *__restrict__ q, const double *__restric
 
 // qbar = sum_a (dF_a/dq)^T mu_a,  Gbar = sum_a (dF_a/dG)^T mu_a
 template <bool VISC>
-__global__ void k_flux_adj(const double *__restrict__ q, const double *__restrict__ G, const double *__restrict__ mu,
+__global__ void __launch_bounds__(256, 2) k_flux_adj(const double *__restrict__ q, const double *__restrict__ G, const double *__restrict__ mu,
                            double *__restrict__ qbar, double *__restrict__ Gbar, AdjPoint ap, int amask) {
     const int64_t lmx = ap.lmx;
     CSB_GRID_STRIDE(i, lmx) {
@@ -197,10 +502,11 @@ __global__ void k_flux_adj(const double *__restrict__ q, const double *__restric
             g[k] = VISC ? G[k * lmx + i] : 0.0;
             gb[k] = 0.0;
         }
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
             if (!(amask >> a & 1)) continue;
             for (int m = 0; m < 5; ++m) fb[m] = mu[(a * 5 + m) * lmx + i];
-            flux_adj<VISC>(a, qq, g, fb, ap.ph, qb, gb);
+            flux_adj<VISC, true>(a, qq, g, fb, ap.ph, qb, gb);
         }
         for (int m = 0; m < 5; ++m) qbar[m * lmx + i] = qb[m];
         if (VISC)

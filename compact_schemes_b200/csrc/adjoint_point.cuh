@@ -113,8 +113,22 @@ CSB_HD void flux_eval(int a, const double q[5], const double G[12], const PointP
     }
 }
 
+// The linearizations take DIAG where the metric matrix is diagonal (the uniform
+// Cartesian grid) and the axis a compile-time constant of an unrolled loop: the
+// products with the matrix' zero entries are then left out.
+template <bool DIAG>
+CSB_HD double metric_dot(const double *Ma, int a, double x0, double x1, double x2) {
+    if (DIAG) return Ma[a] * (a == 0 ? x0 : (a == 1 ? x1 : x2));
+    return Ma[0] * x0 + Ma[1] * x1 + Ma[2] * x2;
+}
+template <bool DIAG>
+CSB_HD double metric_grad(const PointPhys &ph, const double *G, int c, int k) {
+    if (DIAG) return ph.M[k][k] * G[4 * k + c];
+    return ph.M[0][k] * G[c] + ph.M[1][k] * G[4 + c] + ph.M[2][k] * G[8 + c];
+}
+
 // dF = (dF/dq) dq + (dF/dG) dG
-template <bool VISC>
+template <bool VISC, bool DIAG = false>
 CSB_HD void flux_tan(int a, const double q[5], const double G[12], const double dq[5], const double dG[12],
                      const PointPhys &ph, double dF[5]) {
     const double ri = 1.0 / q[0];
@@ -126,20 +140,21 @@ CSB_HD void flux_tan(int a, const double q[5], const double G[12], const double 
     const double dmm = 2.0 * (q[1] * dq[1] + q[2] * dq[2] + q[3] * dq[3]);
     const double dp = kGamm1 * (dq[4] - 0.5 * (dmm * ri + mm * dri));
     const double *Ma = ph.M[a];
-    const double ss = Ma[0] * (u + ph.umf[0]) + Ma[1] * (v + ph.umf[1]) + Ma[2] * (w + ph.umf[2]);
-    const double dss = Ma[0] * du + Ma[1] * dv + Ma[2] * dw;
-    const double mu_dot = ph.umf[0] * Ma[0] + ph.umf[1] * Ma[1] + ph.umf[2] * Ma[2];
+    const double ss = metric_dot<DIAG>(Ma, a, u + ph.umf[0], v + ph.umf[1], w + ph.umf[2]);
+    const double dss = metric_dot<DIAG>(Ma, a, du, dv, dw);
+    const double mu_dot = metric_dot<DIAG>(Ma, a, ph.umf[0], ph.umf[1], ph.umf[2]);
     dF[0] = dq[0] * ss + q[0] * dss;
-    dF[1] = dq[1] * ss + q[1] * dss + Ma[0] * dp;
-    dF[2] = dq[2] * ss + q[2] * dss + Ma[1] * dp;
-    dF[3] = dq[3] * ss + q[3] * dss + Ma[2] * dp;
+    for (int i = 0; i < 3; ++i) {
+        dF[1 + i] = dq[1 + i] * ss + q[1 + i] * dss;
+        if (!DIAG || i == a) dF[1 + i] += Ma[i] * dp;
+    }
     dF[4] = (dq[4] + dp) * ss + (q[4] + p) * dss - dp * mu_dot;
     if (VISC) {
         double dx[4][3], ddx[4][3];
         for (int c = 0; c < 4; ++c)
             for (int k = 0; k < 3; ++k) {
-                dx[c][k] = ph.M[0][k] * G[c] + ph.M[1][k] * G[4 + c] + ph.M[2][k] * G[8 + c];
-                ddx[c][k] = ph.M[0][k] * dG[c] + ph.M[1][k] * dG[4 + c] + ph.M[2][k] * dG[8 + c];
+                dx[c][k] = metric_grad<DIAG>(ph, G, c, k);
+                ddx[c][k] = metric_grad<DIAG>(ph, dG, c, k);
             }
         const double muj = ph.mu * ph.J, kap = kGamm1Prndtli * muj;
         double t[3][3], dt[3][3];
@@ -153,10 +168,12 @@ CSB_HD void flux_tan(int a, const double q[5], const double G[12], const double 
         const double uu[3] = {u, v, w}, duu[3] = {du, dv, dw};
         for (int i = 0; i < 3; ++i) {
             double s = 0.0;
-            for (int k = 0; k < 3; ++k) s += Ma[k] * dt[i][k];
+            for (int k = 0; k < 3; ++k)
+                if (!DIAG || k == a) s += Ma[k] * dt[i][k];
             dF[1 + i] -= s;
         }
         for (int k = 0; k < 3; ++k) {
+            if (DIAG && k != a) continue;
             double dh = kap * ddx[3][k];
             for (int i = 0; i < 3; ++i) dh += duu[i] * t[i][k] + uu[i] * dt[i][k];
             dF[4] -= Ma[k] * dh;
@@ -165,7 +182,7 @@ CSB_HD void flux_tan(int a, const double q[5], const double G[12], const double 
 }
 
 // qbar += (dF/dq)^T Fb,  Gbar += (dF/dG)^T Fb
-template <bool VISC>
+template <bool VISC, bool DIAG = false>
 CSB_HD void flux_adj(int a, const double q[5], const double G[12], const double Fb[5], const PointPhys &ph,
                      double qbar[5], double Gbar[12]) {
     const double ri = 1.0 / q[0];
@@ -173,14 +190,14 @@ CSB_HD void flux_adj(int a, const double q[5], const double G[12], const double 
     const double mm = q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
     const double p = kGamm1 * (q[4] - 0.5 * (q[1] * u + q[2] * v + q[3] * w));
     const double *Ma = ph.M[a];
-    const double ss = Ma[0] * (u + ph.umf[0]) + Ma[1] * (v + ph.umf[1]) + Ma[2] * (w + ph.umf[2]);
-    const double mu_dot = ph.umf[0] * Ma[0] + ph.umf[1] * Ma[1] + ph.umf[2] * Ma[2];
+    const double ss = metric_dot<DIAG>(Ma, a, u + ph.umf[0], v + ph.umf[1], w + ph.umf[2]);
+    const double mu_dot = metric_dot<DIAG>(Ma, a, ph.umf[0], ph.umf[1], ph.umf[2]);
     double ub[3] = {0.0, 0.0, 0.0};
     if (VISC) {
         double dx[4][3];
         for (int c = 0; c < 4; ++c)
             for (int k = 0; k < 3; ++k)
-                dx[c][k] = ph.M[0][k] * G[c] + ph.M[1][k] * G[4 + c] + ph.M[2][k] * G[8 + c];
+                dx[c][k] = metric_grad<DIAG>(ph, G, c, k);
         const double muj = ph.mu * ph.J, kap = kGamm1Prndtli * muj;
         const double div = 2.0 / 3.0 * (dx[0][0] + dx[1][1] + dx[2][2]);
         double t[3][3];
@@ -189,47 +206,61 @@ CSB_HD void flux_adj(int a, const double q[5], const double G[12], const double 
         const double uu[3] = {u, v, w};
         // F4 -= sum_k Ma[k] h_k,  h_k = kap dx[3][k] + sum_i u_i t[i][k]
         // F(1+i) -= sum_k Ma[k] t[i][k]
-        double tb[3][3], dxb[4][3];
-        for (int c = 0; c < 4; ++c)
-            for (int k = 0; k < 3; ++k) dxb[c][k] = 0.0;
-        for (int k = 0; k < 3; ++k) {
-            const double hb = -Ma[k] * Fb[4];
-            dxb[3][k] += kap * hb;
+        if (DIAG) {
+            // only column a of t enters, and dx[c][k] = M[k][k] G[4 k + c]
+            const double hb = -Ma[a] * Fb[4];
+            Gbar[4 * a + 3] += ph.M[a][a] * (kap * hb);
+            double divb = 0.0;
             for (int i = 0; i < 3; ++i) {
-                ub[i] += t[i][k] * hb;
-                tb[i][k] = uu[i] * hb - Ma[k] * Fb[1 + i];
+                ub[i] += t[i][a] * hb;
+                const double tb = muj * (uu[i] * hb - Ma[a] * Fb[1 + i]);
+                Gbar[4 * a + i] += ph.M[a][a] * tb;
+                Gbar[4 * i + a] += ph.M[i][i] * tb;
+                if (i == a) divb = -tb;
             }
-        }
-        // t[i][k] = muj (dx[i][k] + dx[k][i]) - [i==k] muj div
-        double divb = 0.0;
-        for (int i = 0; i < 3; ++i)
+            for (int i = 0; i < 3; ++i) Gbar[4 * i + i] += ph.M[i][i] * (2.0 / 3.0 * divb);
+        } else {
+            double tb[3][3], dxb[4][3];
+            for (int c = 0; c < 4; ++c)
+                for (int k = 0; k < 3; ++k) dxb[c][k] = 0.0;
             for (int k = 0; k < 3; ++k) {
-                dxb[i][k] += muj * tb[i][k];
-                dxb[k][i] += muj * tb[i][k];
-                if (i == k) divb -= muj * tb[i][k];
+                const double hb = -Ma[k] * Fb[4];
+                dxb[3][k] += kap * hb;
+                for (int i = 0; i < 3; ++i) {
+                    ub[i] += t[i][k] * hb;
+                    tb[i][k] = uu[i] * hb - Ma[k] * Fb[1 + i];
+                }
             }
-        for (int i = 0; i < 3; ++i) dxb[i][i] += 2.0 / 3.0 * divb;
-        // dx[c][k] = sum_b M[b][k] G[b*4 + c]
-        for (int b = 0; b < 3; ++b)
-            for (int c = 0; c < 4; ++c) {
-                double s = 0.0;
-                for (int k = 0; k < 3; ++k) s += ph.M[b][k] * dxb[c][k];
-                Gbar[b * 4 + c] += s;
-            }
+            // t[i][k] = muj (dx[i][k] + dx[k][i]) - [i==k] muj div
+            double divb = 0.0;
+            for (int i = 0; i < 3; ++i)
+                for (int k = 0; k < 3; ++k) {
+                    dxb[i][k] += muj * tb[i][k];
+                    dxb[k][i] += muj * tb[i][k];
+                    if (i == k) divb -= muj * tb[i][k];
+                }
+            for (int i = 0; i < 3; ++i) dxb[i][i] += 2.0 / 3.0 * divb;
+            // dx[c][k] = sum_b M[b][k] G[b*4 + c]
+            for (int b = 0; b < 3; ++b)
+                for (int c = 0; c < 4; ++c) {
+                    double s = 0.0;
+                    for (int k = 0; k < 3; ++k) s += ph.M[b][k] * dxb[c][k];
+                    Gbar[b * 4 + c] += s;
+                }
+        }
     }
     // inviscid part
     // F0 = q0 ss; F(1+i) = q(1+i) ss + Ma[i] p; F4 = (q4 + p) ss - p mu_dot
     double ssb = q[0] * Fb[0] + q[1] * Fb[1] + q[2] * Fb[2] + q[3] * Fb[3] + (q[4] + p) * Fb[4];
-    const double pb = Ma[0] * Fb[1] + Ma[1] * Fb[2] + Ma[2] * Fb[3] + (ss - mu_dot) * Fb[4];
+    const double pb = metric_dot<DIAG>(Ma, a, Fb[1], Fb[2], Fb[3]) + (ss - mu_dot) * Fb[4];
     qbar[0] += ss * Fb[0];
     qbar[1] += ss * Fb[1];
     qbar[2] += ss * Fb[2];
     qbar[3] += ss * Fb[3];
     qbar[4] += ss * Fb[4];
     // ss = sum_k Ma[k] (u_k + umf_k)
-    ub[0] += Ma[0] * ssb;
-    ub[1] += Ma[1] * ssb;
-    ub[2] += Ma[2] * ssb;
+    for (int i = 0; i < 3; ++i)
+        if (!DIAG || i == a) ub[i] += Ma[i] * ssb;
     // p = (g-1)(q4 - 0.5 mm ri)
     qbar[4] += kGamm1 * pb;
     const double mmb = -0.5 * kGamm1 * ri * pb;

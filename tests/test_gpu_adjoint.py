@@ -45,6 +45,34 @@ def test_transposed_derivative_dot_product(cuda, dims, nbc_code):
 
 
 @pytest.mark.parametrize("nbc_code", ["periodic", "physical"])
+@pytest.mark.parametrize("n", [8, 10, 17, 33, 66, 68, 127, 132, 255, 260, 512])
+def test_line_operators_lengths(cuda, n, nbc_code):
+    """D against the oracle and D^T by the dot product at lengths around the
+    chunk and vector-access edges, along every axis, with accumulation and with
+    the fields off a 16-byte boundary (the x rows' staged path)."""
+    import compact_schemes_b200 as cs
+    nd = int(nbc_code == "periodic")
+    b = cs.BC_PERIODIC if nd else cs.BC_NON_REFLECTIVE
+    g = torch.Generator(device="cuda:0").manual_seed(n)
+    for axis in range(3):
+        dims = [9, 8, 10]
+        dims[axis] = n
+        _, _, a, _ = _setup(tuple(dims), nbc=[[b] * 3] * 2)
+        m = int(np.prod(dims))
+        for off in (0, 1):
+            x, y, acc = (torch.randn(2 * m + off, dtype=torch.float64, device="cuda:0", generator=g)[off:]
+                         for _ in range(3))
+            Dx, DTy = acc.clone(), torch.empty_like(y)
+            a.deriv(axis, x, Dx, nfields=2, accumulate=True)
+            a.deriv(axis, y, DTy, nfields=2, transpose=True)
+            Dx -= acc
+            for f in range(2):
+                ref = O.deriv(x[f * m:(f + 1) * m].cpu().numpy(), dims, axis, nd, nd)
+                assert np.abs(Dx[f * m:(f + 1) * m].cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
+            assert abs(_dot(y, Dx) - _dot(DTy, x)) <= 1e-12 * float((y.abs() * Dx.abs()).sum()), (axis, off)
+
+
+@pytest.mark.parametrize("nbc_code", ["periodic", "physical"])
 @pytest.mark.parametrize("af", [0.0, 0.45, -0.3])
 def test_transposed_filter_dot_product_and_forward(cuda, nbc_code, af):
     import compact_schemes_b200 as cs
