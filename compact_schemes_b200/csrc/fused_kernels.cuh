@@ -82,6 +82,31 @@ __device__ __forceinline__ void prefetch_tile(const CUtensorMap *map, const Flux
     }
 }
 
+// L2 prefetch of a later tile's inputs: the CTA of tile t fetches the state and
+// the gradients that tile t + kAheadTiles will read.  A pass's CTAs start in
+// order, so that tile starts about one HBM latency later (0.1 us between starts
+// at 256^3) and its loads find the data in L2 or on the way.  An SM keeps only so
+// many load misses in flight, and 64-byte rows use them at half their width (plain
+// copies of tiles with 64 / 128 / 256-byte rows: 3.0 / 5.9 / 6.7 TB/s); the copy
+// engine is not bound by that.
+constexpr int kAheadTiles = 4;
+struct AheadMaps {
+    CUtensorMap m[4];  // state, own axis' gradients, two ranges of the other axes' gradients
+};
+struct Ahead {
+    FluxPrefetch geo;
+    int maps;  // maps in use (bit mask); 0: no prefetch
+};
+template <int AXIS, int TL>
+__device__ __forceinline__ void prefetch_ahead(const AheadMaps &am, const Ahead &ah, int64_t F) {
+    const int64_t line = ((int64_t)blockIdx.x + kAheadTiles) * TL;
+    if (ah.maps && threadIdx.x == 0 && line < F) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (ah.maps >> k & 1) prefetch_tile<AXIS>(&am.m[k], ah.geo, line);
+    }
+}
+
 struct Phys {
     double M[3][3];  // metric rows xim, etm, zem (J^-1 grad xi_a)
     double J;        // yaco
@@ -464,8 +489,9 @@ template <int LT, int AXIS, int TL, bool DTRED, bool FM>
 __global__ void __launch_bounds__(TL * 32, 512 / (TL * 32))
 k_grad_col(const double *__restrict__ q, double *__restrict__ g, DevTables<double> tab, int lxi, int let,
            int64_t lmx, int F, int nstart, int nend, Coeffs cf, Phys ph, unsigned long long *__restrict__ dtacc,
-           FieldMet fm) {
+           FieldMet fm, const __grid_constant__ AheadMaps am, Ahead ah) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (LT == 8) prefetch_ahead<AXIS, TL>(am, ah, F);
     double m1 = 0.0, m2 = 0.0;
     grad_col_tile<LT, AXIS, TL, 32, DTRED, FM>(reinterpret_cast<double *>(smem_raw), (int)blockIdx.x * TL, F, q, g,
                                                tab, lxi, let, lmx, nstart, nend, cf, ph, m1, m2, fm);
@@ -713,8 +739,9 @@ __global__ void __launch_bounds__(TL * 32, TL == 8 ? CSB_FLUX_MINB : 1)
 k_flux(const double *__restrict__ q, const double *__restrict__ g, double *__restrict__ rhs,
        const double *__restrict__ qn, double *__restrict__ qout, double *__restrict__ drva,
        DevTables<double> tab, int lxi, int let, int64_t lmx, int64_t F, int nstart, int nend,
-       Coeffs cf, Phys ph, RkParams rk, FieldMet fm) {
+       Coeffs cf, Phys ph, RkParams rk, FieldMet fm, const __grid_constant__ AheadMaps am, Ahead ah) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (LT == 8) prefetch_ahead<AXIS, TL>(am, ah, F);
     constexpr int P = MODE == kAccum ? (LT >= 16 ? 2 : CSB_RMW_CHUNK) : (LT >= 16 ? 1 : CSB_RMW_CHUNK_RK);
     flux_tile<LT, AXIS, TL, MODE, VISC, false, P, FM>(reinterpret_cast<double *>(smem_raw), (int64_t)blockIdx.x * TL,
                                                       q, g, rhs, qn, qout, drva, tab, lxi, let, lmx, F, nstart, nend,
@@ -1073,6 +1100,42 @@ FluxPrefetch flux_prefetch(const PassArgs &b, const RT *rhs, const double *qn, C
     return pf;
 }
 
+// Tensor maps and geometry of prefetch_ahead for a pass along AXIS with TL-line
+// tiles; `inputs`: the maps the pass reads.  Only for lines of 129..256 points:
+// passes over shorter lines mostly run from L2 and do not gain, a 512-point line's
+// tile fills an SM by itself.  Not on per-point metrics, where rows or field blocks
+// are not 16-byte multiples, and for passes whose tiles all start together.
+// Measured at 256^3 (gradient y, z, flux x, y, z + RK with 16 lines): 0.387, 0.371,
+// 0.520, 0.731, 0.889 -> 0.327, 0.359, 0.495, 0.705, 0.834 ms, at 192^3 0.221,
+// 0.219, 0.266, 0.373, 0.459 -> 0.188, 0.192, 0.259, 0.356, 0.407 ms.  Two to eight
+// tiles ahead are alike, 48 make the flux passes 15-30 % slower, and fetching R and
+// q^n too costs more than it gives.  The z flux pass with 8 lines got slower with
+// it (1.11 -> 1.18 ms at 256^3) and goes without, as do the mixed form's passes
+// (flux y 0.776 -> 0.822, z 1.421 -> 1.481 ms at 512^3).
+template <int AXIS, int TL>
+Ahead pass_ahead(const PassArgs &b, int inputs, const double *q, const double *grad, AheadMaps &am) {
+    Ahead ah{};
+    const int lze = (int)(b.lmx / ((int64_t)b.lxi * b.let));
+    const cs_dcomp d{(int)b.lmx, b.lxi, b.let, lze};
+    const int n = AXIS == 0 ? b.lxi : (AXIS == 1 ? b.let : lze);
+    if (b.tab->lt != 8 || n > 256 || b.fm.xim || (b.F + TL - 1) / TL < 2 * (int64_t)b.nsm) return ah;
+    if (b.lmx % 4 || (AXIS < 2 ? b.lxi % 4 : ((int64_t)b.lxi * b.let) % 4)) return ah;
+    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(grad)) % 16) return ah;
+    ah.geo.nbox = 1;
+    ah.geo.boxlen = (n + 3) / 4 * 4;
+    ah.geo.lxi = b.lxi;
+    // gradients of the other axes on a diagonal metric: x reads u_y v_y | u_z (v_z) w_z, y u_x v_x | v_z w_z,
+    // z u_x (v_x) w_x | v_y w_y
+    constexpr int first[3][2] = {{4, 8}, {0, 9}, {0, 5}}, count[3][2] = {{2, 3}, {2, 2}, {3, 2}};
+    const double *base[4] = {q, grad + 4 * AXIS * b.lmx, grad + first[AXIS][0] * b.lmx, grad + first[AXIS][1] * b.lmx};
+    const int nf[4] = {5, 4, count[AXIS][0], count[AXIS][1]};
+    for (int k = 0; k < 4; ++k)
+        if (inputs >> k & 1)
+            if (tma_field_map_t(AXIS, d, TL, ah.geo.boxlen, nf[k], base[k], am.m[k])) return Ahead{};
+    ah.maps = inputs;
+    return ah;
+}
+
 template <int LT, int VB>
 int launch_grad_row(const PassArgs &a, const double *q, bool dtred, cudaStream_t st) {
     auto kern = dtred ? k_grad_row<LT, VB, true, false> : k_grad_row<LT, VB, false, false>;
@@ -1116,27 +1179,30 @@ int launch_grad_col(const PassArgs &a, const double *q, bool dtred, cudaStream_t
     auto kern = dtred ? k_grad_col<LT, AXIS, TL, true, false> : k_grad_col<LT, AXIS, TL, false, false>;
     if (dtred && a.fm.xim) kern = k_grad_col<LT, AXIS, TL, true, true>;
     if (int rc = set_smem(kern, smem)) return rc;
+    AheadMaps am{};
+    const Ahead ah = pass_ahead<AXIS, TL>(a, 1, q, a.grad, am);
     kern<<<(unsigned)((a.F + TL - 1) / TL), column_threads(TL, a.tab->t64.p), smem, st>>>(
         q, a.grad + (int64_t)AXIS * 4 * a.lmx, a.tab->t64, a.lxi, a.let, a.lmx, (int)a.F, a.nstart, a.nend, a.cf,
-        a.ph, a.dtacc, a.fm);
+        a.ph, a.dtacc, a.fm, am, ah);
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
 }
 
 template <int LT, int AXIS, int TL>
 int launch_grad_t(const PassArgs &a, const double *q, bool dtred, cudaStream_t st) {
-    if constexpr (LT <= 8 && AXIS > 0) return launch_grad_col<LT, AXIS, TL>(a, q, dtred, st);
-    if constexpr (LT <= 8 && AXIS == 0) {
-        auto aligned = [&](int vb) {
-            return LT * 8 >= vb && a.lxi % (vb / 8) == 0 && a.lmx % (vb / 8) == 0 &&
-                   (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(a.grad)) % vb == 0;
-        };
-        if constexpr (LT >= 4) {
-            if (aligned(32)) return launch_grad_row<LT, 32>(a, q, dtred, st);
+    if constexpr (LT <= 8 && AXIS > 0) {
+        return launch_grad_col<LT, AXIS, TL>(a, q, dtred, st);
+    } else {
+        if constexpr (LT <= 8) {
+            auto aligned = [&](int vb) {
+                return LT * 8 >= vb && a.lxi % (vb / 8) == 0 && a.lmx % (vb / 8) == 0 &&
+                       (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(a.grad)) % vb == 0;
+            };
+            if constexpr (LT >= 4) {
+                if (aligned(32)) return launch_grad_row<LT, 32>(a, q, dtred, st);
+            }
+            if (aligned(16)) return launch_grad_row<LT, 16>(a, q, dtred, st);
         }
-        if (aligned(16)) return launch_grad_row<LT, 16>(a, q, dtred, st);
-    }
-    if constexpr (LT > 8 || AXIS == 0) {
         const size_t smem = (size_t)4 * TL * LineLayout<LT>::kSlot * sizeof(double);
         auto kern = dtred ? k_grad<LT, AXIS, TL, true> : k_grad<LT, AXIS, TL, false>;
         if (dtred && a.fm.xim) kern = k_grad<LT, AXIS, TL, true, true>;
@@ -1169,13 +1235,16 @@ int launch_flux_t(const PassArgs &a, const double *q, const double *qn, double *
         CSB_CUDA(cudaGetLastError());
         return CS_OK;
     } else {
+        AheadMaps am{};
+        const int inputs = AXIS == 2 && TL == 8 ? 0 : (a.viscous ? 15 : 1);
+        const Ahead ah = pass_ahead<AXIS, TL>(a, inputs, q, a.grad, am);
         const size_t smem = (size_t)5 * TL * LineLayout<LT>::kSlot * sizeof(double);
         auto kern = a.viscous ? k_flux<LT, AXIS, TL, MODE, true> : k_flux<LT, AXIS, TL, MODE, false>;
         if (a.fm.xim) kern = a.viscous ? k_flux<LT, AXIS, TL, MODE, true, true> : k_flux<LT, AXIS, TL, MODE, false, true>;
         if (int rc = set_smem(kern, smem)) return rc;
         const unsigned blocks = (unsigned)((a.F + TL - 1) / TL);
         kern<<<blocks, TL * 32, smem, st>>>(q, a.grad, a.rhs, qn, qout, drva, a.tab->t64, a.lxi, a.let, a.lmx,
-                                            a.F, a.nstart, a.nend, a.cf, a.ph, rk, a.fm);
+                                            a.F, a.nstart, a.nend, a.cf, a.ph, rk, a.fm, am, ah);
         CSB_CUDA(cudaGetLastError());
         return CS_OK;
     }

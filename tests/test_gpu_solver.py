@@ -69,6 +69,20 @@ def test_rhs_periodic(cuda, dims, viscous):
     assert rhs_err(out.cpu().numpy(), ref, scale) < 1e-12
 
 
+@pytest.mark.parametrize("dims", [(132, 20, 132), (20, 130, 132), (36, 132, 130), (30, 160, 132)])
+def test_rhs_with_tiles_fetched_ahead(cuda, dims):
+    """Enough tiles of 129..256-point lines for the passes to fetch later tiles
+    ahead: boxes past the row, the line and the last tile, and a row length that
+    rules the copies out."""
+    import torch
+    s = solver(dims)
+    q = O.tgv_init(dims, 0.2, 1e-3, 7)
+    ref, scale = O.rhs(q, s.cfg.mu, O.uniform_metrics(*dims), dims, [[1] * 3] * 2, with_scale=True)
+    out = torch.zeros(q.size, dtype=torch.float64, device=cuda)
+    s.rhs(dev(q), out)
+    assert rhs_err(out.cpu().numpy(), ref, scale) < 1e-12
+
+
 @pytest.mark.parametrize("periodic", [True, False])
 @pytest.mark.parametrize("dims", [(8, 9, 10), (12, 33, 66), (66, 8, 129), (68, 127, 8), (130, 10, 255), (260, 12, 9),
                                   (9, 256, 17), (10, 17, 300)])
