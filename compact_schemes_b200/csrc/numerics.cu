@@ -418,12 +418,20 @@ k_deriv_wcol(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int
 // thread (l, c) holding chunk c of lines l and l + TL, so that addresses, solver
 // constants, table loads and barriers serve two lines (and a row of the tile is
 // 128 bytes).  Bound by its instructions and load latency (24 warps per SM): one
-// 256^3 field 78 us, 3.4 TB/s, against 80 us with one line per thread, 87 us with
+// 256^3 field 76 us, 3.5 TB/s, against 80 us with one line per thread, 87 us with
 // 16-line tiles, and 105 us staged through a transposing layout.
+//
+// A CTA also prefetches into L2, a row a thread, the tile `ahead` places on: a
+// prefetch holds no register and no load slot of the SM.  One 256^3 field 80 -> 76
+// us (distance 4: 78), the batched launches of the call sequence 358 -> 331 us along
+// y, 328 -> 296 us along z; with the sum over the axes in the store 774 -> 744 us
+// at distance 4 (32: 766).  Single precision, other chunk lengths and
+// the x rows do not gain (28.0 -> 28.3, 23.5 -> 24.4, 62.2 -> 64.3 us), nor do
+// fields that L2 can still hold; see deriv_ahead.
 template <int LT, int AXIS, int TL, typename T, bool SUM>
 __global__ void __launch_bounds__(TL * 32, LT <= 8 ? 768 / (TL * 32) : (LT == 16 ? 2 : 1))
 k_deriv_col(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int nend, int F, Coeffs cf,
-            DerivSum sum) {
+            DerivSum sum, int ahead) {
     using C = Column<LT, TL>;
     constexpr int NL = 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -439,6 +447,14 @@ k_deriv_col(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int 
         base[h] = (AXIS == 1 ? (fidx / lxi) * (lxi * let) + fidx % lxi : fidx) + j0 * s;
     }
     const T *in = fs.in + blockIdx.y * fs.in_fs;
+    if (LT == 8 && sizeof(T) == 8 && ahead) {
+        const int la = line0 + ahead * (NL * TL);
+        if (la < F) {
+            const T *p = in + (AXIS == 1 ? (la / lxi) * (lxi * let) + la % lxi : la);
+            for (int j = threadIdx.x; j < n; j += blockDim.x)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (int64_t)j * s));
+        }
+    }
     T d[NL][LT];
 #pragma unroll
     for (int t = 0; t < LT; ++t)
@@ -558,6 +574,13 @@ static int prep_smem(KernelT kern, size_t bytes) {
     return CS_OK;
 }
 
+// Distance, in tiles, of k_deriv_col's prefetch.  None below 96 MB of input: 126 MB
+// of L2 keep such a field, and what is already there is only asked for twice.
+static int deriv_ahead(const cs_dcomp &d, int nf, bool with_sum) {
+    if ((int64_t)nf * d.lmx * (int64_t)sizeof(double) < (int64_t)96 << 20) return 0;
+    return with_sum ? 4 : 32;
+}
+
 template <int LT, int AXIS, typename T>
 static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d, int nstart,
                            int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
@@ -609,7 +632,8 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
             }
             if (int rc = prep_smem(kern, smem)) return rc;
             kern<<<dim3((unsigned)((F + 2 * TL - 1) / (2 * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
-                fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, with_sum ? *sum : DerivSum{});
+                fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, with_sum ? *sum : DerivSum{},
+                deriv_ahead(d, nf, with_sum));
         }
     }
     CSB_CUDA(cudaGetLastError());

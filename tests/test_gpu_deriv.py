@@ -105,6 +105,29 @@ def test_deriv2d_recv_path_and_drva(cuda, dims):
                           drva[5 * F + m * F:5 * F + (m + 1) * F]) < TOL
 
 
+def test_deriv_with_tiles_fetched_ahead(cuda):
+    """A field too large for L2, whose y and z kernels fetch later tiles ahead:
+    bit for bit the derivative of slabs of it, which do not."""
+    import torch
+    import compact_schemes_b200 as cs
+    dims = (250, 245, 210)
+    nm = make(cuda, dims, [[45] * 3] * 2)
+    torch.manual_seed(3)
+    f = torch.randn(dims[::-1], dtype=torch.float64, device=cuda)
+    out = torch.empty_like(f)
+    for axis, part, slab in ((1, lambda t, i: t[10 * i:10 * i + 10], (250, 245, 10)),
+                             (2, lambda t, i: t[:, 35 * i:35 * i + 35], (250, 35, 210))):
+        nm.deriv1d(axis, f.reshape(-1), out.reshape(-1), 1, 1, nm.dcomp, 0, halo=cs.HALO_SELF)
+        small = make(cuda, slab, [[45] * 3] * 2)
+        for i in range(0, dims[3 - axis] // slab[3 - axis], 3):
+            g = part(f, i).contiguous()
+            want = torch.empty_like(g)
+            small.deriv1d(axis, g.reshape(-1), want.reshape(-1), 1, 1, small.dcomp, 0, halo=cs.HALO_SELF)
+            assert torch.equal(part(out, i), want), (axis, i)
+        small.close()
+    nm.close()
+
+
 @pytest.mark.parametrize("closure", [45, 10])
 @pytest.mark.parametrize("n", [8, 10, 12, 33, 34, 64, 66, 68, 127, 132, 255, 256, 260, 514, 1000, 1024])
 def test_deriv_row_and_column_lengths(cuda, n, closure):
