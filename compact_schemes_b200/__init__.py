@@ -74,6 +74,9 @@ def ptr(t):
 
 def stream_ptr(stream=None):
     import torch
+    if stream is None and torch.cuda.is_initialized():
+        # the current stream's handle without a Stream object (3.5 us a call)
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     s = stream if stream is not None else torch.cuda.current_stream()
     return ctypes.c_void_p(s.cuda_stream)
 
