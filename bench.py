@@ -37,11 +37,12 @@ UNIT = "Mpts*RK-stages/s"
 MACH, RE, CFL = 0.1, 1600.0, 0.5
 # Algorithmic bytes per grid point per launch of each pass (FP64, constant
 # metrics): gradient pass reads q (5) and writes 4 gradients; flux x reads q
-# and 12 gradients and writes R; flux y also reads R; flux z + RK reads q,
-# 12 gradients, R and q^n and writes q (stage 0: q^n is the stage input).
-ALG_BYTES = {"grad_x": 72, "grad_y": 72, "grad_z": 72, "flux_x": 176, "flux_y": 216,
-             "flux_z_rk": 8 * (5 + 12 + 5 + 5 + 5)}
-STAGE_BYTES = 864  # sum of the passes above per point per stage
+# and 8 gradients (a diagonal metric leaves out the other four) and writes R;
+# flux y also reads R; flux z + RK reads q, 8 gradients, R and q^n and writes q
+# (stage 0: q^n is the stage input).
+ALG_BYTES = {"grad_x": 72, "grad_y": 72, "grad_z": 72, "flux_x": 144, "flux_y": 184,
+             "flux_z_rk": 8 * (5 + 8 + 5 + 5 + 5)}
+STAGE_BYTES = sum(ALG_BYTES.values())  # of the passes above per point per stage
 
 
 def parse():
@@ -1013,7 +1014,7 @@ def run_ours(args):
                 "mixed_512_gcbc": mixed512, "ensemble": ensemble, "adjoint": adjoint,
                 "curvilinear": curvilinear, "reference_kernels": refk, "config1": cfg1, "dropin": dropin,
                 "filter": filt,
-                "gpu_launches": 24 * args.steps, "clocks": clocks,
+                "gpu_launches": sum(cnt for _, cnt in prof.values()), "clocks": clocks,
                 "passes": per_pass,
                 "stage_model": {"bytes_per_point": STAGE_BYTES, "ms_per_stage": stage_ms,
                                 "achieved_gbs": STAGE_BYTES * lmx / (stage_ms * 1e-3) / 1e9,
