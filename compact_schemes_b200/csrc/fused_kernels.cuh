@@ -1106,7 +1106,7 @@ FluxPrefetch flux_prefetch(const PassArgs &b, const RT *rhs, const double *qn, C
 // tile fills an SM by itself.  Not on per-point metrics, where rows or field blocks
 // are not 16-byte multiples, and for passes whose tiles all start together.
 // Measured at 256^3 (gradient y, z, flux x, y, z + RK with 16 lines): 0.387, 0.371,
-// 0.520, 0.731, 0.889 -> 0.327, 0.359, 0.495, 0.705, 0.834 ms, at 192^3 0.221,
+// 0.520, 0.731, 0.889 -> 0.327, 0.362, 0.493, 0.704, 0.823 ms, at 192^3 0.221,
 // 0.219, 0.266, 0.373, 0.459 -> 0.188, 0.192, 0.259, 0.356, 0.407 ms.  Two to eight
 // tiles ahead are alike, 48 make the flux passes 15-30 % slower, and fetching R and
 // q^n too costs more than it gives.  The z flux pass with 8 lines got slower with
@@ -1116,7 +1116,6 @@ template <int AXIS, int TL>
 Ahead pass_ahead(const PassArgs &b, int inputs, const double *q, const double *grad, AheadMaps &am) {
     Ahead ah{};
     const int lze = (int)(b.lmx / ((int64_t)b.lxi * b.let));
-    const cs_dcomp d{(int)b.lmx, b.lxi, b.let, lze};
     const int n = AXIS == 0 ? b.lxi : (AXIS == 1 ? b.let : lze);
     if (b.tab->lt != 8 || n > 256 || b.fm.xim || (b.F + TL - 1) / TL < 2 * (int64_t)b.nsm) return ah;
     if (b.lmx % 4 || (AXIS < 2 ? b.lxi % 4 : ((int64_t)b.lxi * b.let) % 4)) return ah;
@@ -1124,14 +1123,16 @@ Ahead pass_ahead(const PassArgs &b, int inputs, const double *q, const double *g
     ah.geo.nbox = 1;
     ah.geo.boxlen = (n + 3) / 4 * 4;
     ah.geo.lxi = b.lxi;
-    // gradients of the other axes on a diagonal metric: x reads u_y v_y | u_z (v_z) w_z, y u_x v_x | v_z w_z,
-    // z u_x (v_x) w_x | v_y w_y
-    constexpr int first[3][2] = {{4, 8}, {0, 9}, {0, 5}}, count[3][2] = {{2, 3}, {2, 2}, {3, 2}};
+    // gradients of the other axes on a diagonal metric: x reads u_y v_y | u_z w_z, y u_x v_x | v_z w_z,
+    // z u_x w_x | v_y w_y, one or two fields apart
+    constexpr int first[3][2] = {{4, 8}, {0, 9}, {0, 5}}, step[3][2] = {{1, 2}, {1, 1}, {2, 1}};
     const double *base[4] = {q, grad + 4 * AXIS * b.lmx, grad + first[AXIS][0] * b.lmx, grad + first[AXIS][1] * b.lmx};
-    const int nf[4] = {5, 4, count[AXIS][0], count[AXIS][1]};
-    for (int k = 0; k < 4; ++k)
+    const int nf[4] = {5, 4, 2, 2}, apart[4] = {1, 1, step[AXIS][0], step[AXIS][1]};
+    for (int k = 0; k < 4; ++k) {
+        const cs_dcomp d{apart[k] * (int)b.lmx, b.lxi, b.let, lze};  // lmx: the distance of the fields
         if (inputs >> k & 1)
-            if (tma_field_map_t(AXIS, d, TL, ah.geo.boxlen, nf[k], base[k], am.m[k])) return Ahead{};
+            if (tma_field_map(AXIS, d, TL, ah.geo.boxlen, nf[k], base[k], am.m[k])) return Ahead{};
+    }
     ah.maps = inputs;
     return ah;
 }
