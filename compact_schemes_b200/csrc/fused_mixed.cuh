@@ -476,7 +476,14 @@ k_flux_mx(const float *__restrict__ sh, const float *__restrict__ g, float *__re
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t line0 = (int64_t)blockIdx.x * TL;
     const PhysF pf = phys_f32(ph);
-    tile_for_each<AXIS, TL, CSB_MX_FLUX_UNROLL>(line0, F, n, lxi, let, [&](int l, int j, int64_t gi) {
+    // Points whose loads are in flight together: four where 128 registers a thread
+    // hold them, that is along x with the FP64 pointwise arithmetic (512-point lines
+    // 747 -> 723 us at 512x256x256, 256-point lines 405 -> 382 us at 256^3, 160-point
+    // lines 187 -> 182 us; 192-point lines, six points a thread, 168 -> 170 us) and
+    // along z in 16-line tiles with FP32 (1.43 -> 1.40 ms); the 80-register kernels
+    // spill with it.
+    constexpr int kPoints = (AXIS == 0 && !CF) || (AXIS == 2 && TL == 16 && CF) ? 4 : CSB_MX_FLUX_UNROLL;
+    tile_for_each<AXIS, TL, kPoints>(line0, F, n, lxi, let, [&](int l, int j, int64_t gi) {
         float fl[5];
         if (CF) point_flux_f32<AXIS, VISC>(sh, g, lmx, gi, pf, fl);
         else point_flux_mx<AXIS, VISC>(sh, g, lmx, gi, ph, fl);
@@ -525,7 +532,11 @@ k_flux_mx(const float *__restrict__ sh, const float *__restrict__ g, float *__re
             }
         });
     } else {
-        constexpr int P = MODE == kAccum ? (LT >= 16 ? 2 : CSB_RMW_CHUNK) : (LT >= 16 ? 1 : CSB_RMW_CHUNK_RK);
+        // One point at a time in the 16-line RK pass: R and q^n come from L2 by the
+        // prefetch above, and two points with the new shadow spill 68 bytes a thread
+        // (z at 512x256x256 1.40 -> 1.34 ms).
+        constexpr int P = MODE == kAccum ? (LT >= 16 ? 2 : CSB_RMW_CHUNK)
+                                         : (LT >= 16 || TL == 16 ? 1 : CSB_RMW_CHUNK_RK);
         float rv[P][5];
         double qv[P][5];
         tile_for_each_chunked<AXIS, TL, P>(
