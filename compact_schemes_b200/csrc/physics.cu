@@ -131,12 +131,16 @@ __global__ void k_visc_stress(double *__restrict__ de, double *__restrict__ tau,
     de[4 * n + i] = div;
 }
 
+// The larger of m and v, NaN if either is (fmax would drop it): a blown-up
+// state must show in the time step.
+__device__ __forceinline__ double nan_max(double m, double v) { return v > m || v != v ? v : m; }
+
 // calc_time_step_kernel (physics.hpp:335-427): two maxima, reduced per thread
 // over a grid-stride loop, then by warp shuffles and an integer atomic max on
-// the non-negative bit patterns.  A few atomics per block of a grid that fills
-// the chip once: one pair per warp of one point each (2 x 524288 at 256^3)
-// queued on two addresses for 1.45 ms; with 1184 blocks the 16 fields read take
-// 0.43 ms.
+// the non-negative bit patterns (those of a NaN lie above all others).  A few
+// atomics per block of a grid that fills the chip once: one pair per warp of one
+// point each (2 x 524288 at 256^3) queued on two addresses for 1.45 ms; with 1184
+// blocks the 16 fields read take 0.43 ms.
 constexpr int kTimeStepBlocks = 148 * 8;
 __global__ void k_time_step(const double *__restrict__ xim, const double *__restrict__ etm,
                             const double *__restrict__ zem, const double *__restrict__ de,
@@ -162,13 +166,13 @@ __global__ void k_time_step(const double *__restrict__ xim, const double *__rest
             rr2 += fabs(xmul(M[a][0], de[n + i] + u0) + xmul(M[a][1], de[2 * n + i] + u1) +
                         xmul(M[a][2], de[3 * n + i] + u2));
         const double ssi = fabs(yaco[i]);
-        m1 = fmax(m1, xmul(sqrt(xmul(de[4 * n + i], rr1)) + rr2, ssi));
-        m2 = fmax(m2, de[i] * ssk[i] * rr1 * ssi * ssi);
+        m1 = nan_max(m1, xmul(sqrt(xmul(de[4 * n + i], rr1)) + rr2, ssi));
+        m2 = nan_max(m2, de[i] * ssk[i] * rr1 * ssi * ssi);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-        m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+        m1 = nan_max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+        m2 = nan_max(m2, __shfl_xor_sync(0xffffffffu, m2, o));
     }
     if ((threadIdx.x & 31) == 0) {
         atomicMax(acc, (unsigned long long)__double_as_longlong(m1));
@@ -654,7 +658,7 @@ int cs_calc_time_step(cs_physics *ph, const double *xim, const double *etm, cons
     CSB_CUDA(cudaMemcpyAsync(h, ph->dt_acc, sizeof h, cudaMemcpyDeviceToHost, st));
     CSB_CUDA(cudaStreamSynchronize(st));
     const double a = cfl / h[0], b = 0.5 / h[1];
-    *dte = a < b ? a : b;
+    *dte = a < b || a != a ? a : b;  // NaN if either is
     return CS_OK;
 }
 

@@ -177,7 +177,7 @@ int cs_calc_viscous_shear_stress(cs_physics *ph, cs_numerics *nm, double *de, co
                                  const double *yaco, cs_dcomp d, void *stream);
 /* physics::calc_time_step (src/physics_pc.hpp:229-256): the CFL and viscous
  * maxima on the device, dte = min(cfl / max1, 0.5 / max2) on the host
- * (synchronizes the stream). */
+ * (synchronizes the stream).  A NaN in either quantity at any point makes dte NaN. */
 int cs_calc_time_step(cs_physics *ph, const double *xim, const double *etm, const double *zem,
                       const double *de, const double *yaco, const double *ssk, double cfl,
                       double *dte, size_t size, void *stream);

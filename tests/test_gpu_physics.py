@@ -317,3 +317,39 @@ def test_gcbc_apply_non_reflective_equals_numerics_path(cuda):
     c1, c2 = (d1 - dev(de)).cpu().numpy(), (d2 - dev(de)).cpu().numpy()
     assert np.abs(c1).max() > 0
     assert np.abs(c1 - c2).max() / np.abs(c1).max() < 1e-13
+
+
+def _time_step_fields(n, seed):
+    """Metrics, thermodynamic fields, Jacobian and viscosity of n points for calc_time_step."""
+    r = np.random.default_rng(seed)
+    xim, etm, zem = (0.1 * r.standard_normal((3, n)) for _ in range(3))
+    for a, m in enumerate((xim, etm, zem)):
+        m[a] += 1.0
+    de = np.concatenate([1 + 0.1 * r.random((1, n)), 0.2 * r.standard_normal((3, n)), 1 + 0.1 * r.random((1, n))])
+    return xim.ravel(), etm.ravel(), zem.ravel(), de, 1 + 0.1 * r.random(n), MU * (1 + r.random(n))
+
+
+def _device_time_step(xim, etm, zem, de, yaco, ssk, umf, cfl):
+    import compact_schemes_b200 as cs
+    n = yaco.size
+    ph = cs.physics((n, 1, 1), False)
+    ph.umf = umf
+    return ph.calc_time_step(dev(xim), dev(etm), dev(zem), dev(de), dev(yaco), dev(ssk), cfl, n)
+
+
+@pytest.mark.parametrize("n", [31, 1000, 400001])
+def test_time_step_of_a_state_with_nans_is_nan(cuda, n):
+    """A blown-up state shows in dt whether one point of it is NaN or all are, in the
+    acoustic maximum only (temperature), in the viscous one only (1 / rho) or in both."""
+    xim, etm, zem, de, yaco, ssk = _time_step_fields(n, 11)
+    umf = (0.02, -0.01, 0.0)
+    assert np.isfinite(_device_time_step(xim, etm, zem, de, yaco, ssk, umf, 0.5))
+    for point in (0, n // 2, n - 1, slice(None)):
+        for comp in (4, 0, 1, slice(None)):
+            bad = de.copy()
+            bad[comp, point] = np.nan
+            assert np.isnan(_device_time_step(xim, etm, zem, bad, yaco, ssk, umf, 0.5)), (point, comp)
+    bad = de.copy()
+    bad[4, n - 1] = -1.0  # sqrt of a negative temperature
+    assert np.isnan(_device_time_step(xim, etm, zem, bad, yaco, ssk, umf, 0.5))
+    assert np.isnan(_device_time_step(xim, etm, zem, np.full_like(de, -np.nan), yaco, ssk, umf, 0.5))
