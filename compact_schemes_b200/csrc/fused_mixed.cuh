@@ -462,6 +462,20 @@ __device__ __forceinline__ void point_flux_f32(const float *__restrict__ sh, con
     }
 }
 
+// Whether a flux pass loads four points of a line at a time instead of two (the
+// 80-register kernels spill with four).  Points past the last batch go one by one,
+// up to three of them after fours: fours pay where at most one whole row of 32
+// points is left (x flux of 4M points, two / four at a time: 112-point lines 164 /
+// 187 us, 64 171 / 185, 240 121 / 127, but 128 129 / 124, 160 152 / 146, 256 113 /
+// 108), along x on lines of more than 256 points with open faces only (512 points,
+// open 114 / 112, periodic 105 / 107), along z not on short lines (72 points 229 /
+// 245, 128 172 / 171, 256 182 / 170).
+template <int AXIS>
+__device__ __forceinline__ bool mx_load_four(int n, int nstart) {
+    if (n / 32 % 4 > 1) return false;
+    return AXIS == 0 ? n <= 256 || !nstart : n >= 128;
+}
+
 template <int LT, int AXIS, int TL, int MODE, bool VISC, bool SHADOW_OUT, bool REF, bool CF = false>
 __global__ void __launch_bounds__(TL * 32, TL == 8 ? (CF && !REF ? CSB_MX_FLUX_MINB : 2) : 1)
 k_flux_mx(const float *__restrict__ sh, const float *__restrict__ g, float *__restrict__ rhs,
@@ -476,21 +490,19 @@ k_flux_mx(const float *__restrict__ sh, const float *__restrict__ g, float *__re
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t line0 = (int64_t)blockIdx.x * TL;
     const PhysF pf = phys_f32(ph);
-    // Points whose loads are in flight together: four where 128 registers a thread
-    // hold them, that is along x with the FP64 pointwise arithmetic (512-point lines
-    // 747 -> 723 us at 512x256x256, 256-point lines 405 -> 382 us at 256^3, 160-point
-    // lines 187 -> 182 us; 192-point lines, six points a thread, 168 -> 170 us) and
-    // along z in 16-line tiles with FP32 (1.43 -> 1.40 ms); the 80-register kernels
-    // spill with it.
-    constexpr int kPoints = (AXIS == 0 && !CF) || (AXIS == 2 && TL == 16 && CF) ? 4 : CSB_MX_FLUX_UNROLL;
-    tile_for_each<AXIS, TL, kPoints>(line0, F, n, lxi, let, [&](int l, int j, int64_t gi) {
+    // Points whose loads are in flight together: two, or four where 128 registers a
+    // thread hold them and mx_load_four says that it pays.
+    auto load = [&](int l, int j, int64_t gi) {
         float fl[5];
         if (CF) point_flux_f32<AXIS, VISC>(sh, g, lmx, gi, pf, fl);
         else point_flux_mx<AXIS, VISC>(sh, g, lmx, gi, ph, fl);
         const int pj = L::pos(j);
 #pragma unroll
         for (int m = 0; m < 5; ++m) field_line32<LT, TL>(sm, m, l)[pj] = fl[m];
-    });
+    };
+    constexpr bool kFour = (AXIS == 0 && !CF) || (AXIS == 2 && TL == 16 && CF);
+    if (kFour && mx_load_four<AXIS>(n, nstart)) tile_for_each<AXIS, TL, 4>(line0, F, n, lxi, let, load);
+    else tile_for_each<AXIS, TL, CSB_MX_FLUX_UNROLL>(line0, F, n, lxi, let, load);
     // the RK store phase's R and q^n of this tile, fetched into L2 while the
     // tile is solved (measured at 256^3: flux z + RK 0.689 -> 0.639 ms; issued
     // before the load phase it competed with it and was slower, and the
