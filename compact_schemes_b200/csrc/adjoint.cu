@@ -78,10 +78,14 @@ static int lines_t(cs_adjoint *a, const LineSet &ls, int nf, const DevTables<dou
                     ls, tab, a->d.lxi, a->d.let, F, nstart, nend, a->cf, bcol);
         } else {
             constexpr int TL = 8;
-            const size_t smem = (size_t)2 * (Column<LT, TL>::kField + 16 * TL) * sizeof(double);
+            const size_t smem = (size_t)2 * (Column<LT, TL>::kField + 4 * TL) * sizeof(double);
             auto kern = k_lines_col<LT, AXIS, TL, TRANS>;
             if (int rc = set_smem(kern, smem)) return rc;
-            kern<<<dim3((unsigned)((F + 2 * TL - 1) / (2 * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
+            // Where not every SM gets a CTA, eight warps in each solve the reduced systems
+            // in one round, whatever the lines' chunks need (a 20^3 tangent step 308 -> 287 us).
+            const int64_t blocks = (F + 2 * TL - 1) / (2 * TL);
+            const int threads = blocks * nf < a->nsm ? TL * 32 : column_threads(TL, tab.p);
+            kern<<<dim3((unsigned)blocks, (unsigned)nf), threads, smem, st>>>(
                 ls, tab, a->d.lxi, a->d.let, F, nstart, nend, a->cf, bcol);
         }
     }

@@ -140,7 +140,7 @@ struct LineSet {
 // each lane loading its chunks with VB-byte vectors.  The transposed closure
 // columns are formed by 16 lanes and handed to the chunks that hold them.
 template <int LT, int NV, int VB, bool TRANS>
-__global__ void __launch_bounds__(256, LT <= 8 ? 3 : 1)
+__global__ void __launch_bounds__(256, TRANS && LT <= 4 ? 4 : (LT <= 8 ? 3 : 2))
 k_lines_row(LineSet ls, DevTables<double> tab, int F, int nstart, int nend, Coeffs cf, const double *__restrict__ bcol) {
     constexpr int VE = VB / 8;
     __shared__ double ends[8][NV][2 * kLmd + 1];
@@ -303,7 +303,7 @@ k_lines_col(LineSet ls, DevTables<double> tab, int lxi, int let, int F, int nsta
     using C = Column<LT, TL>;
     constexpr int NL = 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *V = reinterpret_cast<double *>(smem_raw), *rows = V + NL * C::kField;  // rows: [NL][TL][16]
+    double *V = reinterpret_cast<double *>(smem_raw), *rows = V + NL * C::kField;
     const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL, j0 = c * LT;
     const int len = lane_len(c, LT, tab.p, tab.last_len);
     const int line0 = (int)blockIdx.x * (NL * TL), s = AXIS == 1 ? lxi : lxi * let;
@@ -345,12 +345,6 @@ k_lines_col(LineSet ls, DevTables<double> tab, int lxi, int let, int F, int nsta
 #pragma unroll
         for (int h = 0; h < NL; ++h) column_put_raw<LT, TL, double>(V + h * C::kField, d[h], c, l, n);
         __syncthreads();
-        for (int i = threadIdx.x; i < NL * TL * 16; i += blockDim.x) {
-            const int ll = i % TL, h = i / TL % NL, k = i / (TL * NL);
-            const double *z = V + h * C::kField, *cw = bcol + 4 * k;
-            rows[(h * TL + ll) * 16 + k] = z[C::pos(0, ll)] * cw[0] + z[C::pos(1, ll)] * cw[1] +
-                                           z[C::pos(n - 2, ll)] * cw[2] + z[C::pos(n - 1, ll)] * cw[3];
-        }
         const int cm = c > 0 ? c - 1 : 0, cp = c < 31 ? c + 1 : 31;
 #pragma unroll
         for (int h = 0; h < NL; ++h) {
@@ -364,17 +358,24 @@ k_lines_col(LineSet ls, DevTables<double> tab, int lxi, int let, int F, int nsta
             for (int t = 0; t < LT; ++t) x[t + 2] = d[h][t];
             chunk_stencil_t<LT>(x, c, n, d[h]);
         }
-        __syncthreads();
+        // closure columns, by the threads that hold the eight points at either end
+        // (made by all threads and handed on through shared memory they cost a
+        // barrier: 56-point lines of 4M points, 5 fields 271 us, 48 points 266 us)
         if (j0 < kLmd || j0 + LT > n - kLmd) {
 #pragma unroll
-            for (int h = 0; h < NL; ++h)
+            for (int h = 0; h < NL; ++h) {
+                const double *z = V + h * C::kField;
+                const double z0 = z[C::pos(0, l)], z1 = z[C::pos(1, l)];
+                const double zm2 = z[C::pos(n - 2, l)], zm1 = z[C::pos(n - 1, l)];
 #pragma unroll
                 for (int t = 0; t < LT; ++t) {
-                    const int j = j0 + t;
-                    const double *e = rows + (h * TL + l) * 16;
-                    if (j < kLmd) d[h][t] += e[j];
-                    else if (t < len && j >= n - kLmd) d[h][t] += e[kLmd + n - 1 - j];
+                    const int j = j0 + t, k = j < kLmd ? j : kLmd + n - 1 - j;
+                    if (t < len && k < 2 * kLmd) {
+                        const double *cw = bcol + 4 * k;
+                        d[h][t] += z0 * cw[0] + z1 * cw[1] + zm2 * cw[2] + zm1 * cw[3];
+                    }
                 }
+            }
         }
     }
     double *out = ls.out + blockIdx.y * ls.out_fs;

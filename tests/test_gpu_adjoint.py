@@ -73,6 +73,32 @@ def test_line_operators_lengths(cuda, n, nbc_code):
 
 
 @pytest.mark.parametrize("nbc_code", ["periodic", "physical"])
+@pytest.mark.parametrize("n", [9, 20, 33, 56, 64, 66, 96, 128, 200, 300])
+def test_line_operators_of_few_and_many_fields(cuda, n, nbc_code):
+    """The launch shape of the y and z operators follows the fields of a call (CTAs of
+    eight warps while there are fewer CTAs than SMs, four lines a warp from half a
+    wave of lines on): every field of a call of many as a call of one, the same bits
+    where only the CTA changes, to rounding where the chunks do (65..128 points)."""
+    import compact_schemes_b200 as cs
+    b = cs.BC_PERIODIC if nbc_code == "periodic" else cs.BC_NON_REFLECTIVE
+    nf = 96  # 72 and 80 lines: 6912 and 7680 in all, either side of half a wave (7104)
+    g = torch.Generator(device="cuda:0").manual_seed(n)
+    for dims, axis in (((9, n, 8), 1), ((8, 9, n), 2), ((10, n, 8), 1), ((8, 10, n), 2)):
+        _, _, a, _ = _setup(dims, nbc=[[b] * 3] * 2)
+        m = int(np.prod(dims))
+        x = torch.randn(nf * m, dtype=torch.float64, device="cuda:0", generator=g)
+        for trans in (False, True):
+            many, one = torch.empty_like(x), torch.empty_like(x)
+            a.deriv(axis, x, many, nfields=nf, transpose=trans)
+            for f in range(nf):
+                a.deriv(axis, x[f * m:(f + 1) * m], one[f * m:(f + 1) * m], nfields=1, transpose=trans)
+            if n <= 64 or n > 128:
+                assert torch.equal(many, one), (dims, trans)
+            else:
+                assert float((many - one).abs().max()) <= 1e-13 * float(one.abs().max()), (dims, trans)
+
+
+@pytest.mark.parametrize("nbc_code", ["periodic", "physical"])
 @pytest.mark.parametrize("af", [0.0, 0.45, -0.3])
 def test_transposed_filter_dot_product_and_forward(cuda, nbc_code, af):
     import compact_schemes_b200 as cs
