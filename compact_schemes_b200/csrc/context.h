@@ -61,6 +61,7 @@ struct cs_numerics {
     int ndf[2][3]{};
     csb::Coeffs cf{};
     bool setup_done = false;
+    int nsm = 1;  // SMs of the device
     double *drva[3] = {nullptr, nullptr, nullptr};
     double *send[3] = {nullptr, nullptr, nullptr};
     double *recv[3] = {nullptr, nullptr, nullptr};

@@ -2,12 +2,14 @@
 // C-ABI (replaces src/numerics_base.hpp, src/numerics_pc.hpp,
 // src/numerics_rtc.hpp and src/cuda/kernels/numerics_*.hpp of the reference).
 //
-// Kernel shape: a CTA of 8 warps stages a tile of 8 lines in shared memory
-// (LineLayout order), each warp solves one line with the partitioned
-// warp-shuffle solver, and the tile is written back.  x lines are
-// contiguous, so each warp stages its own line with 256-byte coalesced
-// accesses; y and z lines are staged cooperatively as rows of 8 consecutive
-// lines (64-byte segments per row, full 32-byte sectors).
+// Derivatives: along x a warp solves one or two lines, each lane loading its own
+// chunks as vectors (k_deriv_row) or, for rows of any length and start and for
+// chunks too long for that, the warp staging its lines in shared memory with
+// 256-byte coalesced accesses (k_deriv_row_any).  Along y and z threads load their
+// chunks of a tile of neighbouring lines straight into registers (k_deriv_col,
+// column.cuh), or four lines share a warp (k_deriv_wcol).  blockIdx.y is the field.
+// The filter stages a tile of 8 lines in shared memory (LineLayout order), one warp
+// solving each line.
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -257,7 +259,7 @@ struct FieldSet {
 // registers.  Neighbouring points come by shuffle, and only the eight points
 // at either end of a line pass through shared memory (the interface sums).
 template <int LT, int NV, int VB, typename T>
-__global__ void __launch_bounds__(kThreads, LT <= 8 ? 3 : 1)
+__global__ void __launch_bounds__(kThreads, LT <= 8 ? 3 : (LT == 16 ? 2 : 1))
 k_deriv_row(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, Coeffs cf) {
     constexpr int VE = VB / (int)sizeof(T);
     __shared__ T ends[kThreads / 32][NV][2 * kLmd + 1];
@@ -313,7 +315,7 @@ k_deriv_row(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, C
 // shared memory (LineLayout) with 256-byte coalesced accesses and solves them
 // from there.
 template <int LT, int NV, typename T>
-__global__ void __launch_bounds__(kThreads, LT <= 8 ? 3 : 1)
+__global__ void __launch_bounds__(kThreads, LT <= 8 ? 3 : (LT == 16 || sizeof(T) == 4 ? 2 : 1))
 k_deriv_row_any(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t F, Coeffs cf) {
     using L = LineLayout<LT>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -324,8 +326,11 @@ k_deriv_row_any(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t 
     const T *in = fs.in + blockIdx.y * fs.in_fs + line0 * n;
     T *out = fs.out + blockIdx.y * fs.out_fs + line0 * n;
     const int nl = F - line0 < NV ? (int)(F - line0) : NV;
-    for (int h = 0; h < nl; ++h)
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        if (h >= nl) break;
         for (int j = lane; j < n; j += 32) sm[h * L::kSlot + L::pos(j)] = in[(int64_t)h * n + j];
+    }
     __syncwarp();
     T d[NV][LT];
 #pragma unroll
@@ -357,8 +362,11 @@ k_deriv_row_any(FieldSet<T> fs, DevTables<T> tab, int nstart, int nend, int64_t 
         store_line_regs<LT, T>(sm + h * L::kSlot, d[h], lane, n);
     }
     __syncwarp();
-    for (int h = 0; h < nl; ++h)
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+        if (h >= nl) break;
         for (int j = lane; j < n; j += 32) out[(int64_t)h * n + j] = sm[h * L::kSlot + L::pos(j)];
+    }
 }
 
 // The same along y and z for the lines of warp_column (column.cuh): four lines
@@ -428,17 +436,16 @@ k_deriv_wcol(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int
 // at distance 4 (32: 766).  Single precision, other chunk lengths and
 // the x rows do not gain (28.0 -> 28.3, 23.5 -> 24.4, 62.2 -> 64.3 us), nor do
 // fields that L2 can still hold; see deriv_ahead.
-template <int LT, int AXIS, int TL, typename T, bool SUM>
-__global__ void __launch_bounds__(TL * 32, LT <= 8 ? 768 / (TL * 32) : (LT == 16 ? 2 : 1))
+template <int LT, int AXIS, int TL, int NL, typename T, bool SUM>
+__global__ void __launch_bounds__(TL * 32, LT <= 8 ? 768 / (TL * 32) : 2)
 k_deriv_col(FieldSet<T> fs, DevTables<T> tab, int lxi, int let, int nstart, int nend, int F, Coeffs cf,
             DerivSum sum, int ahead) {
     using C = Column<LT, TL>;
-    constexpr int NL = 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *V = reinterpret_cast<T *>(smem_raw), *rows = V + NL * C::kField;
     const int n = tab.n, l = threadIdx.x % TL, c = threadIdx.x / TL, j0 = c * LT;
     const int len = lane_len(c, LT, tab.p, tab.last_len);
-    const int line0 = (int)blockIdx.x * (NL * TL) , s = AXIS == 1 ? lxi : lxi * let;
+    const int line0 = (int)blockIdx.x * (NL * TL), s = AXIS == 1 ? lxi : lxi * let;
     int base[NL];
 #pragma unroll
     for (int h = 0; h < NL; ++h) {
@@ -581,16 +588,41 @@ static int deriv_ahead(const cs_dcomp &d, int nf, bool with_sum) {
     return with_sum ? 4 : 32;
 }
 
+// y and z lines in column tiles (k_deriv_col) of NL groups of eight lines.
+template <int LT, int AXIS, int NL, typename T>
+static int launch_deriv_col(const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d, int nstart,
+                            int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
+    constexpr int TL = 8;
+    const int64_t F = face_size(d, AXIS);
+    const size_t smem = (size_t)NL * (Column<LT, TL>::kField + 4 * TL) * sizeof(T);
+    auto kern = k_deriv_col<LT, AXIS, TL, NL, T, false>;
+    if constexpr (AXIS == 2 && sizeof(T) == 8) {
+        if (sum) kern = k_deriv_col<LT, AXIS, TL, NL, T, true>;
+    }
+    if (int rc = prep_smem(kern, smem)) return rc;
+    kern<<<dim3((unsigned)((F + NL * TL - 1) / (NL * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
+        fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, sum ? *sum : DerivSum{}, deriv_ahead(d, nf, sum != nullptr));
+    CSB_CUDA(cudaGetLastError());
+    return CS_OK;
+}
+
 template <int LT, int AXIS, typename T>
 static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d, int nstart,
-                           int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
+                           int nend, const Coeffs &cf, const DerivSum *sum, int nsm, cudaStream_t st) {
     const int64_t F = face_size(d, AXIS);
     if constexpr (AXIS == 0) {
         constexpr int NV = LT <= 8 ? 2 : 1, WARPS = kThreads / 32;
+        // A lane's chunk of more than 64 bytes spreads each of its vector loads over
+        // 4 KB and more.  With 128 bytes (FP64, lines of 257..512 points) that still
+        // pays for the table-driven solve (400x96x96, physical closure 31 -> 25 us;
+        // staged 33), not for the faster interior one (512x88x88, interface closure
+        // 24.6 against 22.6 us staged), and not on lines of more than 512 points
+        // (1024x64x64: FP64 28.7 against 26.7, FP32 18.5 against 14.4 us).
+        const bool vectors = LT * sizeof(T) <= 64 || (LT == 16 && !tab.interior);
         const dim3 grid((unsigned)((F + NV * WARPS - 1) / (NV * WARPS)), (unsigned)nf);
         auto aligned = [&](int vb) {
             const int64_t ve = vb / (int)sizeof(T);
-            return LT % ve == 0 && d.lxi % ve == 0 && (nf == 1 || (fs.in_fs % ve == 0 && fs.out_fs % ve == 0)) &&
+            return vectors && LT % ve == 0 && d.lxi % ve == 0 && (nf == 1 || (fs.in_fs % ve == 0 && fs.out_fs % ve == 0)) &&
                    reinterpret_cast<uintptr_t>(fs.in) % vb == 0 && reinterpret_cast<uintptr_t>(fs.out) % vb == 0;
         };
         if constexpr (LT * sizeof(T) >= 32) {
@@ -624,16 +656,13 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
                     fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, with_sum ? *sum : DerivSum{});
             }
         } else {
-            constexpr int TL = 8;
-            const size_t smem = (size_t)2 * (Column<LT, TL>::kField + 4 * TL) * sizeof(T);
-            auto kern = k_deriv_col<LT, AXIS, TL, T, false>;
-            if constexpr (AXIS == 2 && sizeof(T) == 8) {
-                if (with_sum) kern = k_deriv_col<LT, AXIS, TL, T, true>;
-            }
-            if (int rc = prep_smem(kern, smem)) return rc;
-            kern<<<dim3((unsigned)((F + 2 * TL - 1) / (2 * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
-                fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, with_sum ? *sum : DerivSum{},
-                deriv_ahead(d, nf, with_sum));
+            // Two lines a thread, but one of 32 rows (two take 147 KB and an SM for
+            // themselves: FP64 72x700x72 39 -> 29 us along y), and one of 16 where two
+            // would not give every SM a CTA (16x400x16 7.5 -> 5.3 us).
+            const DerivSum *s = with_sum ? sum : nullptr;
+            if (LT == 16 && (F + 15) / 16 * nf < nsm)
+                return launch_deriv_col<LT, AXIS, LT >= 16 ? 1 : 2, T>(fs, nf, tab, d, nstart, nend, cf, s, st);
+            return launch_deriv_col<LT, AXIS, LT == 32 ? 1 : 2, T>(fs, nf, tab, d, nstart, nend, cf, s, st);
         }
     }
     CSB_CUDA(cudaGetLastError());
@@ -642,13 +671,14 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
 
 template <int AXIS, typename T>
 static int launch_deriv_axis(int lt, const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d,
-                             int nstart, int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
+                             int nstart, int nend, const Coeffs &cf, const DerivSum *sum, int nsm,
+                             cudaStream_t st) {
     switch (lt) {
-        case 2: return launch_deriv_lt<2, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
-        case 4: return launch_deriv_lt<4, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
-        case 8: return launch_deriv_lt<8, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
-        case 16: return launch_deriv_lt<16, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
-        case 32: return launch_deriv_lt<32, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, st);
+        case 2: return launch_deriv_lt<2, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, nsm, st);
+        case 4: return launch_deriv_lt<4, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, nsm, st);
+        case 8: return launch_deriv_lt<8, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, nsm, st);
+        case 16: return launch_deriv_lt<16, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, nsm, st);
+        case 32: return launch_deriv_lt<32, AXIS, T>(fs, nf, tab, d, nstart, nend, cf, sum, nsm, st);
     }
     return set_error(CS_ERR_UNSUPPORTED, "chunk length %d", lt);
 }
@@ -707,10 +737,10 @@ static int deriv_launch(cs_numerics *nm, int axis, const T *in, int64_t in_fs, T
                         unsigned var, int nstart, int nend, int halo, const DerivSum *sum, cudaStream_t st) {
     const cs_dcomp &d = nm->d;
     const int n = line_len(d, axis);
+    const int64_t F = face_size(d, axis);
     if ((nstart || nend) && n < kLmd) return set_error(CS_ERR_UNSUPPORTED, "interface closure needs n >= 8");
     const DeviceTables *dt = nm->tables.get(n, kDeriv, nstart, nend, 0.0, deriv_chunk(axis, n));
     if (!dt) return CS_ERR_UNSUPPORTED;
-    const int64_t F = face_size(d, axis);
     FieldSet<T> fs{in, out, nullptr, nullptr, in_fs, out_fs};
     if (sizeof(T) == sizeof(double)) {
         if (halo == CS_HALO_RECV) fs.recv = reinterpret_cast<const T *>(nm->recv[axis] + (int64_t)var * 4 * F);
@@ -720,9 +750,9 @@ static int deriv_launch(cs_numerics *nm, int axis, const T *in, int64_t in_fs, T
     }
     const DevTables<T> &tab = pick_tables<T>(*dt);
     switch (axis) {
-        case 0: return launch_deriv_axis<0, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, nullptr, st);
-        case 1: return launch_deriv_axis<1, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, nullptr, st);
-        default: return launch_deriv_axis<2, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, sum, st);
+        case 0: return launch_deriv_axis<0, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, nullptr, nm->nsm, st);
+        case 1: return launch_deriv_axis<1, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, nullptr, nm->nsm, st);
+        default: return launch_deriv_axis<2, T>(dt->lt, fs, nf, tab, d, nstart, nend, nm->cf, sum, nm->nsm, st);
     }
 }
 
@@ -839,6 +869,9 @@ int cs_numerics_create(cs_numerics **out, cs_dcomp d, const int nbc[2][3]) {
     if (int rc = check_dims(d)) return rc;
     auto *nm = new cs_numerics();
     nm->d = d;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&nm->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) nm->nsm = 1;
     for (int f = 0; f < 2; ++f)
         for (int a = 0; a < 3; ++a) {
             const int b = nbc[f][a];
