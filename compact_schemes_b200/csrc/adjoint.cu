@@ -28,9 +28,10 @@ struct cs_adjoint {
     int nsm = 1;
     csb::TableCache tables;
     const csb::DeviceTables *tab[3] = {nullptr, nullptr, nullptr};
-    // tables of the line operators D and D^T (the gradient passes use tab)
-    const csb::DeviceTables *ltab[3] = {nullptr, nullptr, nullptr};
     const csb::DeviceTables *tabT[3] = {nullptr, nullptr, nullptr};
+    // the same for the line operators with four lines a warp (null where it does not apply)
+    const csb::DeviceTables *wtab[3] = {nullptr, nullptr, nullptr};
+    const csb::DeviceTables *wtabT[3] = {nullptr, nullptr, nullptr};
     csb::Coeffs cf{};
     csb::Phys ph{};
     csb::AdjPoint ap{};
@@ -102,7 +103,9 @@ static int lines_ax(cs_adjoint *a, int axis, const LineSet &ls, int nf, const De
 
 static int lines(cs_adjoint *a, int axis, bool trans, const double *in, int64_t in_fs, double *out, int64_t out_fs,
                  int nf, bool accum, cudaStream_t st) {
-    const DeviceTables *t = trans ? a->tabT[axis] : a->ltab[axis];
+    const DeviceTables *t = trans ? a->tabT[axis] : a->tab[axis];
+    if (a->wtab[axis] && warp_column_pays(t->t64.n, a->ndf[0][axis], a->ndf[1][axis], nf * a->F[axis], a->nsm, 8))
+        t = trans ? a->wtabT[axis] : a->wtab[axis];
     const LineSet ls{in, out, in_fs, out_fs, accum ? 1 : 0};
     switch (t->lt) {
         case 2: return trans ? lines_ax<2, true>(a, axis, ls, nf, t->t64, st) : lines_ax<2, false>(a, axis, ls, nf, t->t64, st);
@@ -310,10 +313,13 @@ int cs_adjoint_create(cs_adjoint **out, const cs_solver_config *cfg) {
         if (n[ax] == 1) continue;
         if (n[ax] > 512) { cs_adjoint_destroy(a); return set_error(CS_ERR_UNSUPPORTED, "adjoint: lines of at most 512 points"); }
         a->tab[ax] = a->tables.get(n[ax], kDeriv, a->ndf[0][ax], a->ndf[1][ax], 0.0);
-        const int min_lt = ax > 0 && warp_column(n[ax]) ? kWarpChunk : 2;
-        a->ltab[ax] = a->tables.get(n[ax], kDeriv, a->ndf[0][ax], a->ndf[1][ax], 0.0, min_lt);
-        a->tabT[ax] = a->tables.get(n[ax], kDerivT, a->ndf[0][ax], a->ndf[1][ax], 0.0, min_lt);
-        if (!a->tab[ax] || !a->ltab[ax] || !a->tabT[ax]) { cs_adjoint_destroy(a); return CS_ERR_UNSUPPORTED; }
+        a->tabT[ax] = a->tables.get(n[ax], kDerivT, a->ndf[0][ax], a->ndf[1][ax], 0.0);
+        if (!a->tab[ax] || !a->tabT[ax]) { cs_adjoint_destroy(a); return CS_ERR_UNSUPPORTED; }
+        if (ax > 0 && warp_column(n[ax])) {
+            a->wtab[ax] = a->tables.get(n[ax], kDeriv, a->ndf[0][ax], a->ndf[1][ax], 0.0, kWarpChunk);
+            a->wtabT[ax] = a->tables.get(n[ax], kDerivT, a->ndf[0][ax], a->ndf[1][ax], 0.0, kWarpChunk);
+            if (!a->wtab[ax] || !a->wtabT[ax]) { cs_adjoint_destroy(a); return CS_ERR_UNSUPPORTED; }
+        }
         a->active[ax] = 1;
         a->amask |= 1 << ax;
     }

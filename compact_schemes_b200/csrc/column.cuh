@@ -162,11 +162,29 @@ __device__ __forceinline__ void column_finish(const T *V, const DevTables<T> &ta
 // ----------------------------------------------------------------------------
 constexpr int kWarpLines = 4;
 constexpr int kWarpChunk = 16;
-// Measured on B200 (transposed derivative, 4.5 fields of 128^3): 53 us against
-// 72 us for the column tiles.  Shorter lines leave too few rows per lane to pay
-// for its serial sweeps (64^3: 5.8 us against 4.9 us), longer ones need 32-row
-// chunks, whose registers allow only 16 warps per SM (256^3: 83 against 78 us).
+// Lines that fit it: shorter ones leave too few rows per lane to pay for its
+// serial sweeps (64^3: 5.8 us against 4.9 us), longer ones need 32-row chunks, whose
+// registers allow only 16 warps per SM (256^3: 83 against 78 us).
 __host__ __device__ constexpr bool warp_column(int n) { return n > 64 && n <= 8 * kWarpChunk; }
+// ... and whether a launch of `lines` lines of them is faster with it than with the
+// column tiles below (two lines a thread, chunks of 4 rows).  The lane's serial
+// sweeps take 8 us where the tiles take 5, so it needs half a wave of lines (96 an
+// SM: three CTAs of 32) to be busy with.  With the table-driven factors a second
+// wave costs as much as the first and pays again once it is full; the interior
+// factors (interface closure, full chunks) leave room for it.  FP64 derivatives of
+// one field of 72- to 128-point lines, us, column tiles / four lines a warp:
+//   lines            2304     6400       9216      16384      35000  166464
+//   interior      5.2/5.9  6.3/6.7   11.7/7.4  15.5/13.4  32.2/21.0  116/83
+//   table-driven  5.4/8.9  6.3/9.6  11.8/10.0  16.6/17.6  28.0/28.3 120/113
+// Single precision gains only from the interior factors on large fields (112-point
+// lines: 36864 lines 18.9 / 17.1, 18496 lines 10.3 / 11.5 us).
+inline bool warp_column_pays(int n, int nstart, int nend, int64_t lines, int nsm, int bytes) {
+    const bool interior = nstart && nend && n % kWarpChunk == 0;
+    const int64_t wave = (int64_t)96 * nsm;
+    if (!warp_column(n)) return false;
+    if (bytes == 4) return interior && lines > 2 * wave;
+    return 2 * lines >= wave && (interior || lines <= wave || lines > 2 * wave);
+}
 
 // Right-hand side of a lane's chunk from its field values d; ends: this warp's
 // [4][17] end points in shared memory; far: the received far-end sum that this

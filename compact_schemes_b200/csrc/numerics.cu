@@ -727,9 +727,6 @@ const DevTables<double> &pick_tables<double>(const DeviceTables &dt) { return dt
 template <>
 const DevTables<float> &pick_tables<float>(const DeviceTables &dt) { return dt.t32; }
 
-// Shortest chunk of the tables of a derivative along `axis`.
-static int deriv_chunk(int axis, int n) { return axis > 0 && warp_column(n) ? kWarpChunk : 2; }
-
 // nf derivatives along `axis` in one launch: field f is in + f in_fs -> out +
 // f out_fs, with the numerics object's interface buffers of variable var + f.
 template <typename T>
@@ -739,7 +736,8 @@ static int deriv_launch(cs_numerics *nm, int axis, const T *in, int64_t in_fs, T
     const int n = line_len(d, axis);
     const int64_t F = face_size(d, axis);
     if ((nstart || nend) && n < kLmd) return set_error(CS_ERR_UNSUPPORTED, "interface closure needs n >= 8");
-    const DeviceTables *dt = nm->tables.get(n, kDeriv, nstart, nend, 0.0, deriv_chunk(axis, n));
+    const bool wcol = axis > 0 && warp_column_pays(n, nstart, nend, nf * F, nm->nsm, (int)sizeof(T));
+    const DeviceTables *dt = nm->tables.get(n, kDeriv, nstart, nend, 0.0, wcol ? kWarpChunk : 2);
     if (!dt) return CS_ERR_UNSUPPORTED;
     FieldSet<T> fs{in, out, nullptr, nullptr, in_fs, out_fs};
     if (sizeof(T) == sizeof(double)) {
@@ -918,7 +916,15 @@ int cs_deriv_setup(cs_numerics *nm) {
     for (int a = 0; a < 3; ++a) {
         const int n = line_len(nm->d, a);
         if (n < 5) continue;  // degenerate axis: derivative along it is rejected at call time
-        if (!nm->tables.get(n, kDeriv, nm->ndf[0][a], nm->ndf[1][a], 0.0, deriv_chunk(a, n))) return CS_ERR_UNSUPPORTED;
+        // the tables of every form that this object's launches (1, 4 or 5 fields) take
+        const int64_t F = face_size(nm->d, a);
+        bool use[2] = {false, false};  // four lines a warp: no, yes
+        for (int nf : {1, 4, 5})
+            for (int bytes : {8, 4})
+                use[a > 0 && warp_column_pays(n, nm->ndf[0][a], nm->ndf[1][a], nf * F, nm->nsm, bytes)] = true;
+        for (int w = 0; w < 2; ++w)
+            if (use[w] && !nm->tables.get(n, kDeriv, nm->ndf[0][a], nm->ndf[1][a], 0.0, w ? kWarpChunk : 2))
+                return CS_ERR_UNSUPPORTED;
     }
     nm->setup_done = true;
     return CS_OK;

@@ -158,6 +158,32 @@ def test_deriv_row_and_column_lengths(cuda, n, closure):
 
 
 @pytest.mark.parametrize("closure", [45, 10])
+@pytest.mark.parametrize("dims", [(120, 72, 60), (90, 80, 80), (172, 72, 84), (172, 96, 84), (172, 168, 72),
+                                  (172, 168, 128), (60, 300, 39), (60, 300, 42), (60, 39, 300), (60, 42, 300),
+                                  (300, 8, 300), (320, 300, 8)])
+def test_deriv_forms_by_number_of_lines(cuda, dims, closure):
+    """Fields on both sides of the numbers of lines at which the y and z kernels change
+    (65..128 points: column tiles, four lines a warp from 7104 lines on, not between
+    one and two waves of 14208 with the table-driven factors; 257..512 points: one
+    line a thread below 2368) and x lines of 257..512 points with either kind of
+    factors: against the oracle, FP32 within 2e-6."""
+    import torch
+    import compact_schemes_b200 as cs
+    nd = int(closure == 45)
+    coeffs = O.deriv_setup()
+    nm = make(cuda, dims, [[closure] * 3] * 2)
+    f = field(dims, 5)
+    f32 = torch.from_numpy(f).to(cuda).float()
+    for axis in range(3):
+        for x, tol in ((torch.from_numpy(f).to(cuda), TOL), (f32, 2e-6)):
+            out = torch.empty_like(x)
+            nm.deriv1d(axis, x, out, nd, nd, nm.dcomp, 0, halo=cs.HALO_SELF)
+            want = O.deriv(x.double().cpu().numpy(), dims, axis, nd, nd, coeffs=coeffs)
+            assert relerr(out.double().cpu().numpy(), want) < tol, (axis, x.dtype)
+    nm.close()
+
+
+@pytest.mark.parametrize("closure", [45, 10])
 @pytest.mark.parametrize("n", [7, 9, 16, 33, 34, 64, 66, 127, 132, 256, 260, 511, 1000])
 def test_filter_lengths(cuda, n, closure):
     """The filter at lengths around the chunk, tile and vector-access edges,
