@@ -538,6 +538,13 @@ static PointPhys point_phys(const double M[9], double J, double mu, const double
     return p;
 }
 
+static bool is_diagonal(const PointPhys &p) {
+    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < 3; ++k)
+            if (a != k && p.M[a][k] != 0.0) return false;
+    return true;
+}
+
 int cs_point_flux(int axis, int viscous, const double q[5], const double G[12], const double M[9], double J,
                   double mu, const double umf[3], double F[5]) {
     if (axis < 0 || axis > 2 || !q || !G || !M || !umf || !F) return set_error(CS_ERR_INVALID, "bad argument");
@@ -547,11 +554,16 @@ int cs_point_flux(int axis, int viscous, const double q[5], const double G[12], 
     return CS_OK;
 }
 
+// Where M is diagonal the linearizations take the form that the kernels run on
+// the uniform grid (DIAG).
 int cs_point_flux_jvp(int axis, int viscous, const double q[5], const double G[12], const double dq[5],
                       const double dG[12], const double M[9], double J, double mu, const double umf[3], double dF[5]) {
     if (axis < 0 || axis > 2 || !q || !G || !dq || !dG || !M || !umf || !dF) return set_error(CS_ERR_INVALID, "bad argument");
     const PointPhys p = point_phys(M, J, mu, umf);
-    if (viscous) flux_tan<true>(axis, q, G, dq, dG, p, dF);
+    const bool diag = is_diagonal(p);
+    if (viscous && diag) flux_tan<true, true>(axis, q, G, dq, dG, p, dF);
+    else if (viscous) flux_tan<true>(axis, q, G, dq, dG, p, dF);
+    else if (diag) flux_tan<false, true>(axis, q, G, dq, dG, p, dF);
     else flux_tan<false>(axis, q, G, dq, dG, p, dF);
     return CS_OK;
 }
@@ -563,7 +575,10 @@ int cs_point_flux_vjp(int axis, int viscous, const double q[5], const double G[1
     const PointPhys p = point_phys(M, J, mu, umf);
     for (int m = 0; m < 5; ++m) qbar[m] = 0.0;
     for (int k = 0; k < 12; ++k) Gbar[k] = 0.0;
-    if (viscous) flux_adj<true>(axis, q, G, Fbar, p, qbar, Gbar);
+    const bool diag = is_diagonal(p);
+    if (viscous && diag) flux_adj<true, true>(axis, q, G, Fbar, p, qbar, Gbar);
+    else if (viscous) flux_adj<true>(axis, q, G, Fbar, p, qbar, Gbar);
+    else if (diag) flux_adj<false, true>(axis, q, G, Fbar, p, qbar, Gbar);
     else flux_adj<false>(axis, q, G, Fbar, p, qbar, Gbar);
     return CS_OK;
 }

@@ -60,3 +60,37 @@ def test_primitive_linearizations(seed):
     pb = r.standard_normal(4)
     qb = np.array(A.point_prim_vjp(q, pb))
     assert abs(pb @ t - qb @ dq) <= 1e-13 * (abs(pb) @ abs(t))
+
+
+# The kernels run on the uniform grid, whose metric matrix is diagonal, in the form
+# that leaves the zero entries out; the point functions take it where M is diagonal.
+def _diagonal(M):
+    return np.diag(np.diag(M.reshape(3, 3))).ravel()
+
+
+@pytest.mark.parametrize("viscous", [True, False])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("seed", [5, 6])
+def test_flux_linearizations_on_a_diagonal_metric(viscous, axis, seed):
+    """Tangent against central differences, adjoint against the tangent, and both
+    against the general form (which an off-diagonal entry of 1e-300 selects; it
+    changes no sum, so the two differ by the order of their sums only)."""
+    r, q, G, M, J, mu, umf = _case(seed)
+    M = _diagonal(M)
+    general = M.copy()
+    general[1] = 1e-300
+    dq = r.standard_normal(5) * np.array([0.1, 0.1, 0.1, 0.1, 0.3])
+    dG, fb = r.standard_normal(12), r.standard_normal(5)
+    eps = 1e-6
+    fp = np.array(A.point_flux(axis, viscous, q + eps * dq, G + eps * dG, M, J, mu, umf))
+    fm = np.array(A.point_flux(axis, viscous, q - eps * dq, G - eps * dG, M, J, mu, umf))
+    fd = (fp - fm) / (2 * eps)
+    t = np.array(A.point_flux_jvp(axis, viscous, q, G, dq, dG, M, J, mu, umf))
+    assert np.abs(t - fd).max() <= 1e-7 * np.abs(fd).max()
+    tg = np.array(A.point_flux_jvp(axis, viscous, q, G, dq, dG, general, J, mu, umf))
+    assert np.abs(t - tg).max() <= 1e-13 * np.abs(tg).max()
+    qb, gb = (np.array(x) for x in A.point_flux_vjp(axis, viscous, q, G, fb, M, J, mu, umf))
+    assert abs(fb @ t - (qb @ dq + gb @ dG)) <= 1e-13 * (abs(fb) @ abs(t))
+    qg, gg = (np.array(x) for x in A.point_flux_vjp(axis, viscous, q, G, fb, general, J, mu, umf))
+    assert np.abs(qb - qg).max() <= 1e-13 * np.abs(qg).max()
+    assert np.abs(gb - gg).max() <= 1e-13 * max(np.abs(gg).max(), 1e-300)
