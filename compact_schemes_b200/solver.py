@@ -106,7 +106,8 @@ class Solver:
         check(lib().cs_solver_profile_begin(self._h))
 
     def profile_end(self):
-        """{pass name: (total ms, launches)} since profile_begin (synchronizes)."""
+        """{pass name: (total ms, launches)} since profile_begin (synchronizes).
+        A stage's x gradient and flux in one launch count as flux_x."""
         ms = (ctypes.c_double * len(self.PASS_NAMES))()
         n = (ctypes.c_int * len(self.PASS_NAMES))()
         check(lib().cs_solver_profile_end(self._h, ms, n))
@@ -120,7 +121,8 @@ class Solver:
 
     def schedule(self):
         """Current schedule per pass: {(kind, axis): 8 | 16 (one-phase tile
-        lines) | 0 (pipelined) | 1 (TMA-staged gradient pass)}."""
+        lines) | 0 (pipelined) | 1 (TMA-staged gradient pass)}.  The one-phase
+        x passes may run as one launch: then profile_end has no grad_x."""
         ch = (ctypes.c_int * 3 * 2)()
         check(lib().cs_solver_schedule(self._h, ctypes.byref(ch)))
         return {(k, a): ch[k][a] for k in range(2) for a in range(3)}

@@ -335,14 +335,23 @@ int cs_solver_dt_device(cs_solver *s, double **dt_dev);
  * profiled): between begin and end every pass is bracketed by CUDA events on
  * its stream; end synchronizes and returns the summed milliseconds and launch
  * counts per pass kind: 0-2 gradient x/y/z, 3-5 flux x/y/z (z carries the RK
- * update), 6 GCBC, 7 filter (one launch per axis). */
+ * update), 6 GCBC, 7 filter (one launch per axis).  Stages whose x gradient and
+ * flux run as one launch (cs_solver_autotune) count it as flux x and have no
+ * gradient x launch. */
 #define CS_PASS_KINDS 8
 /* Autotuner: times `reps` eager steps of every feasible pass schedule (one-
- * phase with 8- or 16-line tiles, pipelined) on a scratch copy of q (q is not
+ * phase with 8- or 16-line tiles, pipelined, TMA-staged gradient passes, and the
+ * one-phase x gradient and flux as one launch) on a scratch copy of q (q is not
  * modified) and keeps the fastest per pass; choice[kind][axis] (may be NULL)
  * receives 8 or 16 (one-phase tile lines), 0 (pipelined) or 1 (TMA-staged,
  * gradient passes) for the gradient (kind 0) and flux (kind 1) passes.
- * Synchronizes. */
+ * Synchronizes.
+ * The one launch applies to the viscous FP64 right-hand side on the uniform grid
+ * with at least two active axes, x lines of up to 128 points whose rows, fields
+ * and arrays start on multiples of a chunk (2 points up to 64, else 4), and
+ * one-phase x passes; there it also runs without the autotuner.  Both x choices
+ * are then 8, its results are those of the two launches bit for bit, and
+ * cs_solver_profile_end shows whether it ran. */
 int cs_solver_autotune(cs_solver *s, const double *q, int reps, int choice[2][3], void *stream);
 /* The schedule each pass runs now, coded as cs_solver_autotune's choice. */
 int cs_solver_schedule(const cs_solver *s, int choice[2][3]);

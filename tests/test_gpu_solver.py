@@ -440,3 +440,32 @@ def test_filter_config_rejected_where_unsupported(cuda):
         solver((32, 24, 20), filter=FILTER_STAGE, precision=1)
     with pytest.raises(cs.CSError):
         cs.Adjoint(cs.tgv_config(None, dims=(32, 24, 20), filter=FILTER_STEP))
+
+
+@pytest.mark.parametrize("dims", [(12, 10, 9), (64, 9, 8), (68, 9, 8), (128, 10, 12), (36, 20, 1)])
+@pytest.mark.parametrize("open_x", [False, True])
+def test_merged_x_passes_equal_the_separate_ones(cuda, dims, open_x):
+    """The x gradient and flux in one launch (no x gradient launch in the profile)
+    give the bits of the two launches that a state off the vector boundary takes:
+    right-hand side, and a step with the CFL maxima and the characteristic faces."""
+    import torch
+    import compact_schemes_b200 as cs
+    b = cs.BC_NON_REFLECTIVE if open_x else cs.BC_PERIODIC
+    nbc = [[b, cs.BC_PERIODIC, cs.BC_PERIODIC]] * 2
+    s = solver(dims, nbc=nbc, gcbc=open_x, use_graph=False)
+    q = dev(O.tgv_init(dims, 0.2, 1e-3, 7))
+    out = {}
+    for off in (0, 1):
+        buf = torch.zeros(q.numel() + off, dtype=torch.float64, device=cuda)
+        buf[off:] = q
+        r = torch.zeros_like(q)
+        s.profile_begin()
+        s.rhs(buf[off:], r)
+        launches = {k: v[1] for k, v in s.profile_end().items()}
+        assert (launches["grad_x"], launches["flux_x"]) == (off, 1)
+        s.profile_begin()
+        s.step(buf[off:], 0.0)
+        launches = {k: v[1] for k, v in s.profile_end().items()}
+        assert (launches["grad_x"], launches["flux_x"]) == (off, 4)  # later stages start from the solver's own state
+        out[off] = (r, buf[off:].clone(), s.last_dt())
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
