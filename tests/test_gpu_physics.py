@@ -353,3 +353,67 @@ def test_time_step_of_a_state_with_nans_is_nan(cuda, n):
     bad[4, n - 1] = -1.0  # sqrt of a negative temperature
     assert np.isnan(_device_time_step(xim, etm, zem, bad, yaco, ssk, umf, 0.5))
     assert np.isnan(_device_time_step(xim, etm, zem, np.full_like(de, -np.nan), yaco, ssk, umf, 0.5))
+
+
+@pytest.mark.parametrize("viscous_limit", [False, True])
+def test_time_step_of_many_points_with_the_limit_in_the_last(cuda, viscous_limit):
+    """More points than one pass of the reduction's grid takes (148 * 8 * 256), the
+    limiting one last: the same bits as the oracle, whose maxima no order changes."""
+    n = 400001
+    xim, etm, zem, de, yaco, ssk = _time_step_fields(n, 12)
+    if viscous_limit:
+        ssk[-1] = 1e3
+    else:
+        de[1:4, -1] = 5.0
+    umf = (0.02, -0.01, 0.0)
+    dte = _device_time_step(xim, etm, zem, de, yaco, ssk, umf, 0.5)
+    ref = O.time_step(xim, etm, zem, de.ravel(), yaco, ssk, np.array(umf), 0.5)
+    head = O.time_step(*(m.reshape(3, n)[:, :-1].ravel() for m in (xim, etm, zem)), de[:, :-1].ravel(), yaco[:-1],
+                       ssk[:-1], np.array(umf), 0.5)
+    assert dte == ref and ref < head
+
+
+# (132, 160, 152): five fields, and four, are more than the 96 MB above which the
+# y and z derivatives fetch later tiles ahead, with the sum over the axes (z) and without (y)
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("dims", [tuple(n if a == axis else m for a, m in enumerate((9, 8, 10)))
+                                  for axis in range(3) for n in (40, 66, 127, 132, 255, 260, 514)]
+                         + [(70, 68, 66), (132, 160, 152)])
+def test_batched_call_sequence_line_lengths(cuda, dims, periodic):
+    """calc_viscous_shear_stress + calc_fluxes at the line lengths of every derivative
+    kernel (chunks of 2 to 32 rows, four lines per warp, ragged last chunks): several
+    fields per launch, received interface sums, the sum over the axes in the last
+    launch's store, against the oracle's right-hand side; and, where no sums are
+    received, the same bits as the fields' derivatives one call at a time."""
+    import torch
+    import compact_schemes_b200 as cs
+    b = cs.BC_PERIODIC if periodic else cs.BC_NON_REFLECTIVE
+    nbc = [[b] * 3, [b] * 3]
+    n = int(np.prod(dims))
+    q = O.tgv_init(dims, 0.2, 1e-3, 5)
+    q[3 * n:4 * n] = 0.05 * q[:n] * np.sin(np.arange(n) * 0.01)
+    xim, etm, zem, yaco = metric_fields(dims)
+    ref, scale = O.rhs(q, MU, O.field_metrics(xim, etm, zem, yaco), dims, [[int(periodic)] * 3] * 2, with_scale=True)
+    nm = cs.numerics_pc(dims, nbc)
+    nm.deriv_setup()
+    ph = cs.physics(dims, True)
+    qd, X, E, Z, Y = dev(q), dev(xim), dev(etm), dev(zem), dev(yaco)
+    de = torch.zeros(5 * n, dtype=torch.float64, device="cuda")
+    p = torch.zeros(n, dtype=torch.float64, device="cuda")
+    ssk = torch.full((n,), MU, dtype=torch.float64, device="cuda")
+    cs.thermo(qd, de, p)
+    ph.calc_viscous_shear_stress(de, ssk, X, E, Z, Y, dims, None, nm)
+    cs.thermo(qd, de, p)
+    ph.calc_fluxes(qd, p, de, X, E, Z, dims, None, nm)
+    torch.cuda.synchronize()
+    got = de.cpu().numpy().reshape(5, n)
+    assert max(np.abs(got[i] - ref.reshape(5, n)[i]).max() / scale[i] for i in range(5)) < 1e-12
+    if periodic:
+        return
+    b0 = device_view(ph.buffers()[0], 15 * n)  # the fluxes [5][3][n]
+    one = torch.empty(3 * n, dtype=torch.float64, device="cuda")
+    for m in range(5):
+        for a in range(3):
+            nm.deriv1d(a, b0[(3 * m + a) * n:(3 * m + a + 1) * n], one[a * n:(a + 1) * n], 0, 0, nm.dcomp, 0)
+        total = (one[:n] + one[n:2 * n]) + one[2 * n:]
+        assert torch.equal(total, de[m * n:(m + 1) * n]), m
