@@ -302,15 +302,27 @@ __device__ __forceinline__ void warp_solve(const DevTables<CT> &T, CT (&d)[NV][L
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         y0[v] = d[v][0];
-        y1[v] = CT(0);
-        // Every row is read and the value selected: a conditional read becomes one
-        // from a selected address and leaves the array in local memory (a 33x352x352
-        // step with two such axes took 8.6 ms for 8.2, a 264x120x120 derivative along
-        // x 72 us for 47).
+        if constexpr (NV > 1) {
+            y1[v] = CT(0);
 #pragma unroll
-        for (int t = 1; t < LT; ++t) {
-            const CT x = d[v][t];
-            y1[v] = t == len - 1 ? x : y1[v];
+            for (int t = 1; t < LT; ++t)
+                if (t == len - 1) y1[v] = d[v][t];
+        } else {
+            // With one right-hand side the compiler makes a conditional read one from a
+            // selected address and leaves the array in local memory (a 33x352x352 step
+            // with two such axes took 8.6 ms for 8.2, a 264x120x120 derivative along x
+            // 72 us for 47): read every row and select the value, where the last chunk
+            // is not full (the same in every lane).
+            y1[v] = len >= 2 ? d[v][LT - 1] : CT(0);
+            if (T.last_len < LT) {
+                CT r = CT(0);
+#pragma unroll
+                for (int t = 0; t < LT; ++t) {
+                    const CT x = d[v][t];
+                    r = t == len - 1 ? x : r;
+                }
+                y1[v] = len >= 2 ? r : CT(0);
+            }
         }
     }
     reduced_solve<NV, CT, W>(T, y0, y1, lane);
