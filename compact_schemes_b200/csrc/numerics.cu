@@ -591,7 +591,7 @@ static int deriv_ahead(const cs_dcomp &d, int nf, bool with_sum) {
 // y and z lines in column tiles (k_deriv_col) of NL groups of eight lines.
 template <int LT, int AXIS, int NL, typename T>
 static int launch_deriv_col(const FieldSet<T> &fs, int nf, const DevTables<T> &tab, const cs_dcomp &d, int nstart,
-                            int nend, const Coeffs &cf, const DerivSum *sum, cudaStream_t st) {
+                            int nend, const Coeffs &cf, const DerivSum *sum, int nsm, cudaStream_t st) {
     constexpr int TL = 8;
     const int64_t F = face_size(d, AXIS);
     const size_t smem = (size_t)NL * (Column<LT, TL>::kField + 4 * TL) * sizeof(T);
@@ -600,7 +600,11 @@ static int launch_deriv_col(const FieldSet<T> &fs, int nf, const DevTables<T> &t
         if (sum) kern = k_deriv_col<LT, AXIS, TL, NL, T, true>;
     }
     if (int rc = prep_smem(kern, smem)) return rc;
-    kern<<<dim3((unsigned)((F + NL * TL - 1) / (NL * TL)), (unsigned)nf), column_threads(TL, tab.p), smem, st>>>(
+    // Where not every SM gets a CTA, eight warps in each solve the reduced systems in
+    // one round, whatever the lines' chunks need (24x24x16 along z 5.2 -> 4.0 us).
+    const int64_t blocks = (F + NL * TL - 1) / (NL * TL);
+    const int threads = blocks * nf < nsm ? TL * 32 : column_threads(TL, tab.p);
+    kern<<<dim3((unsigned)blocks, (unsigned)nf), threads, smem, st>>>(
         fs, tab, d.lxi, d.let, nstart, nend, (int)F, cf, sum ? *sum : DerivSum{}, deriv_ahead(d, nf, sum != nullptr));
     CSB_CUDA(cudaGetLastError());
     return CS_OK;
@@ -616,9 +620,11 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
         // 4 KB and more.  With 128 bytes (FP64, lines of 257..512 points) that still
         // pays for the table-driven solve (400x96x96, physical closure 31 -> 25 us;
         // staged 33), not for the faster interior one (512x88x88, interface closure
-        // 24.6 against 22.6 us staged), and not on lines of more than 512 points
-        // (1024x64x64: FP64 28.7 against 26.7, FP32 18.5 against 14.4 us).
-        const bool vectors = LT * sizeof(T) <= 64 || (LT == 16 && !tab.interior);
+        // 24.6 against 22.6 us staged), and on lines of more than 512 points only in FP32
+        // with fewer CTAs than SMs (FP32 1024x16x16 7.5 against 10.8 us, 1024x64x64 18.5
+        // against 14.4; FP64 28.7 against 26.7 us).
+        const bool vectors = LT * sizeof(T) <= 64 || (LT == 16 && !tab.interior) ||
+                             (LT == 32 && sizeof(T) == 4 && (F + WARPS - 1) / WARPS * nf < nsm);
         const dim3 grid((unsigned)((F + NV * WARPS - 1) / (NV * WARPS)), (unsigned)nf);
         auto aligned = [&](int vb) {
             const int64_t ve = vb / (int)sizeof(T);
@@ -661,8 +667,8 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
             // would not give every SM a CTA (16x400x16 7.5 -> 5.3 us).
             const DerivSum *s = with_sum ? sum : nullptr;
             if (LT == 16 && (F + 15) / 16 * nf < nsm)
-                return launch_deriv_col<LT, AXIS, LT >= 16 ? 1 : 2, T>(fs, nf, tab, d, nstart, nend, cf, s, st);
-            return launch_deriv_col<LT, AXIS, LT == 32 ? 1 : 2, T>(fs, nf, tab, d, nstart, nend, cf, s, st);
+                return launch_deriv_col<LT, AXIS, LT >= 16 ? 1 : 2, T>(fs, nf, tab, d, nstart, nend, cf, s, nsm, st);
+            return launch_deriv_col<LT, AXIS, LT == 32 ? 1 : 2, T>(fs, nf, tab, d, nstart, nend, cf, s, nsm, st);
         }
     }
     CSB_CUDA(cudaGetLastError());
