@@ -274,7 +274,7 @@ int cs_ensemble_create(cs_ensemble **out, int nbox, const cs_solver_config *boxe
     cudaMemset(e->grad, 0, e->ng * sizeof(double));
     cudaMemset(e->dt, 0, nbox * sizeof(double));
     cudaMemset(e->ctl, 0, (2 + kEnsPhases * nbox) * sizeof(int));
-    if (e->lt_max > 4) e->tune.tile = 4;  // 8-line tiles of 256-point lines need 82 KB
+    if (e->lt_max > 4) e->tune.tile = 4;  // 8-line tiles of 256-point lines need 97 KB
     if (int rc = ens_check_tuning(e, e->tune)) { cs_ensemble_destroy(e); return rc; }
     if (int rc = ens_build_lists(e)) { cs_ensemble_destroy(e); return rc; }
     if (cudaDeviceSynchronize() != cudaSuccess) {

@@ -621,7 +621,7 @@ static int launch_deriv_lt(const FieldSet<T> &fs, int nf, const DevTables<T> &ta
         // pays for the table-driven solve (400x96x96, physical closure 31 -> 25 us;
         // staged 33), not for the faster interior one (512x88x88, interface closure
         // 24.6 against 22.6 us staged), and on lines of more than 512 points only in FP32
-        // with fewer CTAs than SMs (FP32 1024x16x16 7.5 against 10.8 us, 1024x64x64 18.5
+        // with fewer CTAs than SMs (FP32 1024x16x16 5.5 against 10.8 us, 1024x64x64 18.5
         // against 14.4; FP64 28.7 against 26.7 us).
         const bool vectors = LT * sizeof(T) <= 64 || (LT == 16 && !tab.interior) ||
                              (LT == 32 && sizeof(T) == 4 && (F + WARPS - 1) / WARPS * nf < nsm);

@@ -2,10 +2,11 @@
 // physics::calc_fluxes, physics::calc_viscous_shear_stress,
 // physics::calc_time_step (src/physics_pc.hpp:83-256) and gcbc_go
 // (src/gcbc.hpp:86-186) with per-point metric arrays, for drop-in callers
-// that hold the reference's buffers.  Line solves go through cs_deriv with
-// the numerics object's interface buffers (fill_buffers -> single-rank halo
-// exchange -> deriv2d), exactly the reference's data flow.  The fused solver
-// (fused.cu) is the fast path; this file is the compatibility path.
+// that hold the reference's buffers.  The data flow is the reference's (interface
+// sums -> single-rank exchange -> derivatives, through the numerics object's
+// buffers), one launch for all faces' sums (exchange_self) and one per axis for
+// all fields' derivatives (deriv_fields).  The fused solver (fused.cu) is the fast
+// path; this file is the compatibility path.
 #include <cmath>
 #include <cstring>
 
